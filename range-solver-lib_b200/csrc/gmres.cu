@@ -3,11 +3,16 @@
 //   cycle start  true residual ro = b - A x, ||x||, beta = ||ro||, error and
 //                stopping rule (:401-427)
 //   inner step k v_k = w / h_{k,k-1} (v_0 = ro / beta), z_k = P v_k (:430-446)
-//                w = A z_k (:451-455)
-//                h_{i,k} = v_i^T w for i <= k, one batched pass (:457-484)
-//                w -= sum_i h_{i,k} v_i and ||w|| in one pass (:486-510)
-//                Givens rotations on column k, g update, inner exit when
-//                |g_{k+1}| < 1e-4 beta (:519-550)
+//                w = A z_k (:451-455) and h_{i,k} = v_i^T w for i <= k (:457-484)
+//                in one kernel (k_gm_step)
+//                w -= sum_i h_{i,k} v_i, ||w||, P w (:486-510), and in its last
+//                block the Givens rotations on column k, the g update and the
+//                inner exit when |g_{k+1}| < 1e-4 beta (:519-550) (k_gm_correct)
+// The basis is stored unnormalised: slot k + 1 of V holds w and slot k + 1 of Z
+// holds P w as k_gm_correct leaves them, and inv[k + 1] = 1 / ||w|| multiplies
+// whatever is read from those slots, so an inner step is two launches and V is
+// never rewritten.  (The learned preconditioner needs v_k itself: there k_gm_vz
+// normalises the slot in place and inv stays 1.)
 //   cycle end    back substitution (:554-567), x += sum_j z_j y_j (:570-578)
 // Z is stored, so a variable preconditioner (flexible GMRES) needs no change.
 // Each cycle is one captured CUDA graph; the host polls the device state once
@@ -92,25 +97,59 @@ __global__ void __launch_bounds__(kBlock) k_gm_residual(Csr<double> M, Sell<doub
     }
 }
 
-// v_k = src / s (0 if s == 0), z_k = P v_k.  src = ro for k = 0, else w.  T: vector type
-// of the Arnoldi vectors (double, or float in mixed precision); D: preconditioner values.
+// 16-byte packs of the basis type.
+template <typename T>
+struct Pack;
+template <>
+struct Pack<double> {
+    static constexpr int N = 2;
+    __device__ __forceinline__ static void ld(const double *p, double (&v)[2])
+    {
+        const double2 t = *reinterpret_cast<const double2 *>(p);
+        v[0] = t.x;
+        v[1] = t.y;
+    }
+    __device__ __forceinline__ static void st(double *p, const double (&v)[2])
+    {
+        *reinterpret_cast<double2 *>(p) = make_double2(v[0], v[1]);
+    }
+};
+template <>
+struct Pack<float> {
+    static constexpr int N = 4;
+    __device__ __forceinline__ static void ld(const float *p, float (&v)[4])
+    {
+        const float4 t = *reinterpret_cast<const float4 *>(p);
+        v[0] = t.x;
+        v[1] = t.y;
+        v[2] = t.z;
+        v[3] = t.w;
+    }
+    __device__ __forceinline__ static void st(float *p, const float (&v)[4])
+    {
+        *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
+    }
+};
+
+// v_k = src / s (0 if s == 0), z_k = P v_k.  src = ro for k = 0, else slot k of V, in place.  T: vector
+// type of the Arnoldi vectors (double, or float in mixed precision); D: preconditioner values.
 template <int PK, typename T, typename D>
-__global__ void __launch_bounds__(kBlock) k_gm_vz(uint32_t n, uint32_t w_, const D *__restrict__ d,
-                                                  const double *__restrict__ ro, const T *__restrict__ wv,
-                                                  const double *__restrict__ wnorm, T *__restrict__ V,
-                                                  T *__restrict__ Z, const GmresState *st, uint32_t k)
+__global__ void __launch_bounds__(kBlock) k_gm_vz(uint32_t n, size_t ld, uint32_t w_, const D *__restrict__ d,
+                                                  const double *__restrict__ ro, const double *__restrict__ wnorm,
+                                                  T *V, T *Z, double *inv, const GmresState *st, uint32_t k)
 {
     pdl_wait();
     pdl_release();
     if (st->done || st->inner_done) return;
     const double s = (k == 0) ? st->beta : wnorm[k];
-    T *v = V + size_t(k) * n, *z = Z + size_t(k) * n;
+    T *v = V + size_t(k) * ld, *z = Z + size_t(k) * ld;
+    if (blockIdx.x == 0 && threadIdx.x == 0) inv[k] = 1.0;
     const uint32_t G = PK == 2 ? w_ : 1, ng = n / G;
     for (uint32_t gi = blockIdx.x * blockDim.x + threadIdx.x; gi < ng; gi += gridDim.x * blockDim.x) {
         T vl[kMaxBlock];
         for (uint32_t j = 0; j < G; j++) {
             const size_t i = size_t(gi) * G + j;
-            const double src = (k == 0) ? ro[i] : double(wv[i]);
+            const double src = (k == 0) ? ro[i] : double(v[i]);
             vl[j] = T((s == 0.0) ? 0.0 : src / s);
             v[i] = vl[j];
         }
@@ -126,146 +165,338 @@ __global__ void __launch_bounds__(kBlock) k_gm_vz(uint32_t n, uint32_t w_, const
     }
 }
 
+// w = A z_k, for matrices without the SELL-32 copy (k_gm_step then starts from the stored w).
 template <int RPW, typename T>
-__global__ void __launch_bounds__(kBlock) k_gm_spmv(Csr<T> M, Sell<T> S, int use_sell, const T *__restrict__ Z,
-                                                    T *__restrict__ wv, GmresState *st, uint32_t k)
+__global__ void __launch_bounds__(kBlock) k_gm_spmv(Csr<T> M, Sell<T> S, int use_sell, const T *__restrict__ z,
+                                                    T *__restrict__ wv, const double *inv, GmresState *st, uint32_t k)
 {
     pdl_wait();
     pdl_release();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     if (st->done || st->inner_done) return;
-    const T *z = Z + size_t(k) * M.n;
+    const double s = inv[k];
     auto gx = [&](uint32_t c) { return z[c]; };
-    auto epi = [&](uint32_t row, T v) { wv[row] = v; };
+    auto epi = [&](uint32_t row, T v) { wv[row] = T(double(v) * s); };
     for_rows_any<T, RPW>(M, S, use_sell != 0, gx, epi, smem_raw, &st->ticket[7], true);
 }
 
-// h_i = v_i^T w for i <= k: blockIdx.y = i.  Last block of the 2-D grid stores column k of H.
-template <typename T>
-__global__ void __launch_bounds__(kBlock) k_gm_dots(uint32_t n, const T *__restrict__ V,
-                                                    const T *__restrict__ wv, double *__restrict__ H,
-                                                    double *__restrict__ hv, double *partials, GmresState *st,
-                                                    uint32_t k)
+// One Arnoldi product: w = A z_k (FUSE; otherwise w is read) and h_i = v_i^T w for i <= k.
+//
+// A block takes tiles of 256 rows: its eight warps form w of their 32-row slices, leave it in shared
+// memory, and then split the vectors (warp j takes v_j, v_{j+8}, ...: JM of them at most), each reading
+// its vectors' tile with 16-byte loads and keeping one accumulator per vector and thread.  So w is
+// read once instead of once per vector, and a vector costs one warp reduction per block instead of a
+// block reduction.  Bound by the chain of a launch (state, slices, gathers, vectors, ticket, partials)
+// up to about ten vectors and by reading V above.  61^3 convection-diffusion (226,981 rows, 1.6M
+// entries, FP64, GMRES(30)), an inner step on average: w, normalisation, product, dots and correction as
+// four launches with w re-read per vector 59.4 us; this kernel and k_gm_correct 27.8 us (20.0 -> 9.7 ms a
+// solve).  A separate product kernel in front of the dots: 32.3 us.
+template <typename T, bool FUSE, int JM>
+__global__ void __launch_bounds__(kBlock) k_gm_step(Sell<T> S, uint32_t n, size_t ld, const T *V, const T *__restrict__ z,
+                                                    T *wv, double *__restrict__ H, double *__restrict__ hv,
+                                                    const double *inv, double *partials, GmresState *st, uint32_t k)
 {
     pdl_wait();
     pdl_release();
-    __shared__ double sh[32];
+    using P = Pack<T>;
+    __shared__ __align__(16) T ws[kBlock];
     __shared__ bool is_last;
     if (st->done || st->inner_done) return;
-    if (blockIdx.y > k) return;
-    const T *v = V + size_t(blockIdx.y) * n;
-    double acc[1] = {0.0};
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        acc[0] += double(wv[i]) * double(v[i]);
-    block_sum<1>(acc, sh);
-    const unsigned int nblocks = gridDim.x * (k + 1);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const double s = FUSE ? inv[k] : 1.0;
+    double acc[JM];
+#pragma unroll
+    for (int j = 0; j < JM; j++) acc[j] = 0.0;
+    const uint32_t tiles = (n + kBlock - 1) / kBlock;
+    for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x) {
+        const uint32_t row0 = t * kBlock;
+        if (FUSE) {
+            T mine = T(0);
+            auto gx = [&](uint32_t c) { return z[c]; };
+            auto epi = [&](uint32_t row, T v) {
+                mine = T(double(v) * s);
+                wv[row] = mine;
+            };
+            for_rows_sell_v<T>(S, gx, epi, t, tiles);  // exactly this tile: one slice per warp
+            ws[threadIdx.x] = mine;
+        } else {
+            const uint32_t row = row0 + threadIdx.x;
+            ws[threadIdx.x] = row < n ? wv[row] : T(0);
+        }
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < JM; j++) {
+            const uint32_t i = uint32_t(warp + 8 * j);
+            if (i <= k) {
+                const T *v = V + size_t(i) * ld + row0;
+                if (row0 + kBlock <= n) {
+                    constexpr int L = kBlock / (32 * P::N);
+                    T a[L][P::N];
+#pragma unroll
+                    for (int u = 0; u < L; u++) P::ld(v + (u * 32 + lane) * P::N, a[u]);
+#pragma unroll
+                    for (int u = 0; u < L; u++) {
+                        T b[P::N];
+                        P::ld(ws + (u * 32 + lane) * P::N, b);
+#pragma unroll
+                        for (int e = 0; e < P::N; e++) acc[j] += double(b[e]) * double(a[u][e]);
+                    }
+                } else {
+                    for (uint32_t e = lane; row0 + e < n; e += 32) acc[j] += double(ws[e]) * double(v[e]);
+                }
+            }
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int j = 0; j < JM; j++) {
+        const uint32_t i = uint32_t(warp + 8 * j);
+        if (i <= k) {
+            const double v = warp_sum(acc[j]);
+            if (lane == 0) partials[size_t(i) * gridDim.x + blockIdx.x] = v;
+        }
+    }
+    __syncthreads();
     if (threadIdx.x == 0) {
-        partials[size_t(blockIdx.y) * gridDim.x + blockIdx.x] = acc[0];
         __threadfence();
-        is_last = (atomicAdd(&st->ticket[1], 1u) == nblocks - 1);
+        is_last = (atomicAdd(&st->ticket[1], 1u) == gridDim.x - 1);
     }
     __syncthreads();
     if (!is_last) return;
     __threadfence();
+    // the last block adds the partials: a warp sums its vectors side by side, so that all their loads
+    // are in flight together
     const uint32_t m = st->m;
-    for (uint32_t i = 0; i <= k; i++) {
-        double s[1] = {0.0};
-        for (uint32_t bx = threadIdx.x; bx < gridDim.x; bx += blockDim.x) s[0] += __ldcg(&partials[size_t(i) * gridDim.x + bx]);
-        block_sum<1>(s, sh);
-        if (threadIdx.x == 0) {
-            H[size_t(i) * m + k] = s[0];
-            hv[i] = s[0];
+#pragma unroll
+    for (int j = 0; j < JM; j++) acc[j] = 0.0;
+#pragma unroll 4
+    for (uint32_t bx = lane; bx < gridDim.x; bx += 32)
+#pragma unroll
+        for (int j = 0; j < JM; j++) {
+            const uint32_t i = uint32_t(warp + 8 * j);
+            if (i <= k) acc[j] += __ldcg(&partials[size_t(i) * gridDim.x + bx]);
+        }
+#pragma unroll
+    for (int j = 0; j < JM; j++) {
+        const uint32_t i = uint32_t(warp + 8 * j);
+        if (i <= k) {
+            const double sum = warp_sum(acc[j]);
+            if (lane == 0) {
+                const double h = sum * inv[i];  // v_i = inv_i (slot i)
+                H[size_t(i) * m + k] = h;
+                hv[i] = h * inv[i];             // the factor of slot i in w -= h_i v_i
+            }
         }
     }
     if (threadIdx.x == 0) st->ticket[1] = 0u;
 }
 
-// w -= sum_i hv_i v_i; ||w|| -> Givens update of column k (last block).
-template <typename T>
-__global__ void __launch_bounds__(kBlock) k_gm_correct(uint32_t n, const T *__restrict__ V,
-                                                       T *__restrict__ wv, const double *__restrict__ hv_g,
-                                                       double *__restrict__ H, double *__restrict__ cs,
-                                                       double *__restrict__ sn, double *__restrict__ g,
-                                                       double *__restrict__ wnorm, double *partials, GmresState *st,
-                                                       uint32_t k)
+// w -= sum_i h_i v_i (hv holds h_i inv_i, the factor of slot i), P w and ||w||; the last block applies
+// the Givens rotations to column k.  16-byte loads of V, eight vectors in flight; the rotations, a
+// serial chain, run on shared-memory copies of the column (from L2 each of its 2k loads cost a round
+// trip: about 10 us of a step at k = 30).
+template <int PK, typename T, typename D>
+__global__ void __launch_bounds__(kBlock) k_gm_correct(uint32_t n, size_t ld, uint32_t w_, const D *__restrict__ d,
+                                                       const T *V, T *wv, T *__restrict__ zn,
+                                                       const double *__restrict__ hv_g, double *__restrict__ H,
+                                                       double *__restrict__ cs, double *__restrict__ sn,
+                                                       double *__restrict__ g, double *__restrict__ wnorm,
+                                                       double *inv, double *partials, GmresState *st, uint32_t k)
 {
     pdl_wait();
     pdl_release();
+    using P = Pack<T>;
     __shared__ double sh[32];
     __shared__ double hv[kMaxRestart + 1];
+    __shared__ double hc[kMaxRestart + 1], cc[kMaxRestart], ss[kMaxRestart];
     if (st->done || st->inner_done) return;
     for (uint32_t i = threadIdx.x; i <= k; i += blockDim.x) hv[i] = hv_g[i];
     __syncthreads();
     double acc[1] = {0.0};
-    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
+    auto row_value = [&](uint32_t j) {
         double value = double(wv[j]);
-        for (uint32_t i = 0; i <= k; i++) value -= hv[i] * double(V[size_t(i) * n + j]);
-        const T stored = T(value);
-        wv[j] = stored;
-        acc[0] += double(stored) * double(stored);
+        for (uint32_t i = 0; i <= k; i++) value -= hv[i] * double(V[size_t(i) * ld + j]);
+        return T(value);
+    };
+    const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+    if (PK < 2) {
+        constexpr int N = P::N;
+        const uint32_t np = n / N;
+        for (uint32_t p = tid; p < np; p += stride) {
+            T w[N];
+            P::ld(wv + size_t(p) * N, w);
+            double val[N];
+#pragma unroll
+            for (int e = 0; e < N; e++) val[e] = double(w[e]);
+            const T *vp = V + size_t(p) * N;
+            uint32_t i = 0;
+            for (; i + 8 <= k + 1; i += 8) {
+                T a[8][N];
+#pragma unroll
+                for (int u = 0; u < 8; u++) P::ld(vp + size_t(i + u) * ld, a[u]);
+#pragma unroll
+                for (int u = 0; u < 8; u++)
+#pragma unroll
+                    for (int e = 0; e < N; e++) val[e] -= hv[i + u] * double(a[u][e]);
+            }
+            if (i <= k) {  // the last one to seven vectors, loaded together
+                T a[7][N];
+#pragma unroll
+                for (int u = 0; u < 7; u++)
+                    if (i + u <= k) P::ld(vp + size_t(i + u) * ld, a[u]);
+#pragma unroll
+                for (int u = 0; u < 7; u++)
+                    if (i + u <= k)
+#pragma unroll
+                        for (int e = 0; e < N; e++) val[e] -= hv[i + u] * double(a[u][e]);
+            }
+            T z[N];
+#pragma unroll
+            for (int e = 0; e < N; e++) {
+                w[e] = T(val[e]);
+                acc[0] += double(w[e]) * double(w[e]);
+                z[e] = PK == 1 ? T(d[size_t(p) * N + e]) * w[e] : w[e];
+            }
+            P::st(wv + size_t(p) * N, w);
+            if (zn) P::st(zn + size_t(p) * N, z);
+        }
+        const uint32_t j = np * N + tid;
+        if (j < n) {
+            const T w = row_value(j);
+            wv[j] = w;
+            acc[0] += double(w) * double(w);
+            if (zn) zn[j] = PK == 1 ? T(d[j]) * w : w;
+        }
+    } else {
+        const uint32_t G = w_, ng = n / G;
+        for (uint32_t gi = tid; gi < ng; gi += stride) {
+            T wl[kMaxBlock];
+            for (uint32_t j = 0; j < G; j++) {
+                const uint32_t r = gi * G + j;
+                wl[j] = row_value(r);
+                wv[r] = wl[j];
+                acc[0] += double(wl[j]) * double(wl[j]);
+            }
+            if (zn)
+                for (uint32_t j = 0; j < G; j++) {
+                    const D *row = d + (size_t(gi) * G + j) * G;
+                    T z = T(0);
+                    for (uint32_t l = 0; l < G; l++) z += T(row[l]) * wl[l];
+                    zn[size_t(gi) * G + j] = z;
+                }
+        }
     }
     double tot[1];
-    if (grid_sum<1>(acc, partials, &st->ticket[2], sh, tot) && threadIdx.x == 0) {
-        const uint32_t m = st->m;
-        auto h = [&](uint32_t i, uint32_t j) -> double & { return H[size_t(i) * m + j]; };
-        h(k + 1, k) = sqrt(tot[0]);
-        // v_{k+1} = w / h_{k+1,k} is formed by the next step's k_gm_vz, after the
-        // rotation below has zeroed h_{k+1,k}; keep the norm for it
-        wnorm[k + 1] = h(k + 1, k);
+    if (!grid_sum<1>(acc, partials, &st->ticket[2], sh, tot)) return;
+    const uint32_t m = st->m;
+    for (uint32_t i = threadIdx.x; i <= k; i += blockDim.x) {
+        hc[i] = __ldcg(&H[size_t(i) * m + k]);
+        if (i < k) {
+            cc[i] = __ldcg(&cs[i]);
+            ss[i] = __ldcg(&sn[i]);
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        // v_{k+1} = w / h_{k+1,k}: its scale is kept in inv, h_{k+1,k} itself is rotated away
+        const double hn = sqrt(tot[0]);
+        wnorm[k + 1] = hn;
+        inv[k + 1] = hn == 0.0 ? 0.0 : 1.0 / hn;
         for (uint32_t i = 1; i <= k; i++) {
-            const double hsave = h(i - 1, k);
-            h(i - 1, k) = cs[i - 1] * hsave + sn[i - 1] * h(i, k);
-            h(i, k) = -sn[i - 1] * hsave + cs[i - 1] * h(i, k);
+            const double hsave = hc[i - 1], hi = hc[i];
+            hc[i - 1] = cc[i - 1] * hsave + ss[i - 1] * hi;
+            hc[i] = -ss[i - 1] * hsave + cc[i - 1] * hi;
         }
-        const double gg = sqrt(h(k, k) * h(k, k) + h(k + 1, k) * h(k + 1, k));
-        if (gg == 0.0) {
-            cs[k] = sn[k] = 0.0;
-        } else {
-            cs[k] = h(k, k) / gg;
-            sn[k] = h(k + 1, k) / gg;
+        const double hk = hc[k];
+        const double gg = sqrt(hk * hk + hn * hn);
+        double ck = 0.0, sk = 0.0;
+        if (gg != 0.0) {
+            ck = hk / gg;
+            sk = hn / gg;
         }
-        h(k, k) = gg;
-        h(k + 1, k) = 0.0;
-        g[k + 1] = -sn[k] * g[k];
-        g[k] = cs[k] * g[k];
+        cs[k] = ck;
+        sn[k] = sk;
+        hc[k] = gg;
+        const double gk = g[k], gn = -sk * gk;
+        g[k + 1] = gn;
+        g[k] = ck * gk;
+        H[size_t(k + 1) * m + k] = 0.0;
         st->total_inner++;
         st->cycle_len = k + 1;
-        if (fabs(g[k + 1]) < st->beta * 1.0e-4) st->inner_done = 1;
+        if (fabs(gn) < st->beta * 1.0e-4) st->inner_done = 1;
         st->k = k + 1;
     }
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i <= k; i += blockDim.x) H[size_t(i) * m + k] = hc[i];
 }
 
-__global__ void k_gm_backsub(double *__restrict__ H, double *__restrict__ g, double *__restrict__ y,
-                             GmresState *st)
+// Back substitution (:554-567) by one block, column by column: as soon as y_j is known every thread
+// subtracts y_j h_ij from its own g_i, the order in which the reference's row loop subtracts them.
+// y is returned with the slots' scale: y_j inv_j multiplies slot j of Z.
+__global__ void __launch_bounds__(kMaxRestart) k_gm_backsub(const double *__restrict__ H, const double *__restrict__ g,
+                                                            const double *__restrict__ inv, double *__restrict__ y,
+                                                            const GmresState *st)
 {
     pdl_wait();
     pdl_release();
-    if (threadIdx.x != 0 || st->done) return;
-    const uint32_t m = st->m, it = st->cycle_len;
-    if (it == 0) return;
-    auto h = [&](uint32_t i, uint32_t j) -> double & { return H[size_t(i) * m + j]; };
-    y[it - 1] = (h(it - 1, it - 1) == 0.0) ? 0.0 : g[it - 1] / h(it - 1, it - 1);
-    for (int i = int(it) - 2; i >= 0; i--) {
-        for (int j = int(it) - 1; j > i; j--) g[i] -= y[j] * h(i, j);
-        y[i] = (h(i, i) == 0.0) ? 0.0 : g[i] / h(i, i);
+    __shared__ double yj;
+    if (st->done) return;
+    const uint32_t m = st->m, it = st->cycle_len, i = threadIdx.x;
+    double gi = i < it ? g[i] : 0.0;
+    const double hii = i < it ? H[size_t(i) * m + i] : 0.0;
+    double next = it > 0 && i < it - 1 ? H[size_t(i) * m + it - 1] : 0.0;
+    for (int j = int(it) - 1; j >= 0; j--) {
+        const double hij = next;
+        next = j > 0 && int(i) < j - 1 ? H[size_t(i) * m + j - 1] : 0.0;  // the next column, loaded ahead
+        if (int(i) == j) {
+            yj = hii == 0.0 ? 0.0 : gi / hii;
+            y[j] = yj * inv[j];
+        }
+        __syncthreads();
+        if (int(i) < j) gi -= yj * hij;
+        __syncthreads();
     }
 }
 
+// x += sum_j y_j z_j (:570-578), 16-byte loads, eight vectors in flight.
 template <typename T>
-__global__ void __launch_bounds__(kBlock) k_gm_update(uint32_t n, const T *__restrict__ Z,
+__global__ void __launch_bounds__(kBlock) k_gm_update(uint32_t n, size_t ld, const T *__restrict__ Z,
                                                       const double *__restrict__ y_g, double *__restrict__ x,
                                                       GmresState *st)
 {
     pdl_wait();
     pdl_release();
+    using P = Pack<T>;
+    constexpr int N = P::N;
     __shared__ double y[kMaxRestart];
     if (st->done) return;
     const uint32_t len = st->cycle_len;
     for (uint32_t j = threadIdx.x; j < len; j += blockDim.x) y[j] = y_g[j];
     __syncthreads();
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const uint32_t np = n / N, tid = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+    for (uint32_t p = tid; p < np; p += stride) {
+        double xv[N];
+#pragma unroll
+        for (int e = 0; e < N; e++) xv[e] = x[size_t(p) * N + e];
+        const T *zp = Z + size_t(p) * N;
+        for (uint32_t j = 0; j < len; j += 8) {
+            T a[8][N];
+#pragma unroll
+            for (int u = 0; u < 8; u++)
+                if (j + u < len) P::ld(zp + size_t(j + u) * ld, a[u]);
+#pragma unroll
+            for (int u = 0; u < 8; u++)
+                if (j + u < len)
+#pragma unroll
+                    for (int e = 0; e < N; e++) xv[e] += double(a[u][e]) * y[j + u];
+        }
+#pragma unroll
+        for (int e = 0; e < N; e++) x[size_t(p) * N + e] = xv[e];
+    }
+    const uint32_t i = np * N + tid;
+    if (i < n) {
         double xi = x[i];
-        for (uint32_t j = 0; j < len; j++) xi += double(Z[size_t(j) * n + i]) * y[j];
+        for (uint32_t j = 0; j < len; j++) xi += double(Z[size_t(j) * ld + i]) * y[j];
         x[i] = xi;
     }
 }
@@ -286,22 +517,20 @@ __global__ void k_gm_cycle_end(GmresState *st)
 size_t gmres_workspace_bytes(uint32_t n, uint32_t m, bool mixed, uint32_t w)
 {
     const size_t vn = arena_bytes(n, sizeof(double));
-    const size_t vt = mixed ? arena_bytes(size_t(m + 1) * n, sizeof(float)) : arena_bytes(size_t(m + 1) * n, 8);
-    return 2 * vt + (mixed ? arena_bytes(n, sizeof(float)) : vn) + vn + arena_bytes(size_t(m + 1) * m, sizeof(double)) +
-           6 * arena_bytes(m + 2, sizeof(double)) + (mixed ? arena_bytes(size_t(n) * w, sizeof(float)) : 0);
+    const size_t vt = arena_bytes(size_t(m + 1) * gmres_ld(n), mixed ? sizeof(float) : sizeof(double));
+    return 2 * vt + vn + arena_bytes(size_t(m + 1) * m, sizeof(double)) + 7 * arena_bytes(m + 2, sizeof(double)) +
+           (mixed ? arena_bytes(size_t(n) * w, sizeof(float)) : 0);
 }
 
 rsg_status gmres_carve(rsg_context *ctx, GmresArgs &a, uint32_t n, uint32_t m)
 {
     if (m > kMaxRestart) return set_error(ctx, RSG_ERR_UNSUPPORTED, "GMRES restart length %u > %u", m, kMaxRestart);
     if (a.mixed) {
-        a.V32 = arena_take<float>(ctx, size_t(m + 1) * n);
-        a.Z32 = arena_take<float>(ctx, size_t(m + 1) * n);
-        a.w32 = arena_take<float>(ctx, n);
+        a.V32 = arena_take<float>(ctx, size_t(m + 1) * gmres_ld(n));
+        a.Z32 = arena_take<float>(ctx, size_t(m + 1) * gmres_ld(n));
     } else {
-        a.V = arena_take<double>(ctx, size_t(m + 1) * n);
-        a.Z = arena_take<double>(ctx, size_t(m + 1) * n);
-        a.w = arena_take<double>(ctx, n);
+        a.V = arena_take<double>(ctx, size_t(m + 1) * gmres_ld(n));
+        a.Z = arena_take<double>(ctx, size_t(m + 1) * gmres_ld(n));
     }
     a.ro = arena_take<double>(ctx, n);
     a.H = arena_take<double>(ctx, size_t(m + 1) * m);
@@ -311,7 +540,8 @@ rsg_status gmres_carve(rsg_context *ctx, GmresArgs &a, uint32_t n, uint32_t m)
     a.y = arena_take<double>(ctx, m + 2);
     a.hv = arena_take<double>(ctx, m + 2);
     a.wnorm = arena_take<double>(ctx, m + 2);
-    if (!a.wnorm) return set_error(ctx, RSG_ERR_OUT_OF_MEMORY, "GMRES workspace");
+    a.inv = arena_take<double>(ctx, m + 2);
+    if (!a.inv) return set_error(ctx, RSG_ERR_OUT_OF_MEMORY, "GMRES workspace");
     return RSG_OK;
 }
 
@@ -319,10 +549,28 @@ namespace {
 
 constexpr double kLearnedMinDrop = 0.1;
 
+// k_gm_step with the accumulator count of step k (vectors per warp: (k + 1) / 8 rounded up, to a power of two).
+template <typename T, bool FUSE>
+void launch_step(cudaStream_t st, bool pdl, int grid, const GmresArgs &a, const Sell<T> &S, uint32_t n, size_t ld,
+                 const T *V, const T *z, T *w, uint32_t k)
+{
+    const uint32_t jm = (k + 8) / 8;
+    auto go = [&](auto kernel) {
+        launch_k(st, pdl, kernel, grid, kBlock, 0, S, n, ld, V, z, w, a.H, a.hv, (const double *)a.inv, a.partials,
+                 a.st, k);
+    };
+    if (jm <= 1) go(k_gm_step<T, FUSE, 1>);
+    else if (jm <= 2) go(k_gm_step<T, FUSE, 2>);
+    else if (jm <= 4) go(k_gm_step<T, FUSE, 4>);
+    else if (jm <= 8) go(k_gm_step<T, FUSE, 8>);
+    else go(k_gm_step<T, FUSE, 16>);
+}
+
 template <int RPW, int PK>
 rsg_status run_typed(rsg_context *ctx, const GmresArgs &a, double *seconds)
 {
     const uint32_t n = a.A->n, m = a.m;
+    const size_t ld = gmres_ld(n);
     const Csr<double> M = view<double>(a.A, true);
     const size_t s64 = a.A->use_sell ? 0 : tma_smem<double>();
     cudaFuncSetAttribute(k_gm_residual<RPW>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(tma_smem<double>()));
@@ -339,9 +587,17 @@ rsg_status run_typed(rsg_context *ctx, const GmresArgs &a, double *seconds)
     const int g_sp = spmv_grid(ctx, a.A, (const void *)k_gm_spmv<RPW, double>, s64, RPW);
     const int g_sp32 = spmv_grid(ctx, a.A, (const void *)k_gm_spmv<RPW, float>, s32, RPW);
     const int g_res = spmv_grid(ctx, a.A, (const void *)k_gm_residual<RPW>, s64, RPW);
-    const int g_vec = std::min(grid_for(ctx, (const void *)k_gm_correct<double>, kBlock, 0, n), kMaxGrid);
-    const int g_dot =
-        std::min(std::min(grid_for(ctx, (const void *)k_gm_dots<double>, kBlock, 0, n), 512), kMaxGrid);
+    const int g_vec = std::min(grid_for(ctx, (const void *)k_gm_update<double>, kBlock, 0, n), kMaxGrid);
+    const int g_cor = std::min(grid_for(ctx, (const void *)k_gm_correct<PK, double, double>, kBlock, 0,
+                                        PK < 2 ? (long long)n / (a.mixed ? 4 : 2) : n),
+                               kMaxGrid);
+    // k_gm_step: every block takes the same number of tiles (the fewest that one wave of blocks allows),
+    // since each block adds a ticket and (k + 1) partials.  226,981 rows = 887 tiles, 740 resident
+    // blocks: 444 blocks of two tiles 9.65 ms a solve; all 740 (some with two) 10.1 ms; one tile per block
+    // (888 blocks at 40 registers) 11.4 ms; 296 blocks of three 10.5 ms.
+    const int tiles = int((n + kBlock - 1) / kBlock);
+    const int full = std::min(grid_for(ctx, (const void *)k_gm_step<double, true, 4>, kBlock, 0, 1ll << 40), 1024);
+    const int g_dot = (tiles + (tiles + full - 1) / full - 1) / ((tiles + full - 1) / full);
 
     // One captured graph per cycle; with the learned preconditioner a second graph
     // (Jacobi z_k) is captured as the fallback.
@@ -353,20 +609,27 @@ rsg_status run_typed(rsg_context *ctx, const GmresArgs &a, double *seconds)
                  a.st);
         for (uint32_t k = 0; k < m; k++) {
             if (a.mixed) {  // FP32 Arnoldi step
-                launch_k(st, pdl, k_gm_vz<PK, float, float>, g_vec, kBlock, 0, n, a.P.w, a.P.d32, a.ro, a.w32,
-                         a.wnorm, a.V32, a.Z32, a.st, k);
-                launch_k(st, pdl, k_gm_spmv<RPW, float>, g_sp32, kBlock, s32, M32, S32, us, a.Z32, a.w32, a.st, k);
-                launch_k(st, pdl, k_gm_dots<float>, dim3(g_dot, k + 1), kBlock, 0, n, a.V32, a.w32, a.H, a.hv,
-                         a.partials, a.st, k);
-                launch_k(st, pdl, k_gm_correct<float>, g_vec, kBlock, 0, n, a.V32, a.w32, a.hv, a.H, a.cs, a.sn, a.g,
-                         a.wnorm, a.partials, a.st, k);
+                float *z = a.Z32 + size_t(k) * ld, *w = a.V32 + size_t(k + 1) * ld;
+                if (k == 0)
+                    launch_k(st, pdl, k_gm_vz<PK, float, float>, g_vec, kBlock, 0, n, ld, a.P.w, a.P.d32, a.ro,
+                             a.wnorm, a.V32, a.Z32, a.inv, a.st, k);
+                if (us) {
+                    launch_step<float, true>(st, pdl, g_dot, a, S32, n, ld, a.V32, z, w, k);
+                } else {
+                    launch_k(st, pdl, k_gm_spmv<RPW, float>, g_sp32, kBlock, s32, M32, S32, us, z, w,
+                             (const double *)a.inv, a.st, k);
+                    launch_step<float, false>(st, pdl, g_dot, a, S32, n, ld, a.V32, z, w, k);
+                }
+                launch_k(st, pdl, k_gm_correct<PK, float, float>, g_cor, kBlock, 0, n, ld, a.P.w, a.P.d32, a.V32, w,
+                         a.Z32 + size_t(k + 1) * ld, a.hv, a.H, a.cs, a.sn, a.g, a.wnorm, a.inv, a.partials, a.st, k);
                 continue;
             }
-            launch_k(st, pdl, k_gm_vz<PK, double, double>, g_vec, kBlock, 0, n, a.P.w, a.P.d, a.ro, a.w, a.wnorm,
-                     a.V, a.Z, a.st, k);
+            double *z = a.Z + size_t(k) * ld, *w = a.V + size_t(k + 1) * ld;
+            if (k == 0 || G)
+                launch_k(st, pdl, k_gm_vz<PK, double, double>, g_vec, kBlock, 0, n, ld, a.P.w, a.P.d, a.ro, a.wnorm,
+                         a.V, a.Z, a.inv, a.st, k);
             if (G) {  // flexible GMRES: z_k = M(v_k) from the network (Z is stored, src/rmatrixsolver.cpp:446)
-                const rsg_status gs =
-                    gnn_forward(ctx, G, a.A, a.V + size_t(k) * n, a.Z + size_t(k) * n, nullptr, false, true);
+                const rsg_status gs = gnn_forward(ctx, G, a.A, a.V + size_t(k) * ld, z, nullptr, false, true);
                 if (gs != RSG_OK) {
                     cudaGraph_t dummy = nullptr;
                     cudaStreamEndCapture(ctx->stream, &dummy);
@@ -374,15 +637,20 @@ rsg_status run_typed(rsg_context *ctx, const GmresArgs &a, double *seconds)
                     return gs;
                 }
             }
-            launch_k(st, pdl, k_gm_spmv<RPW, double>, g_sp, kBlock, s64, M, S, us, a.Z, a.w, a.st, k);
-            launch_k(st, pdl, k_gm_dots<double>, dim3(g_dot, k + 1), kBlock, 0, n, a.V, a.w, a.H, a.hv, a.partials,
+            if (us) {
+                launch_step<double, true>(st, pdl, g_dot, a, S, n, ld, a.V, z, w, k);
+            } else {
+                launch_k(st, pdl, k_gm_spmv<RPW, double>, g_sp, kBlock, s64, M, S, us, z, w, (const double *)a.inv,
+                         a.st, k);
+                launch_step<double, false>(st, pdl, g_dot, a, S, n, ld, a.V, z, w, k);
+            }
+            launch_k(st, pdl, k_gm_correct<PK, double, double>, g_cor, kBlock, 0, n, ld, a.P.w, a.P.d, a.V, w,
+                     G ? nullptr : a.Z + size_t(k + 1) * ld, a.hv, a.H, a.cs, a.sn, a.g, a.wnorm, a.inv, a.partials,
                      a.st, k);
-            launch_k(st, pdl, k_gm_correct<double>, g_vec, kBlock, 0, n, a.V, a.w, a.hv, a.H, a.cs, a.sn, a.g,
-                     a.wnorm, a.partials, a.st, k);
         }
-        launch_k(st, pdl, k_gm_backsub, 1, 32, 0, a.H, a.g, a.y, a.st);
-        if (a.mixed) launch_k(st, pdl, k_gm_update<float>, g_vec, kBlock, 0, n, a.Z32, a.y, a.x, a.st);
-        else launch_k(st, pdl, k_gm_update<double>, g_vec, kBlock, 0, n, a.Z, a.y, a.x, a.st);
+        launch_k(st, pdl, k_gm_backsub, 1, int(kMaxRestart), 0, a.H, a.g, a.inv, a.y, a.st);
+        if (a.mixed) launch_k(st, pdl, k_gm_update<float>, g_vec, kBlock, 0, n, ld, a.Z32, a.y, a.x, a.st);
+        else launch_k(st, pdl, k_gm_update<double>, g_vec, kBlock, 0, n, ld, a.Z, a.y, a.x, a.st);
         launch_k(st, pdl, k_gm_cycle_end, 1, 32, 0, a.st);
         cudaError_t e = cudaStreamEndCapture(ctx->stream, graph);
         if (e != cudaSuccess) return set_error(ctx, RSG_ERR_CUDA, "GMRES capture: %s", cudaGetErrorString(e));
