@@ -32,6 +32,11 @@ struct rsg_assembly {
     uint32_t *adj_ptr = nullptr, *adj_elem = nullptr;
     uint8_t *adj_loc = nullptr;
     uint16_t *adj_off = nullptr;
+    // heat plans: the (row, adjacent tet) pairs and the coordinates as k_asm_heat reads them (pack_heat_plan)
+    uint4 *pair = nullptr;
+    uint32_t *pair_ptr = nullptr;
+    double4 *xyz4 = nullptr;
+    bool near = false;
     uint32_t *tadj_ptr = nullptr, *tadj_tri = nullptr;
     uint8_t *node_mask = nullptr;
     double *stage = nullptr;   // host inputs staged on the device
@@ -80,106 +85,298 @@ __device__ __forceinline__ uint32_t node_of(const uint4 t, int k)
     return k == 0 ? t.x : k == 1 ? t.y : k == 2 ? t.z : t.w;
 }
 
-// Contribution of one (row node, adjacent tet) pair to the row: Ar[n] for the tet's
-// 4 nodes (theta scheme applied when transient) and the right-hand side part be
-// (source, transient history, Dirichlet lifting).
-__device__ __forceinline__ void heat_adj(uint32_t t, const uint32_t *__restrict__ adj_elem,
-                                         const uint8_t *__restrict__ adj_loc, const double *__restrict__ xyz,
-                                         const uint4 *__restrict__ tets, const uint32_t *__restrict__ book,
-                                         const double *__restrict__ k_e, const double *__restrict__ q_e,
-                                         const double *__restrict__ rhoc_e, const double *__restrict__ node_t,
-                                         int transient, double alpha, double dt, double (&Ar)[4], double &be)
+// ---- heat ----
+// What a thread reads for one (row, adjacent tet) pair: 16 bytes, stored in slices of 32 rows -- pair t of
+// lane l of slice s at pair[(pair_ptr[s] + t) * 32 + l], padded with tet RSG_EOD -- so that a warp's reads
+// are one contiguous 512 bytes.  Two forms:
+//   wide   {tet, local index m of the row's node, offsets of the tet's four nodes in the row as 16 bits
+//          each (0xffff: a fixed node)}; the node numbers come from the tet array;
+//   near   for rows of at most 32 entries whose neighbour nodes are numbered within 32767 of the row's:
+//          {tet, m | offsets as 6 bits each (63: a fixed node), node numbers less the row node's as
+//          16 bits each}, which saves the tet array's scattered 16 bytes per pair and a dependent load.
+
+__device__ __forceinline__ double4 ld_node(const double4 *p)
 {
-    const uint32_t e = adj_elem[t];
-    const int m = adj_loc[t];
-    const uint4 tv = tets[e];
-    double G[4][3];
-    const double V = tet_geometry(xyz, tv, G);
-    const double k = k_e[e];
-    double gm[3];
-    grad_row(G, m, gm);
-    for (int n = 0; n < 4; n++) Ar[n] = (gm[0] * G[n][0] + gm[1] * G[n][1] + gm[2] * G[n][2]) * k * V;
-    const double fe = q_e[e] * V / 4.0;
-    if (transient) {
-        const double rc = rhoc_e[e];
-        be = dt * fe;
+    double4 v;  // one 32-byte load (sm_100)
+    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
+    return v;
+}
+
+struct HeatIn {
+    const uint4 *pair;
+    const uint32_t *pair_ptr;
+    const double4 *xyz;
+    const uint4 *tets;
+    const double *k_e, *q_e, *rhoc_e, *node_t;
+    int transient;
+    double alpha, dt;
+    const uint32_t *row_node;
+};
+
+constexpr uint32_t kNoEntry = 0xffffu;
+
+template <bool NEAR>
+__device__ __forceinline__ void unpack_pair(const HeatIn &h, const uint4 pr, uint32_t row_node, uint32_t &m,
+                                            uint32_t (&node)[4], uint32_t (&off)[4])
+{
+    if constexpr (NEAR) {
+        m = pr.y & 3u;
         for (int n = 0; n < 4; n++) {
-            const double Me = rc * V * (m == n ? 2.0 : 1.0) / 20.0;
+            const uint32_t o = (pr.y >> (2 + 6 * n)) & 63u;
+            off[n] = o == 63u ? kNoEntry : o;
+        }
+        node[0] = row_node + uint32_t(int(int16_t(pr.z & 0xffffu)));
+        node[1] = row_node + uint32_t(int(int16_t(pr.z >> 16)));
+        node[2] = row_node + uint32_t(int(int16_t(pr.w & 0xffffu)));
+        node[3] = row_node + uint32_t(int(int16_t(pr.w >> 16)));
+    } else {
+        m = pr.y;
+        off[0] = pr.z & 0xffffu;
+        off[1] = pr.z >> 16;
+        off[2] = pr.w & 0xffffu;
+        off[3] = pr.w >> 16;
+        const uint4 tv = __ldg(h.tets + pr.x);
+        node[0] = tv.x;
+        node[1] = tv.y;
+        node[2] = tv.z;
+        node[3] = tv.w;
+    }
+}
+
+// Contribution of one pair: Ar[n] for the tet's 4 nodes (theta scheme applied when transient) and the
+// right-hand side part be (source, transient history, Dirichlet lifting).  The gradients are kept as
+// cofactors c_n = det grad N_n, so that grad N_m . grad N_n |det| / 6 = c_m . c_n / (6 |det|) takes one
+// division where dividing every gradient took nine.
+template <bool NEAR>
+__device__ __forceinline__ void heat_pair(const HeatIn &h, const uint4 pr, uint32_t row_node, double (&Ar)[4],
+                                          double &be, uint32_t (&off)[4])
+{
+    const uint32_t e = pr.x;
+    uint32_t m, node[4];
+    unpack_pair<NEAR>(h, pr, row_node, m, node, off);
+    const double4 p0 = ld_node(h.xyz + node[0]), p1 = ld_node(h.xyz + node[1]), p2 = ld_node(h.xyz + node[2]),
+                  p3 = ld_node(h.xyz + node[3]);
+    const double k = __ldg(h.k_e + e), q = __ldg(h.q_e + e);
+    const double a[3] = {p1.x - p0.x, p1.y - p0.y, p1.z - p0.z};
+    const double b[3] = {p2.x - p0.x, p2.y - p0.y, p2.z - p0.z};
+    const double c[3] = {p3.x - p0.x, p3.y - p0.y, p3.z - p0.z};
+    double C[4][3] = {{0.0, 0.0, 0.0},
+                      {b[1] * c[2] - b[2] * c[1], b[2] * c[0] - b[0] * c[2], b[0] * c[1] - b[1] * c[0]},
+                      {c[1] * a[2] - c[2] * a[1], c[2] * a[0] - c[0] * a[2], c[0] * a[1] - c[1] * a[0]},
+                      {a[1] * b[2] - a[2] * b[1], a[2] * b[0] - a[0] * b[2], a[0] * b[1] - a[1] * b[0]}};
+    const double det = fabs(a[0] * C[1][0] + a[1] * C[1][1] + a[2] * C[1][2]);
+    for (int i = 0; i < 3; i++) C[0][i] = -(C[1][i] + C[2][i] + C[3][i]);
+    double cm[3];
+    for (int i = 0; i < 3; i++) cm[i] = m == 0 ? C[0][i] : m == 1 ? C[1][i] : m == 2 ? C[2][i] : C[3][i];
+    const double s = k / (6.0 * det), V = det / 6.0;
+    for (int n = 0; n < 4; n++) Ar[n] = (cm[0] * C[n][0] + cm[1] * C[n][1] + cm[2] * C[n][2]) * s;
+    const double fe = q * V / 4.0;
+    if (h.transient) {
+        const double rc = __ldg(h.rhoc_e + e);
+        be = h.dt * fe;
+        for (int n = 0; n < 4; n++) {
+            const double Me = rc * V * (int(m) == n ? 2.0 : 1.0) / 20.0;
             const double Ke = Ar[n];
-            Ar[n] = Me + alpha * dt * Ke;
-            be += (Me - (1.0 - alpha) * dt * Ke) * node_t[node_of(tv, n)];
+            Ar[n] = Me + h.alpha * h.dt * Ke;
+            be += (Me - (1.0 - h.alpha) * h.dt * Ke) * __ldg(h.node_t + node[n]);
         }
     } else {
         be = fe;
     }
-    for (int n = 0; n < 4; n++) {
-        const uint32_t nd = node_of(tv, n);
-        if (book[nd] == RSG_EOD) be -= Ar[n] * node_t[nd];
-    }
+    for (int n = 0; n < 4; n++)
+        if (off[n] == kNoEntry) be -= Ar[n] * __ldg(h.node_t + node[n]);  // a fixed node
 }
 
-// Rows accumulated in global memory (any row length).
-__global__ void __launch_bounds__(kBlock) k_asm_heat(
-    uint32_t n_free, const uint32_t *__restrict__ row_node, const uint32_t *__restrict__ rp,
-    const uint32_t *__restrict__ adj_ptr, const uint32_t *__restrict__ adj_elem, const uint8_t *__restrict__ adj_loc,
-    const ushort4 *__restrict__ adj_off, const double *__restrict__ xyz, const uint4 *__restrict__ tets,
-    const uint32_t *__restrict__ book, const double *__restrict__ k_e, const double *__restrict__ q_e,
-    const double *__restrict__ rhoc_e, const double *__restrict__ node_t, int transient, double alpha, double dt,
-    double *__restrict__ val, double *__restrict__ b)
+// Where the assembled row goes: the CSR values and, once the matrix exists, every copy a refresh would
+// otherwise make in passes of its own (FP32, SELL-32 in both precisions) and ||A||_F^2.
+struct HeatOut {
+    double *val;
+    double *b;
+    float *val32 = nullptr;  // null: only val and b
+    double *sval = nullptr;  // null: no SELL-32 copy
+    float *sval32 = nullptr;
+    const uint32_t *slice_ptr = nullptr;
+    double *partials = nullptr;
+    unsigned int *ticket = nullptr;
+    double *norm = nullptr;
+};
+
+// Rows accumulated in global memory (any row length); val and b only.
+template <bool NEAR>
+__global__ void __launch_bounds__(kBlock) k_asm_heat(uint32_t n_free, const uint32_t *__restrict__ rp, HeatIn h,
+                                                     HeatOut o)
 {
     for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < n_free; r += gridDim.x * blockDim.x) {
-        const uint32_t a = row_node[r], start = rp[r], end = rp[r + 1];
-        for (uint32_t j = start; j < end; j++) val[j] = 0.0;
+        const uint32_t start = rp[r], end = rp[r + 1], s = r >> 5, a = h.row_node[r];
+        for (uint32_t j = start; j < end; j++) o.val[j] = 0.0;
         double bs = 0.0;
-        for (uint32_t t = adj_ptr[a]; t < adj_ptr[a + 1]; t++) {
+        for (uint32_t t = h.pair_ptr[s]; t < h.pair_ptr[s + 1]; t++) {
+            const uint4 pr = h.pair[size_t(t) * 32 + (r & 31u)];
+            if (pr.x == RSG_EOD) break;
             double Ar[4], be;
-            heat_adj(t, adj_elem, adj_loc, xyz, tets, book, k_e, q_e, rhoc_e, node_t, transient, alpha, dt, Ar, be);
-            const ushort4 off4 = adj_off[t];
-            const uint16_t off[4] = {off4.x, off4.y, off4.z, off4.w};
+            uint32_t off[4];
+            heat_pair<NEAR>(h, pr, a, Ar, be, off);
             bs += be;
             for (int n = 0; n < 4; n++)
-                if (off[n] != 0xffffu) val[start + off[n]] += Ar[n];
+                if (off[n] != kNoEntry) o.val[start + off[n]] += Ar[n];
         }
-        b[r] = bs;
+        o.b[r] = bs;
     }
 }
 
-// One thread per row with the row accumulated in shared memory (rows of up to kLocalRowMax
-// entries, the launch sizes it for the plan's longest row; entry j of a thread at
-// acc_s[j * blockDim.x + threadIdx.x]): the same per-entry order
-// as k_asm_heat without read-modify-write round trips through global memory.  A thread-local
-// array indexed by the column offset cannot stay in registers: it went through local memory,
-// 515 MB of DRAM writes per launch at 100^3 against 127 MB of results.
+// One thread per row with the row accumulated in shared memory (rows of up to kLocalRowMax entries; the
+// launch sizes it for the plan's longest row): the same per-entry order as k_asm_heat without
+// read-modify-write round trips through global memory.  Entry j of a thread is at acc[j * (kBlock + 1) +
+// thread], conflict-free both for a thread's own row and for half-warps that copy whole rows.
+//
+// Bound by the L1 traffic of the pairs' scattered 8-byte conductivities and sources and of the node
+// coordinates (24 pairs a row; L1 at 63% and FP64 at 21% of peak in the wide form).  Whole numeric assembly
+// of 100^3 hexes (6M tets, 1M rows): 945 us with separate index, offset and node arrays, nine divisions a
+// pair, one thread's scattered stores and three refresh passes (703 + 94 + 136 us); 500 us with the wide
+// form, 464 us with the near form.  Three blocks an SM (80 registers): two 524, four (64, spills) 521 us.
+// Loading the next pairs' conductivities a step ahead was slower (503-564 us), as was keeping the row's
+// own node out of the loads.
 constexpr uint32_t kLocalRowMax = 32;
-constexpr size_t kHeatLocalSmem = size_t(kLocalRowMax) * kBlock * sizeof(double);
+constexpr size_t heat_local_smem(uint32_t max_row) { return size_t(max_row) * (kBlock + 1) * sizeof(double); }
 
-__global__ void __launch_bounds__(kBlock) k_asm_heat_local(
-    uint32_t n_free, const uint32_t *__restrict__ row_node, const uint32_t *__restrict__ rp,
-    const uint32_t *__restrict__ adj_ptr, const uint32_t *__restrict__ adj_elem, const uint8_t *__restrict__ adj_loc,
-    const ushort4 *__restrict__ adj_off, const double *__restrict__ xyz, const uint4 *__restrict__ tets,
-    const uint32_t *__restrict__ book, const double *__restrict__ k_e, const double *__restrict__ q_e,
-    const double *__restrict__ rhoc_e, const double *__restrict__ node_t, int transient, double alpha, double dt,
-    double *__restrict__ val, double *__restrict__ b)
+template <bool NEAR>
+__global__ void __launch_bounds__(kBlock, 3) k_asm_heat_local(uint32_t n_free, uint32_t max_row,
+                                                           const uint32_t *__restrict__ rp, HeatIn h, HeatOut o)
 {
     extern __shared__ double acc_s[];
+    __shared__ double sh[32];
+    constexpr uint32_t kStride = kBlock + 1;
+    const uint32_t lane = threadIdx.x & 31u, wbase = threadIdx.x & ~31u;
     double *acc = acc_s + threadIdx.x;
-    const uint32_t stride = blockDim.x;
-    for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < n_free; r += gridDim.x * blockDim.x) {
-        const uint32_t a = row_node[r], start = rp[r], len = min(rp[r + 1] - start, kLocalRowMax);
-        for (uint32_t j = 0; j < len; j++) acc[j * stride] = 0.0;
+    double nrm[1] = {0.0};
+    for (uint32_t r0 = blockIdx.x * blockDim.x + wbase; r0 < n_free; r0 += gridDim.x * blockDim.x) {
+        const uint32_t r = r0 + lane, s = r0 >> 5;
+        const bool valid = r < n_free;
+        const uint32_t start = valid ? rp[r] : 0u, len = valid ? min(rp[r + 1] - start, max_row) : 0u;
+        const uint32_t a = valid ? h.row_node[r] : 0u;
+        for (uint32_t j = 0; j < len; j++) acc[j * kStride] = 0.0;
         double bs = 0.0;
-        for (uint32_t t = adj_ptr[a]; t < adj_ptr[a + 1]; t++) {
+        const uint32_t t1 = h.pair_ptr[s + 1];
+        uint32_t t = h.pair_ptr[s];
+        uint4 next = t < t1 ? __ldcs(h.pair + size_t(t) * 32 + lane) : make_uint4(RSG_EOD, 0, 0, 0);
+        for (; t < t1; t++) {
+            const uint4 pr = next;
+            if (t + 1 < t1) next = __ldcs(h.pair + size_t(t + 1) * 32 + lane);
+            if (pr.x == RSG_EOD) continue;
             double Ar[4], be;
-            heat_adj(t, adj_elem, adj_loc, xyz, tets, book, k_e, q_e, rhoc_e, node_t, transient, alpha, dt, Ar, be);
-            const ushort4 off4 = adj_off[t];
-            const uint16_t off[4] = {off4.x, off4.y, off4.z, off4.w};
+            uint32_t off[4];
+            heat_pair<NEAR>(h, pr, a, Ar, be, off);
             bs += be;
             for (int n = 0; n < 4; n++)
-                if (off[n] < len) acc[off[n] * stride] += Ar[n];
+                if (off[n] < len) acc[off[n] * kStride] += Ar[n];
         }
-        for (uint32_t j = 0; j < len; j++) val[start + j] = acc[j * stride];
-        b[r] = bs;
+        if (valid) o.b[r] = bs;
+        if (o.val32) {
+            for (uint32_t j = 0; j < len; j++) {
+                const double v = acc[j * kStride];
+                nrm[0] += v * v;
+            }
+            if (o.sval) {
+                const size_t base = size_t(o.slice_ptr[s]) + 4u * lane;
+                for (uint32_t j = 0; j < len; j += 4) {
+                    double v[4];
+                    for (uint32_t u = 0; u < 4; u++) v[u] = j + u < len ? acc[(j + u) * kStride] : 0.0;
+                    const size_t e = base + size_t(j >> 2) * 128u;
+                    *reinterpret_cast<double2 *>(o.sval + e) = make_double2(v[0], v[1]);
+                    *reinterpret_cast<double2 *>(o.sval + e + 2) = make_double2(v[2], v[3]);
+                    *reinterpret_cast<float4 *>(o.sval32 + e) =
+                        make_float4(__double2float_rn(v[0]), __double2float_rn(v[1]), __double2float_rn(v[2]),
+                                    __double2float_rn(v[3]));
+                }
+            }
+        }
+        __syncwarp();
+        // the CSR rows of the warp, half a warp per row: consecutive lanes store consecutive entries
+        const uint32_t sub = lane & 15u;
+        for (uint32_t i = 0; i < 32; i += 2) {
+            const uint32_t row = i + (lane >> 4);
+            const uint32_t rs = __shfl_sync(0xffffffffu, start, row), rl = __shfl_sync(0xffffffffu, len, row);
+            for (uint32_t j = sub; j < rl; j += 16) {
+                const double v = acc_s[j * kStride + wbase + row];
+                o.val[rs + j] = v;
+                if (o.val32) o.val32[rs + j] = __double2float_rn(v);
+            }
+        }
+        __syncwarp();
     }
+    if (!o.val32) return;
+    double tot[1];
+    if (grid_sum<1>(nrm, o.partials, o.ticket, sh, tot) && threadIdx.x == 0) *o.norm = sqrt(tot[0]);
+}
+
+// Pairs per 32-row slice (the longest adjacency of its rows) and the packed pairs themselves.
+__global__ void k_pair_len(uint32_t n_free, uint32_t n_slices, const uint32_t *__restrict__ row_node,
+                           const uint32_t *__restrict__ adj_ptr, uint32_t *__restrict__ len)
+{
+    for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < n_slices; s += gridDim.x * blockDim.x) {
+        uint32_t m = 0;
+        for (uint32_t r = s * 32u; r < min(n_free, s * 32u + 32u); r++)
+            m = max(m, adj_ptr[row_node[r] + 1] - adj_ptr[row_node[r]]);
+        len[s] = m;
+    }
+}
+
+// near (in: the near form is allowed by the row lengths; out: still 1 if every node number fits).
+__global__ void k_pair_near(uint32_t n_free, const uint32_t *__restrict__ row_node,
+                            const uint32_t *__restrict__ adj_ptr, const uint32_t *__restrict__ adj_elem,
+                            const uint4 *__restrict__ tets, uint32_t *near)
+{
+    bool ok = true;
+    for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < n_free; r += gridDim.x * blockDim.x) {
+        const uint32_t a = row_node[r];
+        for (uint32_t t = adj_ptr[a]; t < adj_ptr[a + 1]; t++)
+            for (int n = 0; n < 4; n++) {
+                const long long d = (long long)node_of(tets[adj_elem[t]], n) - (long long)a;
+                ok = ok && d >= -32768 && d <= 32767;
+            }
+    }
+    if (!ok) *near = 0u;
+}
+
+__global__ void k_pair_fill(uint32_t n_free, uint32_t n_slices, const uint32_t *__restrict__ row_node,
+                            const uint32_t *__restrict__ adj_ptr, const uint32_t *__restrict__ adj_elem,
+                            const uint8_t *__restrict__ adj_loc, const ushort4 *__restrict__ adj_off,
+                            const uint4 *__restrict__ tets, const uint32_t *__restrict__ pair_ptr,
+                            uint4 *__restrict__ pair, int near)
+{
+    for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < n_slices * 32u; r += gridDim.x * blockDim.x) {
+        const uint32_t s = r >> 5, t0 = pair_ptr[s], nt = pair_ptr[s + 1] - t0;
+        const uint32_t a = r < n_free ? row_node[r] : 0u;
+        const uint32_t beg = adj_ptr[a], cnt = r < n_free ? adj_ptr[a + 1] - beg : 0u;
+        for (uint32_t t = 0; t < nt; t++) {
+            uint4 v = make_uint4(RSG_EOD, 0u, 0u, 0u);
+            if (t < cnt) {
+                const ushort4 o4 = adj_off[beg + t];
+                const uint32_t off[4] = {o4.x, o4.y, o4.z, o4.w};
+                v.x = adj_elem[beg + t];
+                v.y = adj_loc[beg + t];
+                if (near) {
+                    uint32_t d[4];
+                    for (int n = 0; n < 4; n++) {
+                        v.y |= (off[n] == kNoEntry ? 63u : off[n]) << (2 + 6 * n);
+                        d[n] = (node_of(tets[v.x], n) - a) & 0xffffu;
+                    }
+                    v.z = d[0] | d[1] << 16;
+                    v.w = d[2] | d[3] << 16;
+                } else {
+                    v.z = off[0] | off[1] << 16;
+                    v.w = off[2] | off[3] << 16;
+                }
+            }
+            pair[size_t(t0 + t) * 32 + (r & 31u)] = v;
+        }
+    }
+}
+
+__global__ void k_xyz4(uint32_t n_nodes, const double *__restrict__ xyz, double4 *__restrict__ out)
+{
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_nodes; i += gridDim.x * blockDim.x)
+        out[i] = make_double4(xyz[3 * size_t(i)], xyz[3 * size_t(i) + 1], xyz[3 * size_t(i) + 2], 0.0);
 }
 
 // Row (3n+j) of the 12x6 strain-displacement matrix Be (strain order xx yy zz yz xz xy).
@@ -535,7 +732,8 @@ void free_plan(rsg_assembly *p)
 {
     if (!p) return;
     void *ptrs[] = {p->xyz, p->tets, p->tris, p->book, p->row_node, p->row_comp, p->rp, p->ci, p->adj_ptr,
-                    p->adj_elem, p->adj_loc, p->adj_off, p->tadj_ptr, p->tadj_tri, p->node_mask, p->stage};
+                    p->adj_elem, p->adj_loc, p->adj_off, p->pair,     p->pair_ptr, p->xyz4, p->tadj_ptr,
+                    p->tadj_tri, p->node_mask, p->stage};
     for (void *q : ptrs)
         if (q) cudaFree(q);
     delete p;
@@ -590,6 +788,55 @@ rsg_status create_plan(rsg_context *ctx, uint32_t n_nodes, const double *xyz, ui
         return s;
     }
     *out = p;
+    return RSG_OK;
+}
+
+// The pairs and coordinates of a heat plan in the layout of k_asm_heat; the arrays they replace are freed.
+rsg_status pack_heat_plan(rsg_context *ctx, rsg_assembly *p)
+{
+    const uint32_t n_slices = (p->n_free + 31u) / 32u;
+    const int gs = int(std::min<uint32_t>((n_slices + kBlock - 1) / kBlock, 4096u));
+    RSG_TRY(upload<uint32_t>(ctx, &p->pair_ptr, nullptr, size_t(n_slices) + 1));
+    const int gr = int(std::min<uint32_t>((n_slices * 32u + kBlock - 1) / kBlock, 65535u));
+    const uint4 *tets = reinterpret_cast<const uint4 *>(p->tets);
+    k_pair_len<<<gs, kBlock, 0, ctx->stream>>>(p->n_free, n_slices, p->row_node, p->adj_ptr, p->pair_ptr);
+    std::vector<uint32_t> ptr(size_t(n_slices) + 1);  // the last word is the near flag on its way here
+    const uint32_t near0 = p->max_row <= 32 ? 1u : 0u;
+    RSG_CHECK_CUDA(ctx, cudaMemcpyAsync(p->pair_ptr + n_slices, &near0, sizeof(near0), cudaMemcpyHostToDevice,
+                                        ctx->stream));
+    k_pair_near<<<gr, kBlock, 0, ctx->stream>>>(p->n_free, p->row_node, p->adj_ptr, p->adj_elem, tets,
+                                                p->pair_ptr + n_slices);
+    RSG_CHECK_CUDA(ctx, cudaMemcpyAsync(ptr.data(), p->pair_ptr, ptr.size() * sizeof(uint32_t), cudaMemcpyDeviceToHost,
+                                        ctx->stream));
+    RSG_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    p->near = ptr[n_slices] != 0;
+    uint64_t total = 0;
+    for (uint32_t s = 0; s <= n_slices; s++) {
+        const uint32_t len = s < n_slices ? ptr[s] : 0u;
+        ptr[s] = uint32_t(total);
+        total += len;
+    }
+    if (total > 0xffffffffull) return set_error(ctx, RSG_ERR_UNSUPPORTED, "assembly_create: too many row-tet pairs");
+    RSG_CHECK_CUDA(ctx, cudaMemcpyAsync(p->pair_ptr, ptr.data(), ptr.size() * sizeof(uint32_t), cudaMemcpyHostToDevice,
+                                        ctx->stream));
+    RSG_TRY(upload<uint4>(ctx, &p->pair, nullptr, size_t(total) * 32));
+    RSG_TRY(upload<double4>(ctx, &p->xyz4, nullptr, p->n_nodes));
+    k_pair_fill<<<gr, kBlock, 0, ctx->stream>>>(p->n_free, n_slices, p->row_node, p->adj_ptr, p->adj_elem, p->adj_loc,
+                                                reinterpret_cast<const ushort4 *>(p->adj_off), tets, p->pair_ptr,
+                                                p->pair, p->near ? 1 : 0);
+    k_xyz4<<<int(std::min<uint32_t>((p->n_nodes + kBlock - 1) / kBlock, 65535u)), kBlock, 0, ctx->stream>>>(
+        p->n_nodes, p->xyz, p->xyz4);
+    RSG_CHECK_CUDA(ctx, cudaGetLastError());
+    RSG_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    cudaFree(p->adj_ptr);
+    cudaFree(p->adj_elem);
+    cudaFree(p->adj_loc);
+    cudaFree(p->adj_off);
+    cudaFree(p->xyz);
+    p->adj_ptr = p->adj_elem = nullptr;
+    p->adj_loc = nullptr;
+    p->adj_off = nullptr;
+    p->xyz = nullptr;
     return RSG_OK;
 }
 
@@ -662,8 +909,14 @@ extern "C" {
 rsg_status rsg_assembly_create_heat(rsg_context *ctx, uint32_t n_nodes, const double *xyz, uint32_t n_tets,
                                     const uint32_t *tets, const uint32_t *book, uint32_t n_free, rsg_assembly **out)
 {
-    const rsg_status s = create_plan(ctx, n_nodes, xyz, n_tets, tets, 0, nullptr, book, 1, n_free, out);
-    if (s == RSG_OK) (*out)->kind = kPlanHeat;
+    rsg_status s = create_plan(ctx, n_nodes, xyz, n_tets, tets, 0, nullptr, book, 1, n_free, out);
+    if (s != RSG_OK) return s;
+    (*out)->kind = kPlanHeat;
+    s = pack_heat_plan(ctx, *out);
+    if (s != RSG_OK) {
+        free_plan(*out);
+        *out = nullptr;
+    }
     return s;
 }
 
@@ -729,20 +982,46 @@ rsg_status rsg_assemble_heat(rsg_context *ctx, rsg_assembly *p, const double *k_
     RSG_TRY(stage_inputs(ctx, p, memory, {p->n_tets, p->n_tets, p->n_tets, p->n_nodes},
                          {k_e, q_e, transient ? rhoc_e : nullptr, node_t}, d));
     const double alpha = time ? time->alpha : 1.0, dt = time ? time->dt : 0.0;
-    const bool local = p->max_row <= kLocalRowMax && !row_threads_forced();
-    auto kern = local ? k_asm_heat_local : k_asm_heat;
+    const HeatIn h{p->pair, p->pair_ptr, p->xyz4, reinterpret_cast<const uint4 *>(p->tets), d[0], d[1], d[2], d[3],
+                   transient ? 1 : 0, alpha, dt, p->row_node};
+    auto rows_kernel = p->near ? k_asm_heat<true> : k_asm_heat<false>;
+    auto local_kernel = p->near ? k_asm_heat_local<true> : k_asm_heat_local<false>;
+    if (p->max_row > kLocalRowMax || row_threads_forced()) {
+        const int grid = std::min(grid_for(ctx, (const void *)rows_kernel, kBlock, 0, p->n_free), kMaxGrid * 4);
+        return assemble_into(ctx, p, A, [&](double *val) {
+            rows_kernel<<<grid, kBlock, 0, ctx->stream>>>(p->n_free, p->rp, h, HeatOut{val, b_device});
+        });
+    }
     // shared memory for the plan's longest row only (15 entries on tet meshes of structured hexes)
-    const size_t smem = local ? size_t(std::max<uint32_t>(p->max_row, 1)) * kBlock * sizeof(double) : 0;
-    if (local)
-        RSG_CHECK_CUDA(ctx, cudaFuncSetAttribute(k_asm_heat_local, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 int(kHeatLocalSmem)));
-    const int grid = std::min(grid_for(ctx, (const void *)kern, kBlock, smem, p->n_free), kMaxGrid * 4);
-    return assemble_into(ctx, p, A, [&](double *val) {
-        kern<<<grid, kBlock, smem, ctx->stream>>>(p->n_free, p->row_node, p->rp, p->adj_ptr, p->adj_elem, p->adj_loc,
-                                              reinterpret_cast<const ushort4 *>(p->adj_off), p->xyz,
-                                              reinterpret_cast<const uint4 *>(p->tets), p->book, d[0], d[1], d[2],
-                                              d[3], transient ? 1 : 0, alpha, dt, val, b_device);
-    });
+    const uint32_t rows = std::max<uint32_t>(p->max_row, 1);
+    const size_t smem = heat_local_smem(rows);
+    RSG_CHECK_CUDA(ctx, cudaFuncSetAttribute(local_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             int(heat_local_smem(kLocalRowMax))));
+    const int grid = std::min(grid_for(ctx, (const void *)local_kernel, kBlock, smem, p->n_free), kMaxGrid);
+    if (!*A)
+        return assemble_into(ctx, p, A, [&](double *val) {
+            local_kernel<<<grid, kBlock, smem, ctx->stream>>>(p->n_free, rows, p->rp, h, HeatOut{val, b_device});
+        });
+    rsg_csr *M = *A;
+    if (M->n != p->n_free || M->nnz != p->nnz)
+        return set_error(ctx, RSG_ERR_INVALID_ARG, "assemble: matrix does not match the plan's pattern");
+    RSG_TRY(arena_reserve(ctx, arena_bytes(32, sizeof(double)) + arena_bytes(size_t(grid), sizeof(double))));
+    double *scal = arena_take<double>(ctx, 32);
+    HeatOut o{M->val, b_device};
+    o.val32 = M->val32;
+    o.sval = M->sval;
+    o.sval32 = M->sval32;
+    o.slice_ptr = M->slice_ptr;
+    o.partials = arena_take<double>(ctx, grid);
+    o.ticket = reinterpret_cast<unsigned int *>(scal + 16);
+    o.norm = scal;
+    RSG_CHECK_CUDA(ctx, cudaMemsetAsync(scal, 0, 32 * sizeof(double), ctx->stream));
+    local_kernel<<<grid, kBlock, smem, ctx->stream>>>(p->n_free, rows, p->rp, h, o);
+    RSG_CHECK_CUDA(ctx, cudaGetLastError());
+    RSG_CHECK_CUDA(ctx, cudaMemcpyAsync(ctx->pinned, scal, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+    RSG_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    M->norm = ctx->pinned[0];
+    return RSG_OK;
 }
 
 rsg_status rsg_assemble_stress(rsg_context *ctx, rsg_assembly *p, const double *e_mod, const double *nu,
