@@ -691,6 +691,9 @@ rsg_status run_typed(rsg_context *ctx, const CgArgs &a, double *seconds)
                             (a.persistent > 0 || a.A->n <= kPersistRows);
     bool persisted = false;
     if (persist_ok)
+        RSG_TRY(cg_resident_run(ctx, a, a.mixed ? L.g_dir32 : L.g_dir64, a.mixed ? L.g_upd32 : L.g_upd64, L.g_spmv64,
+                                &persisted));
+    if (persist_ok && !persisted)
         RSG_TRY(cg_persist_run(ctx, a, a.mixed ? L.g_dir32 : L.g_dir64, a.mixed ? L.g_upd32 : L.g_upd64, L.g_spmv64,
                                &persisted));
     if (persisted) {

@@ -35,7 +35,7 @@ struct PersistArgs {
     float *r32, *z32, *p32a, *p32b, *q32, *y32;
     double *part_dir, *part_upd, *part_chk;  // per-virtual-block partials of the three phases
     CgState *st;
-    unsigned int *bar;                       // [0] arrivals, [1] generation, [2] abort (grid_sync.cuh)
+    unsigned int *bar;                       // [0] arrivals, [2] abort (grid_sync.cuh)
     uint32_t g_dir, g_upd, g_chk;           // the graph loop's grids (virtual)
     unsigned int *err;
 };
@@ -296,11 +296,12 @@ __global__ void __launch_bounds__(kBlock) k_cg_persist(PersistArgs a)
     __syncthreads();
     int half = 0;
     bool ok = true;
+    unsigned int passed = 0;
     while (!s.done) {
         // direction + SpMV, then alpha (k_cg_dir / k_mx_dir)
         if (MIXED) dir32(a, s, half ? a.p32b : a.p32a, half ? a.p32a : a.p32b, sh);
         else dir64(a, s, half ? a.p1 : a.p0, half ? a.p0 : a.p1, sh);
-        if (!(ok = grid_barrier(a.bar, a.err))) break;
+        if (!(ok = grid_barrier_count(a.bar, a.err, passed))) break;
         {
             double tot[1];
             final_sum<1>(a.part_dir, a.g_dir, sh, tot);
@@ -324,7 +325,7 @@ __global__ void __launch_bounds__(kBlock) k_cg_persist(PersistArgs a)
         // update, then beta and the stopping rule (k_cg_update / k_mx_update)
         if (MIXED) update32<PK>(a, s, half ? a.p32a : a.p32b, sh);
         else update64<PK>(a, s, half ? a.p0 : a.p1, sh);
-        if (!(ok = grid_barrier(a.bar, a.err))) break;
+        if (!(ok = grid_barrier_count(a.bar, a.err, passed))) break;
         if (MIXED) {
             double tot[2];
             final_sum<2>(a.part_upd, a.g_upd, sh, tot);
@@ -339,7 +340,7 @@ __global__ void __launch_bounds__(kBlock) k_cg_persist(PersistArgs a)
         if (!s.done && s.need_check) {
             if (MIXED) check32<PK>(a, s, sh);
             else check64<PK>(a, sh);
-            if (!(ok = grid_barrier(a.bar, a.err))) break;
+            if (!(ok = grid_barrier_count(a.bar, a.err, passed))) break;
             double tot[2];
             final_sum<2>(a.part_chk, a.g_chk, sh, tot);
             if (threadIdx.x == 0) {
@@ -373,6 +374,23 @@ __global__ void __launch_bounds__(kBlock) k_cg_persist(PersistArgs a)
 
 }  // namespace
 
+rsg_status persist_workspace(rsg_context *ctx, double **part, unsigned int **bar)
+{
+    *part = nullptr;
+    if (!ctx->persist) {
+        if (cudaMalloc(&ctx->persist, size_t(6) * kMaxGrid * sizeof(double) + 256) != cudaSuccess) {
+            ctx->persist = nullptr;
+            (void)cudaGetLastError();
+            return RSG_OK;
+        }
+        RSG_CHECK_CUDA(ctx, cudaMemsetAsync(ctx->persist, 0, size_t(6) * kMaxGrid * sizeof(double) + 256, ctx->stream));
+    }
+    *part = ctx->persist;
+    *bar = reinterpret_cast<unsigned int *>(ctx->persist + size_t(6) * kMaxGrid);
+    RSG_CHECK_CUDA(ctx, cudaMemsetAsync(*bar, 0, 3 * sizeof(unsigned int), ctx->stream));  // no arrivals, no abort
+    return RSG_OK;
+}
+
 // Runs the loop of cg.cu's run_typed as one cooperative launch; *ran = false (and nothing launched)
 // when the device cannot make every CTA resident, and the caller takes the graph loop.
 rsg_status cg_persist_run(rsg_context *ctx, const CgArgs &a, int g_dir, int g_upd, int g_chk, bool *ran)
@@ -391,17 +409,10 @@ rsg_status cg_persist_run(rsg_context *ctx, const CgArgs &a, int g_dir, int g_up
     // every resident CTA, but no more than the largest virtual grid (measured at 65k rows: 1 CTA per SM
     // 14.4 -> 18.5 us per FP64 iteration; 2 or 5 per SM alike; at 266k rows 5 per SM beats 2)
     const int grid = std::max(1, std::min(per_sm * ctx->num_sms, std::max(g_dir, std::max(g_upd, g_chk))));
-    if (!ctx->persist) {
-        if (cudaMalloc(&ctx->persist, size_t(6) * kMaxGrid * sizeof(double) + 256) != cudaSuccess) {
-            ctx->persist = nullptr;
-            (void)cudaGetLastError();
-            return RSG_OK;
-        }
-        RSG_CHECK_CUDA(ctx, cudaMemsetAsync(ctx->persist, 0, size_t(6) * kMaxGrid * sizeof(double) + 256, ctx->stream));
-    }
-    double *part = ctx->persist;
-    unsigned int *bar = reinterpret_cast<unsigned int *>(part + size_t(6) * kMaxGrid);
-    RSG_CHECK_CUDA(ctx, cudaMemsetAsync(bar, 0, 3 * sizeof(unsigned int), ctx->stream));  // no arrivals, no abort
+    double *part = nullptr;
+    unsigned int *bar = nullptr;
+    RSG_TRY(persist_workspace(ctx, &part, &bar));
+    if (!part) return RSG_OK;
     PersistArgs pa;
     pa.S64 = sell_view<double>(a.A);
     pa.S32 = sell_view<float>(a.A);

@@ -52,6 +52,7 @@ struct rsg_csr {
     double norm = 0.0;                // ||A||_F
     uint32_t max_row = 0;             // longest row
     uint32_t max_warp_nnz = 0;        // longest 32-row chunk
+    uint32_t band = 0;                // largest |column - row|
     bool has_off16 = false;
     // SELL-32 copy (slice = 32 rows = one warp; element k of lane l at
     // slice_ptr[s] + (k/4)*128 + 4l + k%4, rows padded to a multiple of 4)

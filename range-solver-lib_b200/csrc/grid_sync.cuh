@@ -87,4 +87,37 @@ __device__ __forceinline__ bool grid_barrier(unsigned int *bar, unsigned int *er
     return ok_sh != 0;
 }
 
+// The same barrier without a hook, for kernels that pass many: bar[0] only counts arrivals and is never
+// reset, barrier number k (from 1) is passed when it reaches k gridDim.x.  An arrival is one
+// fire-and-forget release reduction instead of fence, atomic, reset, fence and generation update in
+// series; waiters poll the count itself.  148 CTAs, 40^3 CG: 4.9 -> 2.3 and 3.0 -> 1.1 us (the first of an
+// iteration's two waits also absorbs the CTAs' different loads).  `passed` is the caller's per-thread count of barriers so far.
+__device__ __forceinline__ bool grid_barrier_count(unsigned int *bar, unsigned int *err, unsigned int &passed)
+{
+    __shared__ int ok_sh;
+    const unsigned int want = ++passed * gridDim.x;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int ok = 1;
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
+        uint32_t t = 0;
+        while (int(ld_acquire(bar) - want) < 0) {
+            if (++t >= kBarrierPolls) {
+                ok = 0;
+                atomicExch(bar + 2, 1u);
+                if (err) atomicOr(err, 1u);
+                break;
+            }
+            if ((t & 1023u) == 0 && ld_acquire(bar + 2) != 0) {
+                ok = 0;
+                break;
+            }
+            if (t > 4096) __nanosleep(64);
+        }
+        ok_sh = ok;
+    }
+    __syncthreads();
+    return ok_sh != 0;
+}
+
 }  // namespace rsg

@@ -99,6 +99,10 @@ rsg_status cg_run(rsg_context *ctx, const CgArgs &a, double *seconds);
 // The CG loop as one persistent cooperative kernel (cg_persist.cu), bit for bit the graph loop's
 // results with the same grids; *ran = false when it could not be launched (nothing was).
 rsg_status cg_persist_run(rsg_context *ctx, const CgArgs &a, int g_dir, int g_upd, int g_chk, bool *ran);
+// The same loop with the matrix resident in shared memory (cg_resident.cu), likewise bit for bit.
+rsg_status cg_resident_run(rsg_context *ctx, const CgArgs &a, int g_dir, int g_upd, int g_chk, bool *ran);
+// The context's partial sums (6 kMaxGrid doubles; null: none could be had) and zeroed barrier words.
+rsg_status persist_workspace(rsg_context *ctx, double **part, unsigned int **bar);
 // Rows up to which the loop runs persistent by default (conf.persistent = 0): measured per CG
 // iteration, graph loop -> persistent, FP64 / mixed: 8k rows 17.3 -> 12.2 / 17.1 -> 11.3 us;
 // 65k rows 18.4 -> 14.1 / 18.4 -> 12.4 us; 266k rows 29.0 -> 36.9 / 24.5 -> 24.4 us.
