@@ -114,12 +114,16 @@ __device__ __forceinline__ double2 row_product(const MView &M, uint32_t row, boo
 
 // Column sums over the grid: each lane holds NQ quantities for its column pair.
 // Returns true in the last block to finish; tot[q*K + j] then holds the totals
-// (valid in every thread of that block).  Fixed order: lanes, warps, blocks.
+// (valid in every thread of that block).  Fixed order: lanes, warps, blocks -- the last block's
+// kBlock / NV threads per quantity each add every (kBlock / NV)-th block, eight loads in flight,
+// then one adds their sums.  (One thread per quantity walking all blocks' partials through L2 took
+// 30 us of a 60^3, k = 8 iteration.)
 template <int K, int NQ>
 __device__ __forceinline__ bool grid_cols_sum(double2 (&v)[NQ], double *partials, unsigned int *ticket, double *sh,
                                               double *tot)
 {
     constexpr int LPR = Map<K>::LPR, NV = NQ * K;
+    __shared__ double parts[kBlock];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
 #pragma unroll
     for (int q = 0; q < NQ; q++)
@@ -146,10 +150,19 @@ __device__ __forceinline__ bool grid_cols_sum(double2 (&v)[NQ], double *partials
     __syncthreads();
     if (!is_last) return false;
     __threadfence();
-    for (int t = threadIdx.x; t < NV; t += blockDim.x) {
+    constexpr int kParts = kBlock / NV;
+    if (threadIdx.x < kParts * NV) {
+        const int t = threadIdx.x % NV;
         double a = 0.0;
-        for (unsigned int b = 0; b < gridDim.x; b++) a += __ldcg(&partials[size_t(b) * NV + t]);
-        tot[t] = a;
+#pragma unroll 8
+        for (unsigned int b = threadIdx.x / NV; b < gridDim.x; b += kParts) a += __ldcg(&partials[size_t(b) * NV + t]);
+        parts[threadIdx.x] = a;
+    }
+    __syncthreads();
+    if (threadIdx.x < NV) {
+        double a = 0.0;
+        for (int i = 0; i < kParts; i++) a += parts[i * NV + threadIdx.x];
+        tot[threadIdx.x] = a;
     }
     __syncthreads();
     if (threadIdx.x == 0) *ticket = 0u;
@@ -177,15 +190,23 @@ __global__ void k_mr_unpack(uint32_t n, uint32_t k, uint32_t K, const double *__
     }
 }
 
-__device__ void refresh_all_done(MrState *st)
+// The last block's step after a reduction: column j advances in thread j (its divisions and square
+// roots run beside the other columns'), then the flags of all columns.
+template <class F>
+__device__ __forceinline__ void each_column(MrState *st, F f)
 {
-    int all = 1, chk = 0;
-    for (uint32_t j = 0; j < st->k; j++) {
-        all &= st->col[j].done;
-        chk |= st->col[j].need_check;
+    if (threadIdx.x < st->k) f(threadIdx.x, st->col[threadIdx.x]);
+    __threadfence_block();
+    if (threadIdx.x < 32) {
+        __syncwarp();
+        const bool mine = threadIdx.x < st->k;
+        const bool all = __all_sync(0xffffffffu, !mine || st->col[threadIdx.x].done);
+        const bool chk = __any_sync(0xffffffffu, mine && st->col[threadIdx.x].need_check);
+        if (threadIdx.x == 0) {
+            st->all_done = all;
+            st->any_check = chk;
+        }
     }
-    st->all_done = all;
-    st->any_check = chk;
 }
 
 // rows visited by this warp-group pass: grid-stride over groups of RPW rows
@@ -226,9 +247,8 @@ __global__ void __launch_bounds__(kBlock) k_mr_init(MView M, const double *__res
             acc[2].y += rv.y * zv.y;
         }
     }
-    if (grid_cols_sum<K, 3>(acc, partials, &st->ticket[0], sh, tot) && threadIdx.x == 0) {
-        for (uint32_t j = 0; j < st->k; j++) {
-            MrCol &c = st->col[j];
+    if (grid_cols_sum<K, 3>(acc, partials, &st->ticket[0], sh, tot))
+        each_column(st, [&](uint32_t j, MrCol &c) {
             c.bn = sqrt(tot[j]);
             c.rn = sqrt(tot[K + j]);
             c.rho = tot[2 * K + j];
@@ -248,9 +268,7 @@ __global__ void __launch_bounds__(kBlock) k_mr_init(MView M, const double *__res
                 c.done = 1;
                 c.status = RSG_BREAKDOWN;
             }
-        }
-        refresh_all_done(st);
-    }
+        });
 }
 
 // p = z + beta p_old (own row, and gathered on the fly), q = A p; per column p^T q -> alpha
@@ -282,12 +300,11 @@ __global__ void __launch_bounds__(kBlock) k_mr_dir(MView M, const double *__rest
             acc[0].y += pv.y * qv.y;
         }
     }
-    if (grid_cols_sum<K, 1>(acc, partials, &st->ticket[1], sh, tot) && threadIdx.x == 0) {
-        for (uint32_t j = 0; j < st->k; j++) {
-            MrCol &c = st->col[j];
+    if (grid_cols_sum<K, 1>(acc, partials, &st->ticket[1], sh, tot))
+        each_column(st, [&](uint32_t j, MrCol &c) {
             if (c.done) {
                 c.alpha = 0.0;
-                continue;
+                return;
             }
             c.pq = tot[j];
             if (!(c.pq > 0.0) || !isfinite(c.pq)) {
@@ -297,9 +314,7 @@ __global__ void __launch_bounds__(kBlock) k_mr_dir(MView M, const double *__rest
             } else {
                 c.alpha = c.rho / c.pq;
             }
-        }
-        refresh_all_done(st);
-    }
+        });
 }
 
 // x += alpha p, r -= alpha q, z = D r for the active columns; r^T z, ||r||^2 -> beta, stop tests.
@@ -342,25 +357,22 @@ __global__ void __launch_bounds__(kBlock) k_mr_update(uint32_t n, const double *
         acc[1].x += rv.x * rv.x;
         acc[1].y += rv.y * rv.y;
     }
-    if (grid_cols_sum<K, 2>(acc, partials, &st->ticket[2], sh, tot) && threadIdx.x == 0) {
-        for (uint32_t j = 0; j < st->k; j++) {
-            MrCol &c = st->col[j];
-            if (c.done) continue;
+    if (grid_cols_sum<K, 2>(acc, partials, &st->ticket[2], sh, tot))
+        each_column(st, [&](uint32_t j, MrCol &c) {
+            if (c.done) return;
             c.it++;
             const double rho_new = tot[j];
             c.rn = sqrt(tot[K + j]);
             if (!isfinite(c.rn) || !isfinite(rho_new)) {
                 c.done = 1;
                 c.status = RSG_BREAKDOWN;
-                continue;
+                return;
             }
             c.beta = rho_new / c.rho;
             c.rho = rho_new;
             if (c.rn <= st->rtol * c.bn) c.need_check = 1;
             else if (c.it >= st->max_it) c.done = 1;  // status stays NOT_CONVERGED
-        }
-        refresh_all_done(st);
-    }
+        });
 }
 
 // For the columns whose recurrence residual met rtol: the FP64 true residual
@@ -403,10 +415,9 @@ __global__ void __launch_bounds__(kBlock) k_mr_check(MView M, const double *__re
             acc[1].y += rv.y * rv.y;
         }
     }
-    if (grid_cols_sum<K, 2>(acc, partials, &st->ticket[3], sh, tot) && threadIdx.x == 0) {
-        for (uint32_t j = 0; j < st->k; j++) {
-            MrCol &c = st->col[j];
-            if (!c.need_check) continue;
+    if (grid_cols_sum<K, 2>(acc, partials, &st->ticket[3], sh, tot))
+        each_column(st, [&](uint32_t j, MrCol &c) {
+            if (!c.need_check) return;
             c.need_check = 0;
             c.checks++;
             c.rn = sqrt(tot[K + j]);
@@ -424,9 +435,7 @@ __global__ void __launch_bounds__(kBlock) k_mr_check(MView M, const double *__re
                     c.status = RSG_BREAKDOWN;
                 }
             }
-        }
-        refresh_all_done(st);
-    }
+        });
 }
 
 // per column ||b - A x|| / ||b|| of the final x
@@ -450,12 +459,11 @@ __global__ void __launch_bounds__(kBlock) k_mr_true(MView M, const double *__res
             acc[1].y += bv.y * bv.y;
         }
     }
-    if (grid_cols_sum<K, 2>(acc, partials, &st->ticket[4], sh, tot) && threadIdx.x == 0) {
-        for (uint32_t j = 0; j < st->k; j++) {
+    if (grid_cols_sum<K, 2>(acc, partials, &st->ticket[4], sh, tot))
+        each_column(st, [&](uint32_t j, MrCol &c) {
             const double bn = sqrt(tot[K + j]), rn = sqrt(tot[j]);
-            st->col[j].relres = bn > 0.0 ? rn / bn : rn;
-        }
-    }
+            c.relres = bn > 0.0 ? rn / bn : rn;
+        });
 }
 
 __global__ void k_mr_tail(MrState *st, cudaGraphConditionalHandle h, int use_cond)
