@@ -8,9 +8,11 @@
 //   update: x += alpha p, r -= alpha q, z = P r (Jacobi / block Jacobi /
 //           none, src/rmatrixpreconditioner.cpp:150-190), partial r^T z,
 //           ||r||^2, ||x||^2  -> last block: beta, error, stopping rule
-// plus a check kernel that is a no-op unless the recurrence residual has
-// reached the tolerance, in which case it recomputes the FP64 true residual
-// b - A x (stop_rule TRUE_RELRES).
+// plus, after every few iterations, a check kernel that is a no-op unless the
+// recurrence residual has reached the tolerance, in which case it recomputes the
+// FP64 true residual b - A x (stop_rule TRUE_RELRES).  An update that asks for
+// the check turns the rest of its body's kernels into no-ops, so the check sees
+// the state of that update as if it had followed at once.
 //
 // Mixed precision (reliable updates, van der Vorst & Ye 2000): the matrix is
 // read as FP32 values with 16-bit column offsets, vectors are FP32 scaled by
@@ -20,7 +22,8 @@
 // FP64 solution x and restarts the recurrence from the true residual while
 // keeping the search direction.
 //
-// The loop runs on the device: the kernels of two iterations form the body of
+// The loop runs on the device: the kernels of kBodyIterations iterations (two with
+// the multilevel preconditioner, whose cycle needs the check before it) form the body of
 // a CUDA graph `while` node whose condition the tail kernel sets from the
 // device state, so a whole solve is a single graph launch.  The tail kernel
 // also counts bodies and forces termination past a hard limit, so the loop
@@ -40,6 +43,34 @@ namespace rsg {
 // (Software-pipelining the next slice's matrix loads needed 64-80 registers with spills
 // and measured 38.9-44.5 us.)
 constexpr int kDirMinBlocks32 = 8;
+// CG iterations per body of the loop graph.  Each body ends with a check and a tail launch (2 + 1.5 us and the
+// while node's own step); an update that asks for a check idles the rest of its body (2 us a launch).  2 -> 4
+// -> 8 -> 16 iterations, ms a solve: 220k rows FP64 11.37, 11.06, 10.60, 10.43; 1M rows 45.96, 44.95, 44.29,
+// 44.11; every body iteration is also two graph nodes to build per solve.
+constexpr int kBodyIterations = 8;
+constexpr int kUpdateBlocksPerSm = 3;
+
+// The grid reduction of a loop kernel and, in its last block, the step of the state that it leads to.  The
+// step works on a shared-memory copy that the block loads beside the partials and stores at the end: on the
+// state in global memory its loads, kept in order by its stores, cost a round trip to L2 each (a last block
+// of 4 to 5 us; 220k rows FP64 23.9 -> 21.8 us per iteration).  Leaving the sums to the next kernel, every
+// block adding all partials itself and stepping its own copy of the state, was no faster: 22.0 us, 1M rows
+// 53.8 -> 56.2 us.
+template <int NV, class F>
+__device__ __forceinline__ void state_step(CgState *st, double (&v)[NV], double *partials, int ticket, double *sh, F step)
+{
+    __shared__ CgState s;
+    auto load = [&]() {
+        for (uint32_t w = threadIdx.x; w < kStateWords; w += blockDim.x)
+            reinterpret_cast<uint32_t *>(&s)[w] = __ldcg(reinterpret_cast<const uint32_t *>(st) + w);
+    };
+    double tot[NV];
+    if (!grid_sum<NV>(v, partials, &st->ticket[ticket], sh, tot, load)) return;
+    if (threadIdx.x == 0) step(&s, tot);
+    __syncthreads();
+    for (uint32_t w = threadIdx.x; w < kStateWords; w += blockDim.x)
+        reinterpret_cast<uint32_t *>(st)[w] = reinterpret_cast<const uint32_t *>(&s)[w];
+}
 
 // ---------------- FP64 kernels ----------------
 
@@ -125,14 +156,16 @@ __global__ void __launch_bounds__(kBlock) k_cg_prec(uint32_t n, uint32_t w, cons
 
 template <int RPW>
 __global__ void __launch_bounds__(kBlock) k_cg_dir(Csr<double> M, Sell<double> S, int use_sell, const double *__restrict__ z,
-                                                   const double *__restrict__ p_old, double *__restrict__ p_new,
-                                                   double *__restrict__ q, double *partials, CgState *st)
+                                                   double *p0, double *p1, double *__restrict__ q, double *partials,
+                                                   CgState *st)
 {
     pdl_wait();
     pdl_release();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ double sh[32];
-    if (st->done) return;
+    if (st->done || st->need_check) return;
+    const double *__restrict__ p_old = st->pcur ? p1 : p0;
+    double *__restrict__ p_new = st->pcur ? p0 : p1;
     const double beta = st->beta;
     double acc[1] = {0.0};
     auto gx = [&](uint32_t c) { return fma(beta, p_old[c], z[c]); };
@@ -143,25 +176,27 @@ __global__ void __launch_bounds__(kBlock) k_cg_dir(Csr<double> M, Sell<double> S
         acc[0] += p * v;
     };
     for_rows_any<double, RPW>(M, S, use_sell != 0, gx, epi, smem_raw, &st->ticket[7], true);
-    double tot[1];
-    if (grid_sum<1>(acc, partials, &st->ticket[0], sh, tot) && threadIdx.x == 0) {
-        const double pq = clamp_pq(tot[0], st->eps);
-        st->pq = pq;
-        st->rho = st->rho_new;
-        st->alpha = st->rho / pq;
-    }
+    state_step<1>(st, acc, partials, 0, sh, [](CgState *s, const double *tot) {
+        const double pq = clamp_pq(tot[0], s->eps);
+        s->pq = pq;
+        s->rho = s->rho_new;
+        s->alpha = s->rho / pq;
+        s->pcur ^= 1u;
+    });
 }
 
 template <int PK>
 __global__ void __launch_bounds__(kBlock) k_cg_update(uint32_t n, uint32_t w, const double *__restrict__ d,
-                                                      const double *__restrict__ p, const double *__restrict__ q,
-                                                      double *__restrict__ x, double *__restrict__ r,
-                                                      double *__restrict__ z, double *partials, CgState *st)
+                                                      const double *p0, const double *p1,
+                                                      const double *__restrict__ q, double *__restrict__ x,
+                                                      double *__restrict__ r, double *__restrict__ z,
+                                                      double *partials, CgState *st)
 {
     pdl_wait();
     pdl_release();
     __shared__ double sh[96];
-    if (st->done) return;
+    if (st->done || st->need_check) return;
+    const double *__restrict__ p = st->pcur ? p1 : p0;
     const double alpha = st->alpha;
     double acc[3] = {0.0, 0.0, 0.0};
     const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
@@ -220,9 +255,8 @@ __global__ void __launch_bounds__(kBlock) k_cg_update(uint32_t n, uint32_t w, co
             acc[0] += prec_group64<PK>(g, w, d, rl, z);
         }
     }
-    double tot[3];
-    if (grid_sum<3>(acc, partials, &st->ticket[1], sh, tot) && threadIdx.x == 0)
-        finalize_update64(st, tot[0], tot[1], tot[2]);
+    state_step<3>(st, acc, partials, 1, sh,
+                  [](CgState *s, const double *tot) { finalize_update64(s, tot[0], tot[1], tot[2]); });
 }
 
 template <int RPW, int PK>
@@ -252,11 +286,10 @@ __global__ void __launch_bounds__(kBlock) k_cg_check(Csr<double> M, Sell<double>
         }
     };
     for_rows_any<double, RPW>(M, S, use_sell != 0, gx, epi, smem_raw, &st->ticket[7], true);
-    double tot[2];
-    if (grid_sum<2>(acc, partials, &st->ticket[2], sh, tot) && threadIdx.x == 0) {
-        if (PK == 2) st->check_rn = sqrt(tot[1]);
-        else finalize_check64(st, tot[0], sqrt(tot[1]));
-    }
+    state_step<2>(st, acc, partials, 2, sh, [](CgState *s, const double *tot) {
+        if (PK == 2) s->check_rn = sqrt(tot[1]);
+        else finalize_check64(s, tot[0], sqrt(tot[1]));
+    });
 }
 
 // ---------------- mixed-precision kernels ----------------
@@ -325,15 +358,17 @@ __global__ void __launch_bounds__(kBlock) k_mx_prec(uint32_t n, uint32_t w, cons
 
 template <int RPW>
 __global__ void __launch_bounds__(kBlock, kDirMinBlocks32) k_mx_dir(Csr<float> M, Sell<float> S, int use_sell, const float *__restrict__ z,
-                                                   const float *__restrict__ p_old, float *__restrict__ p_new,
-                                                   float *__restrict__ q, double *__restrict__ x,
-                                                   float *__restrict__ y, double *partials, CgState *st)
+                                                   float *p0, float *p1, float *__restrict__ q,
+                                                   double *__restrict__ x, float *__restrict__ y, double *partials,
+                                                   CgState *st)
 {
     pdl_wait();
     pdl_release();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ double sh[32];
-    if (st->done) return;
+    if (st->done || st->need_check) return;
+    const float *__restrict__ p_old = st->pcur ? p1 : p0;
+    float *__restrict__ p_new = st->pcur ? p0 : p1;
     const float beta = float(st->beta);
     const int fold = st->fold;
     const double inv_sigma = 1.0 / st->sigma;
@@ -351,27 +386,29 @@ __global__ void __launch_bounds__(kBlock, kDirMinBlocks32) k_mx_dir(Csr<float> M
     };
     for_rows_any<float, RPW>(M, S, use_sell != 0, gx, epi, smem_raw, &st->ticket[7], st->evict_first32 != 0);
     double acc[1] = {pq.value()};
-    double tot[1];
-    if (grid_sum<1>(acc, partials, &st->ticket[0], sh, tot) && threadIdx.x == 0) {
+    state_step<1>(st, acc, partials, 0, sh, [](CgState *s, const double *tot) {
         double d = tot[0];
         if (d == 0.0 || !isfinite(d)) d = (d == 0.0) ? 1e-300 : d;
-        st->pq = d;
-        st->rho = st->rho_new;
-        st->alpha = st->rho / d;
-        st->fold = 0;
-    }
+        s->pq = d;
+        s->rho = s->rho_new;
+        s->alpha = s->rho / d;
+        s->fold = 0;
+        s->pcur ^= 1u;
+    });
 }
 
 template <int PK>
 __global__ void __launch_bounds__(kBlock) k_mx_update(uint32_t n, uint32_t w, const float *__restrict__ d,
-                                                      const float *__restrict__ p, const float *__restrict__ q,
-                                                      float *__restrict__ y, float *__restrict__ r,
-                                                      float *__restrict__ z, double *partials, CgState *st)
+                                                      const float *p0, const float *p1,
+                                                      const float *__restrict__ q, float *__restrict__ y,
+                                                      float *__restrict__ r, float *__restrict__ z, double *partials,
+                                                      CgState *st)
 {
     pdl_wait();
     pdl_release();
     __shared__ double sh[64];
-    if (st->done) return;
+    if (st->done || st->need_check) return;
+    const float *__restrict__ p = st->pcur ? p1 : p0;
     const float alpha = float(st->alpha);
     Dot2 rz, rr;
     const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
@@ -439,9 +476,8 @@ __global__ void __launch_bounds__(kBlock) k_mx_update(uint32_t n, uint32_t w, co
         }
     }
     double acc[2] = {rz.value(), rr.value()};
-    double tot[2];
-    if (grid_sum<2>(acc, partials, &st->ticket[1], sh, tot) && threadIdx.x == 0)
-        finalize_update_mixed(st, tot[0], tot[1]);
+    state_step<2>(st, acc, partials, 1, sh,
+                  [](CgState *s, const double *tot) { finalize_update_mixed(s, tot[0], tot[1]); });
 }
 
 template <int RPW, int PK>
@@ -477,11 +513,10 @@ __global__ void __launch_bounds__(kBlock) k_mx_check(Csr<double> M, Sell<double>
     };
     for_rows_any<double, RPW>(M, S, use_sell != 0, gx, epi, smem_raw, &st->ticket[7], true);
     double acc[2] = {rz.value(), rr[0]};
-    double tot[2];
-    if (grid_sum<2>(acc, partials, &st->ticket[2], sh, tot) && threadIdx.x == 0) {
-        if (PK >= 2) st->check_rn = sqrt(tot[1]);  // the preconditioner pass that follows finalizes
-        else finalize_check_mixed(st, tot[0], sqrt(tot[1]));
-    }
+    state_step<2>(st, acc, partials, 2, sh, [](CgState *s, const double *tot) {
+        if (PK >= 2) s->check_rn = sqrt(tot[1]);  // the preconditioner pass that follows finalizes
+        else finalize_check_mixed(s, tot[0], sqrt(tot[1]));
+    });
 }
 
 __global__ void k_mx_fold(uint32_t n, double *__restrict__ x, float *__restrict__ y, const CgState *st)
@@ -565,7 +600,7 @@ void launch_init(rsg_context *ctx, const CgArgs &a, const Launch &L)
 
 template <int RPW, int PK>
 void launch_body(rsg_context *ctx, const CgArgs &a, const Launch &L, cudaGraphConditionalHandle h, int use_cond,
-                 bool pdl)
+                 bool pdl, int iterations)
 {
     const uint32_t n = a.A->n;
     const Csr<double> M64 = view<double>(a.A, true);
@@ -573,41 +608,45 @@ void launch_body(rsg_context *ctx, const CgArgs &a, const Launch &L, cudaGraphCo
     const Sell<float> S32 = sell_view<float>(a.A);
     const int us = a.A->use_sell;
     cudaStream_t st = ctx->stream;
-    if (!a.mixed) {
-        for (int half = 0; half < 2; half++) {
-            double *po = half ? a.p1 : a.p0, *pn = half ? a.p0 : a.p1;
-            launch_k(st, pdl, k_cg_dir<RPW>, L.g_dir64, kBlock, L.s64, M64, S64, us, a.z, po, pn, a.q, a.partials,
-                     a.st);
-            launch_k(st, pdl, k_cg_update<PK>, L.g_upd64, kBlock, 0, n, a.P.w, a.P.d, pn, a.q, a.x, a.r, a.z,
-                     a.partials, a.st);
+    auto check = [&]() {
+        if (!a.mixed) {
             launch_k(st, pdl, k_cg_check<RPW, PK>, L.g_spmv64, kBlock, L.s64, M64, S64, us, a.P.d, a.b, a.x, a.r,
                      a.z, a.partials, a.st);
             if (PK == 2)
                 launch_k(st, pdl, k_cg_prec<PK>, L.g_vec, kBlock, 0, n, a.P.w, a.P.d, a.r, a.z, a.partials, a.st, 1);
-        }
-    } else {
-        const Csr<float> M32 = view<float>(a.A, true);
-        for (int half = 0; half < 2; half++) {
-            float *po = half ? a.p32b : a.p32a, *pn = half ? a.p32a : a.p32b;
-            launch_k(st, pdl, k_mx_dir<RPW>, L.g_dir32, kBlock, L.s32, M32, S32, us, a.z32, po, pn, a.q32, a.x,
-                     a.y32, a.partials, a.st);
+        } else {
             float *zx = PK == 3 ? a.amg_x0 : a.z32;  // multilevel: the V-cycle's first smoothing step
-            launch_k(st, pdl, k_mx_update<PK>, L.g_upd32, kBlock, 0, n, a.P.w, a.P.d32, pn, a.q32, a.y32, a.r32,
-                     zx, a.partials, a.st);
             launch_k(st, pdl, k_mx_check<RPW, PK>, L.g_spmv64, kBlock, L.s64, M64, S64, us, a.P.d32, a.b, a.x,
                      a.y32, a.r32, zx, a.partials, a.st);
             if (PK == 2)
                 launch_k(st, pdl, k_mx_prec<PK>, L.g_vec, kBlock, 0, n, a.P.w, a.P.d32, (const double *)nullptr,
                          a.r32, a.z32, a.partials, a.st, 1);
-            if (PK == 3)
+        }
+    };
+    const Csr<float> M32 = view<float>(a.A, true);
+    for (int it = 0; it < iterations; it++) {
+        if (!a.mixed) {
+            launch_k(st, pdl, k_cg_dir<RPW>, L.g_dir64, kBlock, L.s64, M64, S64, us, a.z, a.p0, a.p1, a.q, a.partials,
+                     a.st);
+            launch_k(st, pdl, k_cg_update<PK>, L.g_upd64, kBlock, 0, n, a.P.w, a.P.d, a.p0, a.p1, a.q, a.x, a.r, a.z,
+                     a.partials, a.st);
+        } else {
+            launch_k(st, pdl, k_mx_dir<RPW>, L.g_dir32, kBlock, L.s32, M32, S32, us, a.z32, a.p32a, a.p32b, a.q32,
+                     a.x, a.y32, a.partials, a.st);
+            launch_k(st, pdl, k_mx_update<PK>, L.g_upd32, kBlock, 0, n, a.P.w, a.P.d32, a.p32a, a.p32b, a.q32, a.y32,
+                     a.r32, PK == 3 ? a.amg_x0 : a.z32, a.partials, a.st);
+            if (PK == 3) {  // the cycle works on the checked residual and finalizes the check
+                check();
                 amg_vcycle(ctx, a.A, a.amg, a.r32, a.amg_x0, a.q32, a.z32, a.amg_sweeps, a.partials,
                            &a.st->ticket[5], a.st, 1, nullptr, pdl);
+            }
         }
     }
+    if (PK != 3) check();
     launch_k(st, pdl, k_tail, 1, 32, 0, a.st, h, use_cond);
 }
 
-// The solve loop as a graph: one while node whose body is two CG iterations (launch_body)
+// The solve loop as a graph: one while node whose body is kBodyIterations CG iterations (launch_body)
 // captured from the stream.  On failure nothing is left allocated.
 template <int RPW, int PK>
 rsg_status build_loop_graph(rsg_context *ctx, const CgArgs &a, const Launch &L, bool pdl, cudaGraph_t *graph_out,
@@ -641,7 +680,7 @@ rsg_status build_loop_graph(rsg_context *ctx, const CgArgs &a, const Launch &L, 
             s = set_error(ctx, RSG_ERR_CUDA, "capture into the loop body failed");
             break;
         }
-        launch_body<RPW, PK>(ctx, a, L, h, 1, pdl);
+        launch_body<RPW, PK>(ctx, a, L, h, 1, pdl, PK == 3 ? 2 : kBodyIterations);
         cudaGraph_t captured = nullptr;
         cudaError_t e = cudaStreamEndCapture(ctx->stream, &captured);
         if (e != cudaSuccess) {
@@ -676,7 +715,11 @@ rsg_status run_typed(rsg_context *ctx, const CgArgs &a, double *seconds)
     (void)chunk_threads;
     L.g_spmv64 = spmv_grid(ctx, a.A, (const void *)k_cg_dir<RPW>, L.s64, RPW);
     L.g_spmv32 = spmv_grid(ctx, a.A, (const void *)k_mx_dir<RPW>, L.s32, RPW);
-    L.g_vec = std::min(grid_for(ctx, (const void *)k_cg_update<PK>, kBlock, 0, a.A->n), kMaxGrid);
+    // the update's grid: a block for every 256 pairs (FP64) or quadruples (FP32) of rows, at most three an SM --
+    // every block adds a ticket and partials (220k rows, us per iteration: FP64 20.6 with 8 blocks an SM, 20.2
+    // with 3, 21.7 with 2; FP32 20.8 with a block per 256 rows, 18.2 with 296 blocks)
+    L.g_vec = std::min(grid_for(ctx, (const void *)k_cg_update<PK>, kBlock, 0, a.A->n / (a.mixed ? 4 : 2)),
+                       kUpdateBlocksPerSm * ctx->num_sms);
     const rsg_csr::Tune &T = a.A->tune;
     L.g_dir64 = T.valid && T.g_dir64 > 0 ? T.g_dir64 : L.g_spmv64;
     L.g_dir32 = T.valid && T.g_dir32 > 0 ? T.g_dir32 : L.g_spmv32;
@@ -728,7 +771,7 @@ rsg_status run_typed(rsg_context *ctx, const CgArgs &a, double *seconds)
         const uint32_t bodies_per_poll = std::max<uint32_t>(1, a.check_interval / 2);
         int32_t *done_h = reinterpret_cast<int32_t *>(ctx->pinned);
         for (;;) {
-            for (uint32_t k = 0; k < bodies_per_poll; k++) launch_body<RPW, PK>(ctx, a, L, 0, 0, pdl_for(a.A, a.mixed));
+            for (uint32_t k = 0; k < bodies_per_poll; k++) launch_body<RPW, PK>(ctx, a, L, 0, 0, pdl_for(a.A, a.mixed), 2);
             RSG_CHECK_CUDA(ctx, cudaGetLastError());
             RSG_CHECK_CUDA(ctx, cudaMemcpyAsync(done_h, &a.st->done, sizeof(int32_t), cudaMemcpyDeviceToHost,
                                                 ctx->stream));
@@ -788,8 +831,8 @@ rsg_status profile_typed(rsg_context *ctx, const rsg_csr *A, int kernel, uint32_
     h.eps = 1e-300;
     h.max_it = 0xffffffffu;
     h.stop_rule = RSG_STOP_TRUE_RELRES;
-    h.rtol = 0.0;
-    h.delta = 0.0;
+    h.rtol = h.delta = -1.0;  // never asks for a check: the update would then be a no-op
+    h.max_r = 1.0;
     h.bn = 1.0;
     RSG_CHECK_CUDA(ctx, cudaMemcpyAsync(st, &h, sizeof(h), cudaMemcpyHostToDevice, ctx->stream));
     const size_t s64 = A->use_sell ? 0 : tma_smem<double>(), s32 = A->use_sell ? 0 : tma_smem<float>();
@@ -820,11 +863,11 @@ rsg_status profile_typed(rsg_context *ctx, const rsg_csr *A, int kernel, uint32_
                                                              v32[4], partials, st);
             break;
         case RSG_KERNEL_CG_UPDATE_FP64:
-            k_cg_update<1><<<gv64, kBlock, 0, ctx->stream>>>(n, 1, v64[4], v64[0], v64[1], v64[2], v64[3], v64[4],
+            k_cg_update<1><<<gv64, kBlock, 0, ctx->stream>>>(n, 1, v64[4], v64[0], v64[0], v64[1], v64[2], v64[3], v64[4],
                                                           partials, st);
             break;
         case RSG_KERNEL_CG_UPDATE_MIXED:
-            k_mx_update<1><<<gv32, kBlock, 0, ctx->stream>>>(n, 1, v32[5], v32[0], v32[1], v32[2], v32[3], v32[4],
+            k_mx_update<1><<<gv32, kBlock, 0, ctx->stream>>>(n, 1, v32[5], v32[0], v32[0], v32[1], v32[2], v32[3], v32[4],
                                                           partials, st);
             break;
         case RSG_KERNEL_SPMV_FP64:

@@ -160,31 +160,50 @@ __device__ __forceinline__ void block_sum(double (&v)[NV], double *sh)
     __syncthreads();
 }
 
+struct NoLoad {
+    __device__ void operator()() const {}
+};
+
 // Deterministic grid reduction: every block writes NV partials, the last block
 // to finish sums them in block order and returns true (in all its threads).
-// `total` (valid in thread 0 of the last block) receives the sums.
-template <int NV>
+// `total` (valid in thread 0 of the last block) receives the sums.  `load` runs in the last block beside
+// its reading of the partials.
+template <int NV, class LOAD = NoLoad>
 __device__ __forceinline__ bool grid_sum(double (&v)[NV], double *partials, unsigned int *ticket, double *sh,
-                                         double (&total)[NV])
+                                         double (&total)[NV], LOAD load = LOAD())
 {
     block_sum<NV>(v, sh);
     __shared__ bool is_last;
     if (threadIdx.x == 0) {
 #pragma unroll
         for (int k = 0; k < NV; k++) partials[size_t(blockIdx.x) * NV + k] = v[k];
-        __threadfence();
-        unsigned int t = atomicAdd(ticket, 1u);
+        // one acquire-release atomic: the partials are visible before it, the others' after it (with a
+        // fence on either side a 220k-row update kernel took 1 us longer)
+        unsigned int t;
+        asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(t) : "l"(ticket) : "memory");
         is_last = (t == gridDim.x - 1);
     }
     __syncthreads();
     if (!is_last) return false;
-    __threadfence();
+    load();
     double acc[NV];
 #pragma unroll
     for (int k = 0; k < NV; k++) acc[k] = 0.0;
-    for (unsigned int b = threadIdx.x; b < gridDim.x; b += blockDim.x)
+    // four rounds of loads in flight (added in the same order)
+    for (unsigned int b0 = threadIdx.x; b0 < gridDim.x; b0 += 4 * blockDim.x) {
+        double w[4][NV];
 #pragma unroll
-        for (int k = 0; k < NV; k++) acc[k] += __ldcg(&partials[size_t(b) * NV + k]);
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int k = 0; k < NV; k++) {
+                const unsigned int b = b0 + i * blockDim.x;
+                w[i][k] = b < gridDim.x ? __ldcg(&partials[size_t(b) * NV + k]) : 0.0;
+            }
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int k = 0; k < NV; k++) acc[k] += w[i][k];
+    }
     block_sum<NV>(acc, sh);
     if (threadIdx.x == 0) {
 #pragma unroll

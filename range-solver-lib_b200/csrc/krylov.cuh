@@ -3,6 +3,7 @@
 
 #include "csr.cuh"
 
+#include <cstddef>
 #include <utility>
 
 namespace rsg {
@@ -30,15 +31,17 @@ struct CgState {
     int32_t need_check;
     int32_t fold;
     uint32_t n_updates;
+    uint32_t pcur;          // which direction buffer holds the latest p (graph and host loops)
     uint32_t body_count;
     uint32_t body_limit;
     int32_t evict_first32;  // L2 policy of the FP32 matrix stream (1 evict_first, 0 evict_last)
     int32_t auto_switch;    // RSG_PRECISION_AUTO: a drifted refresh ends the mixed loop (switched = 1)
     int32_t switched;
-    unsigned int ticket[8];  // [7] = bounded-wait error word
     double *history;   // error per iteration (may be null)
     double *trend_hist;
+    unsigned int ticket[8];  // [7] = bounded-wait error word; not part of a copied state (kStateWords)
 };
+constexpr uint32_t kStateWords = uint32_t(offsetof(CgState, ticket) / sizeof(uint32_t));
 
 struct AmgHierarchy;
 
