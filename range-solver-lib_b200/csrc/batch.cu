@@ -8,17 +8,16 @@
 // every 32-row SELL slice belongs to exactly one system.  Each system keeps its
 // own CG state (the same CgState and transitions as the single-system solver:
 // stop on FP64 true relative residual, FP64 or mixed precision with reliable
-// updates).  Per iteration the same three phases as the single-system solver
-// (direction + SpMV, update, residual check) run over the slices of a list of
-// systems: the active systems for the first two, and for the check only the
-// systems whose update asked for one (a refresh or a convergence claim) -- the
-// check is an FP64 SpMV, and spread over all active systems' slices its few
-// listed systems would leave most warps idle and a few working through long
-// runs of slices.  Each slice writes its partial sums; one block per listed
-// system then adds them in slice order and advances the system's state, and the
-// last of those blocks after an update builds the check list.  The loop is one
-// CUDA graph `while` node; the tail kernel rebuilds the active list and keeps
-// the loop running while any system is active.
+// updates).  Per iteration two kernels (direction + SpMV, update) run over the
+// slices of the active systems: every block takes a contiguous range of the
+// list's slices, so most blocks work for one system, and adds up its part of
+// each system it touches; the last block to finish a system's part (a ticket per
+// system) adds the blocks' sums in block order and advances that system's state.
+// A system whose update asks for a residual check waits (the next directions and
+// updates skip it) until the check that ends each body of kBatchIterations
+// iterations, an FP64 SpMV over the systems that asked.  The loop is one CUDA
+// graph `while` node; the tail kernel rebuilds the active list and keeps the loop
+// running while any system is active.
 #include "krylov.cuh"
 
 #include <algorithm>
@@ -49,8 +48,9 @@ struct BatchCtl {
     uint32_t body_limit;
     int32_t timeout;
     int32_t pad;
-    uint32_t arrive;  // blocks of the update reduction that have finished (reset by the last)
 };
+
+constexpr int kBatchIterations = 4;
 
 struct BView {
     const uint32_t *slice_sys;
@@ -58,57 +58,63 @@ struct BView {
     uint32_t n_slices, n_sys;
 };
 
-// Systems a kernel visits: ids and the exclusive prefix of their slice counts.
+// Systems a kernel visits.  One entry holds all that a block needs to start on a system, so that finding
+// its place takes two round trips to memory (the head beside the entries' first words, then the entry)
+// instead of a binary search through a chain of them.
+struct ListHead {
+    uint32_t n_sys;     // number of listed systems
+    uint32_t n_slices;  // their slices in total
+};
 struct Active {
-    uint32_t n_sys;      // number of listed systems
-    uint32_t n_slices;   // their slices in total
-    uint32_t *sys;       // [capacity]
-    uint32_t *prefix;    // [capacity + 1]
+    ListHead *head;
+    uint4 *entry;  // per listed system: id, first and last + 1 of its slices in the list, its first slice less the former
 };
 
-// Block-wide (blockDim.x == kBlock): lists in order the systems in_sys[0..n_in) (0..n_in when in_sys
-// is null) that keep(system) accepts, with the exclusive prefix of their slice counts.  Every
-// thread calls it; keep must give the same answer on both of its calls.
+// Block-wide (blockDim.x == kBlock): lists in order the systems of `in` (0..n_in when it has no entries)
+// that keep(system) accepts.  Every thread calls it; keep must give the same answer on both of its calls.
 template <class KEEP>
-__device__ __forceinline__ void build_list(uint32_t n_in, const uint32_t *in_sys, const uint32_t *sys_slice,
-                                           Active *out, KEEP keep)
+__device__ __forceinline__ void build_list(uint32_t n_in, const uint4 *in, const uint32_t *sys_slice, const Active &out,
+                                           KEEP keep)
 {
     __shared__ uint32_t cnt_sys[kBlock], cnt_sl[kBlock];
     const uint32_t t = threadIdx.x, per = (n_in + blockDim.x - 1) / blockDim.x;
     const uint32_t i0 = min(n_in, t * per), i1 = min(n_in, i0 + per);
     uint32_t ns = 0, nsl = 0;
     for (uint32_t i = i0; i < i1; i++) {
-        const uint32_t sys = in_sys ? in_sys[i] : i;
+        const uint32_t sys = in ? in[i].x : i;
         if (keep(sys)) {
             ns++;
             nsl += sys_slice[sys + 1] - sys_slice[sys];
         }
     }
-    cnt_sys[t] = ns;
-    cnt_sl[t] = nsl;
-    __syncthreads();
-    if (t == 0) {  // exclusive scan (blockDim entries)
-        uint32_t a = 0, b = 0;
-        for (uint32_t k = 0; k < blockDim.x; k++) {
-            const uint32_t x = cnt_sys[k], y = cnt_sl[k];
-            cnt_sys[k] = a;
-            cnt_sl[k] = b;
+    // exclusive scans over the block
+    uint32_t a = ns, b = nsl;
+    const uint32_t lane = t & 31u, warp = t >> 5;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t x = __shfl_up_sync(0xffffffffu, a, o), y = __shfl_up_sync(0xffffffffu, b, o);
+        if (lane >= uint32_t(o)) {
             a += x;
             b += y;
         }
-        out->n_sys = a;
-        out->n_slices = b;
-        out->prefix[a] = b;
+    }
+    if (lane == 31) {
+        cnt_sys[warp] = a;
+        cnt_sl[warp] = b;
     }
     __syncthreads();
-    uint32_t o = cnt_sys[t], pre = cnt_sl[t];
+    for (uint32_t w = 0; w < warp; w++) {
+        a += cnt_sys[w];
+        b += cnt_sl[w];
+    }
+    if (t == blockDim.x - 1) *out.head = ListHead{a, b};
+    uint32_t o = a - ns, pre = b - nsl;
     for (uint32_t i = i0; i < i1; i++) {
-        const uint32_t sys = in_sys ? in_sys[i] : i;
+        const uint32_t sys = in ? in[i].x : i;
         if (keep(sys)) {
-            out->sys[o] = sys;
-            out->prefix[o] = pre;
-            pre += sys_slice[sys + 1] - sys_slice[sys];
-            o++;
+            const uint32_t first = sys_slice[sys], len = sys_slice[sys + 1] - first;
+            out.entry[o++] = make_uint4(sys, pre, pre + len, first - pre);
+            pre += len;
         }
     }
     __syncthreads();
@@ -149,57 +155,8 @@ __device__ __forceinline__ V sell_row(const Sell<V> &M, uint32_t s, int lane, GX
     return acc;
 }
 
-// Warp loop over a contiguous block of the listed systems' slices (so warps share
-// the active work evenly).  Systems that `skip(st)` rejects are jumped over as a
-// whole.  For every visited slice, `body(s, st, v)` fills this lane's
-// contributions; the warp sums them and lane 0 stores the slice's partials.
-// No atomics: the per-system totals are formed by bk_reduce.
-template <int NV, class SKIP, class BODY>
-__device__ __forceinline__ void batch_loop(const BView &B, const Active *L, CgState *S, double *part, SKIP skip,
-                                           BODY body)
-{
-    const int lane = threadIdx.x & 31;
-    const uint32_t W = gridDim.x * (blockDim.x >> 5);
-    const uint32_t w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    const uint32_t total = L->n_slices, n_list = L->n_sys;
-    const uint32_t per = (total + W - 1) / W;
-    const uint32_t a_begin = min(total, w * per), a_end = min(total, a_begin + per);
-    if (a_begin >= a_end) return;
-    uint32_t lo = 0, hi = n_list;  // last k with prefix[k] <= a_begin
-    while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) / 2;
-        if (L->prefix[mid] <= a_begin) lo = mid;
-        else hi = mid;
-    }
-    uint32_t k = lo;
-    uint32_t a = a_begin;
-    while (a < a_end) {
-        const uint32_t sys = L->sys[k], k_end = L->prefix[k + 1];
-        CgState *st = &S[sys];
-        if (skip(st)) {
-            a = k_end;
-            k++;
-            continue;
-        }
-        const uint32_t base = B.sys_slice[sys] - L->prefix[k];
-        const uint32_t stop = min(a_end, k_end);
-        for (; a < stop; a++) {
-            const uint32_t s = base + a;
-            double v[NV];
-            body(s, st, v);
-#pragma unroll
-            for (int q = 0; q < NV; q++) v[q] = warp_sum(v[q]);
-            if (lane == 0)
-#pragma unroll
-                for (int q = 0; q < NV; q++) part[size_t(s) * NV + q] = v[q];
-        }
-        k++;
-    }
-}
-
-// One block per listed system: adds the system's slice partials in a fixed order
-// and applies the state transition KIND (the same transitions as the
-// single-system solver).
+// The state transition that a phase's per-system sums lead to (the same transitions as the single-system
+// solver).
 enum RedKind { RED_INIT_RES = 0, RED_INIT_Z, RED_DIR64, RED_DIR32, RED_UPD64, RED_UPD32, RED_CHK64, RED_CHK32, RED_TRUE };
 
 template <int NV, int KIND>
@@ -229,6 +186,7 @@ __device__ __forceinline__ void finalize(CgState *st, const double (&acc)[NV], d
         st->rho = st->rho_new;
         st->alpha = st->rho / pq;
         st->fold = 0;
+        st->pcur ^= 1u;
     } else if constexpr (KIND == RED_UPD64) {
         finalize_update64(st, acc[0], acc[1], acc[2]);
     } else if constexpr (KIND == RED_UPD32) {
@@ -242,43 +200,95 @@ __device__ __forceinline__ void finalize(CgState *st, const double (&acc)[NV], d
     }
 }
 
-template <int NV, int KIND>
-__global__ void __launch_bounds__(kBlock) bk_reduce(BView B, const Active *L, CgState *S, const double *part,
-                                                    double *relres, Active *L_chk = nullptr, uint32_t *arrive = nullptr)
+
+// The blocks' loop over the listed systems' slices.  Block j takes slices [j per, (j + 1) per) of the list;
+// systems that `skip(st)` rejects are jumped over as a whole.  For every visited slice one warp runs
+// `body(s, st, v)`, which returns the lane's contributions; at the end of a system's stretch the block adds
+// them up.  A system that lies in one block is finished there; otherwise the block stores its sums in slot
+// (block + list position) -- consecutive for a system's blocks, and no two (block, system) pairs share one,
+// as either grows along the list -- and the last block to take the system's ticket adds the slots.  Sums and
+// transition used to be kernels of their own after every phase, with the check in every iteration: 24 uneven
+// cubes (0.39M rows), six and a half launches an iteration, mixed 14.2, FP64 13.4 ms a solve; now 11.0 and
+// 10.5 (29 us an iteration: direction 18.5, update 10.3).
+struct Sums {
+    double *part;          // [grid + n_sys][NV]
+    unsigned int *ticket;  // per system, zero between uses
+    double *relres;        // RED_TRUE only
+};
+
+template <int NV, int KIND, class SKIP, class BODY>
+__device__ __forceinline__ void batch_run(const BView &B, const Active L, CgState *S, const Sums &T, SKIP skip, BODY body)
 {
     __shared__ double sh[NV * 32];
-    __shared__ uint32_t last_sh;
-    if (blockIdx.x < L->n_sys) {
-        const uint32_t sys = L->sys[blockIdx.x];
+    __shared__ CgState s;
+    __shared__ int last_sh;
+    const uint32_t warp = threadIdx.x >> 5;
+    // the entries that start at or before this block's first slice are the first of the list: count them
+    uint32_t begin = threadIdx.x < B.n_sys ? L.entry[threadIdx.x].y : 0u;
+    const uint32_t total = L.head->n_slices, n_list = L.head->n_sys;
+    const uint32_t per = ((total + gridDim.x - 1) / gridDim.x + kWarpsPerBlock - 1) / kWarpsPerBlock * kWarpsPerBlock;
+    uint32_t a = min(uint64_t(total), uint64_t(blockIdx.x) * per);
+    const uint32_t a_end = min(total, a + per);
+    if (a >= a_end) return;
+    uint32_t k = 0;
+    for (uint32_t i = 0; i < n_list; i += blockDim.x) {
+        if (i) begin = i + threadIdx.x < n_list ? L.entry[i + threadIdx.x].y : 0u;
+        k += __syncthreads_count(i + threadIdx.x < n_list && begin <= a);
+    }
+    k--;
+    for (; a < a_end; k++) {
+        const uint4 e = L.entry[k];
+        const uint32_t sys = e.x, k_begin = e.y, k_end = e.z, stop = min(a_end, k_end);
         CgState *st = &S[sys];
-        const bool skip = (KIND == RED_INIT_RES || KIND == RED_TRUE) ? false
-                          : (KIND == RED_CHK64 || KIND == RED_CHK32) ? (st->done || !st->need_check)
-                                                                     : st->done != 0;
-        if (!skip) {
-            const uint32_t b0 = B.sys_slice[sys], b1 = B.sys_slice[sys + 1];
-            double acc[NV];
+        if (!skip(st)) {
+            const uint32_t base = e.w;
+            double v[NV];
 #pragma unroll
-            for (int q = 0; q < NV; q++) acc[q] = 0.0;
-            for (uint32_t s = b0 + threadIdx.x; s < b1; s += blockDim.x)
+            for (int q = 0; q < NV; q++) v[q] = 0.0;
+            for (uint32_t i = a + warp; i < stop; i += kWarpsPerBlock) {
+                double t[NV];
+                body(base + i, st, t);
 #pragma unroll
-                for (int q = 0; q < NV; q++) acc[q] += part[size_t(s) * NV + q];
-            block_sum<NV>(acc, sh);
-            if (threadIdx.x == 0) finalize<NV, KIND>(st, acc, relres, sys);
+                for (int q = 0; q < NV; q++) v[q] += t[q];
+            }
+            block_sum<NV>(v, sh);
+            const uint32_t first = k_begin / per, n_blocks = (k_end - 1) / per - first + 1;
+            if (threadIdx.x == 0) {
+                last_sh = 1;
+                if (n_blocks > 1) {
+#pragma unroll
+                    for (int q = 0; q < NV; q++) T.part[size_t(blockIdx.x + k) * NV + q] = v[q];
+                    unsigned int t;
+                    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(t) : "l"(T.ticket + sys) : "memory");
+                    last_sh = t == n_blocks - 1;
+                }
+            }
+            __syncthreads();
+            if (last_sh) {
+                for (uint32_t w = threadIdx.x; w < kStateWords; w += blockDim.x)
+                    reinterpret_cast<uint32_t *>(&s)[w] = __ldcg(reinterpret_cast<const uint32_t *>(st) + w);
+                if (n_blocks > 1) {
+#pragma unroll
+                    for (int q = 0; q < NV; q++) v[q] = 0.0;
+#pragma unroll 4
+                    for (uint32_t i = threadIdx.x; i < n_blocks; i += blockDim.x)
+#pragma unroll
+                        for (int q = 0; q < NV; q++) v[q] += __ldcg(&T.part[size_t(first + k + i) * NV + q]);
+                    block_sum<NV>(v, sh);
+                    if (threadIdx.x == 0) T.ticket[sys] = 0u;
+                } else {
+                    __syncthreads();
+                }
+                if (threadIdx.x == 0) finalize<NV, KIND>(&s, v, T.relres, sys);
+                __syncthreads();
+                if (KIND != RED_TRUE)
+                    for (uint32_t w = threadIdx.x; w < kStateWords; w += blockDim.x)
+                        reinterpret_cast<uint32_t *>(st)[w] = reinterpret_cast<const uint32_t *>(&s)[w];
+                __syncthreads();
+            }
         }
+        a = stop;
     }
-    if (!L_chk) return;
-    // after an update: the last block to finish lists the systems that asked for a check
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        last_sh = atomicAdd(arrive, 1u) == gridDim.x - 1;
-    }
-    __syncthreads();
-    if (!last_sh) return;
-    __threadfence();
-    build_list(L->n_sys, L->sys, B.sys_slice, L_chk,
-               [&](uint32_t i) { return __ldcg(&S[i].done) == 0 && __ldcg(&S[i].need_check) != 0; });
-    if (threadIdx.x == 0) *arrive = 0;
 }
 
 #define BATCH_ROWS_LOOP                                                                                      \
@@ -286,14 +296,14 @@ __global__ void __launch_bounds__(kBlock) bk_reduce(BView B, const Active *L, Cg
     const uint32_t warps_total = gridDim.x * (blockDim.x >> 5);                                             \
     for (uint32_t s = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); s < B.n_slices; s += warps_total)
 
-__global__ void __launch_bounds__(kBlock) bk_init_res(Sell<double> M, BView B, const Active *L, const double *__restrict__ b,
+__global__ void __launch_bounds__(kBlock) bk_init_res(Sell<double> M, BView B, const Active L, const double *__restrict__ b,
                                                       const double *__restrict__ x, double *__restrict__ r,
-                                                      double *part, CgState *S)
+                                                      Sums T, CgState *S)
 {
     const int lane = threadIdx.x & 31;
     auto gx = [&](uint32_t c) { return x[c]; };
-    batch_loop<2>(
-        B, L, S, part, [](const CgState *) { return false; },
+    batch_run<2, RED_INIT_RES>(
+        B, L, S, T, [](const CgState *) { return false; },
         [&](uint32_t s, CgState *, double(&v)[2]) {
             const double ax = sell_row<double>(M, s, lane, gx);
             const uint32_t row = s * 32u + lane;
@@ -308,14 +318,14 @@ __global__ void __launch_bounds__(kBlock) bk_init_res(Sell<double> M, BView B, c
 }
 
 template <bool MIXED>
-__global__ void __launch_bounds__(kBlock) bk_init_z(BView B, const Active *L, uint32_t n, const double *__restrict__ d,
+__global__ void __launch_bounds__(kBlock) bk_init_z(BView B, const Active L, uint32_t n, const double *__restrict__ d,
                                                     const float *__restrict__ d32, const double *__restrict__ r,
                                                     double *__restrict__ z, float *__restrict__ r32,
-                                                    float *__restrict__ z32, double *part, CgState *S)
+                                                    float *__restrict__ z32, Sums T, CgState *S)
 {
     const int lane = threadIdx.x & 31;
-    batch_loop<1>(
-        B, L, S, part, [](const CgState *st) { return st->done != 0; },
+    batch_run<1, RED_INIT_Z>(
+        B, L, S, T, [](const CgState *st) { return st->done != 0; },
         [&](uint32_t s, CgState *st, double(&v)[1]) {
             const uint32_t row = s * 32u + lane;
             v[0] = 0.0;
@@ -335,17 +345,21 @@ __global__ void __launch_bounds__(kBlock) bk_init_z(BView B, const Active *L, ui
         });
 }
 
+// Six blocks an SM (40 registers): 0.39M rows mixed 11.0 ms a solve; seven or eight 11.8, FP64 10.5 against 13.3.
 template <typename V, bool MIXED>
-__global__ void __launch_bounds__(kBlock) bk_dir(Sell<V> M, BView B, const Active *L, const V *__restrict__ z,
-                                                 const V *__restrict__ p_old, V *__restrict__ p_new,
-                                                 V *__restrict__ q, double *__restrict__ x, float *__restrict__ y,
-                                                 double *part, CgState *S)
+__global__ void __launch_bounds__(kBlock, 6) bk_dir(Sell<V> M, BView B, const Active L, const V *__restrict__ z, V *p0,
+                                                 V *p1, V *__restrict__ q, double *__restrict__ x,
+                                                 float *__restrict__ y, Sums T, CgState *S)
 {
+    pdl_wait();
+    pdl_release();
     const int lane = threadIdx.x & 31;
-    batch_loop<1>(
-        B, L, S, part, [](const CgState *st) { return st->done != 0; },
+    batch_run<1, MIXED ? RED_DIR32 : RED_DIR64>(
+        B, L, S, T, [](const CgState *st) { return st->done != 0 || st->need_check != 0; },
         [&](uint32_t s, CgState *st, double(&v)[1]) {
             const V beta = V(st->beta);
+            const V *__restrict__ p_old = st->pcur ? p1 : p0;
+            V *__restrict__ p_new = st->pcur ? p0 : p1;
             auto gx = [&](uint32_t c) { return MIXED ? V(fmaf(float(beta), float(p_old[c]), float(z[c])))
                                                      : V(fma(double(beta), double(p_old[c]), double(z[c]))); };
             const V ax = sell_row<V>(M, s, lane, gx);
@@ -365,16 +379,19 @@ __global__ void __launch_bounds__(kBlock) bk_dir(Sell<V> M, BView B, const Activ
 }
 
 template <typename V, bool MIXED>
-__global__ void __launch_bounds__(kBlock) bk_update(BView B, const Active *L, uint32_t n, const V *__restrict__ d,
-                                                    const V *__restrict__ p, const V *__restrict__ q,
+__global__ void __launch_bounds__(kBlock, 6) bk_update(BView B, const Active L, uint32_t n, const V *__restrict__ d,
+                                                    const V *p0, const V *p1, const V *__restrict__ q,
                                                     V *__restrict__ xy, V *__restrict__ r, V *__restrict__ z,
-                                                    double *part, CgState *S)
+                                                    Sums T, CgState *S)
 {
+    pdl_wait();
+    pdl_release();
     const int lane = threadIdx.x & 31;
-    batch_loop<3>(
-        B, L, S, part, [](const CgState *st) { return st->done != 0; },
+    batch_run<3, MIXED ? RED_UPD32 : RED_UPD64>(
+        B, L, S, T, [](const CgState *st) { return st->done != 0 || st->need_check != 0; },
         [&](uint32_t s, CgState *st, double(&v)[3]) {
             const V alpha = V(st->alpha);
+            const V *__restrict__ p = st->pcur ? p1 : p0;
             const uint32_t row = s * 32u + lane;
             v[0] = v[1] = v[2] = 0.0;
             if (row < n) {
@@ -394,16 +411,18 @@ __global__ void __launch_bounds__(kBlock) bk_update(BView B, const Active *L, ui
 }
 
 template <bool MIXED>
-__global__ void __launch_bounds__(kBlock) bk_check(Sell<double> M, BView B, const Active *L, const double *__restrict__ d,
+__global__ void __launch_bounds__(kBlock) bk_check(Sell<double> M, BView B, const Active L, const double *__restrict__ d,
                                                    const float *__restrict__ d32, const double *__restrict__ b,
                                                    const double *__restrict__ x, const float *__restrict__ y,
                                                    double *__restrict__ r, double *__restrict__ z,
-                                                   float *__restrict__ r32, float *__restrict__ z32, double *part,
+                                                   float *__restrict__ r32, float *__restrict__ z32, Sums T,
                                                    CgState *S)
 {
+    pdl_wait();
+    pdl_release();
     const int lane = threadIdx.x & 31;
-    batch_loop<2>(
-        B, L, S, part, [](const CgState *st) { return st->done != 0 || st->need_check == 0; },
+    batch_run<2, MIXED ? RED_CHK32 : RED_CHK64>(
+        B, L, S, T, [](const CgState *st) { return st->done != 0 || st->need_check == 0; },
         [&](uint32_t s, CgState *st, double(&v)[2]) {
             const double sigma = st->sigma, inv_sigma = 1.0 / sigma;
             auto gx = [&](uint32_t c) { return MIXED ? fma(double(y[c]), inv_sigma, x[c]) : x[c]; };
@@ -441,13 +460,13 @@ __global__ void bk_fold(BView B, uint32_t n, double *__restrict__ x, float *__re
     }
 }
 
-__global__ void bk_true_res(Sell<double> M, BView B, const Active *L, const double *__restrict__ b, const double *__restrict__ x,
-                            double *part, CgState *S, double *relres)
+__global__ void bk_true_res(Sell<double> M, BView B, const Active L, const double *__restrict__ b, const double *__restrict__ x,
+                            Sums T, CgState *S)
 {
     const int lane = threadIdx.x & 31;
     auto gx = [&](uint32_t c) { return x[c]; };
-    batch_loop<2>(
-        B, L, S, part, [](const CgState *) { return false; },
+    batch_run<2, RED_TRUE>(
+        B, L, S, T, [](const CgState *) { return false; },
         [&](uint32_t s, CgState *, double(&v)[2]) {
             const double ax = sell_row<double>(M, s, lane, gx);
             const uint32_t row = s * 32u + lane;
@@ -460,16 +479,26 @@ __global__ void bk_true_res(Sell<double> M, BView B, const Active *L, const doub
         });
 }
 
+// The systems of L that asked for a residual check.
+__global__ void __launch_bounds__(kBlock) bk_list(const CgState *S, const uint32_t *sys_slice, const Active L, const Active L_chk)
+{
+    pdl_wait();
+    pdl_release();
+    build_list(L.head->n_sys, L.entry, sys_slice, L_chk, [&](uint32_t i) { return S[i].done == 0 && S[i].need_check != 0; });
+}
+
 // Loop control: rebuilds the list of active systems, keeps the graph's while node
 // running while any system is active, enforces the hard limit.
 __global__ void __launch_bounds__(kBlock) bk_tail(const CgState *S, const uint32_t *sys_slice, uint32_t n_sys,
-                                                  Active *L, BatchCtl *ctl, cudaGraphConditionalHandle h,
+                                                  const Active L, BatchCtl *ctl, cudaGraphConditionalHandle h,
                                                   int use_cond)
 {
+    pdl_wait();
+    pdl_release();
     build_list(n_sys, nullptr, sys_slice, L, [&](uint32_t i) { return S[i].done == 0; });
     if (threadIdx.x == 0) {
         const uint32_t bc = ++ctl->body_count;
-        int keep = L->n_sys > 0;
+        int keep = L.head->n_sys > 0;
         if (keep && bc >= ctl->body_limit) {
             ctl->timeout = 1;
             keep = 0;
@@ -630,23 +659,26 @@ rsg_status rsg_batch_solve(rsg_context *ctx, rsg_batch *B, const rsg_solver_conf
     const uint32_t n = B->pad_rows, ns = B->n_sys, nsl = n / 32;
     const uint32_t max_it = std::max<uint32_t>(conf->n_outer, 1);
     const size_t vn = arena_bytes(n, sizeof(double)), vf = arena_bytes(n, sizeof(float));
-    size_t bytes = 8 * vn + arena_bytes(size_t(nsl) * 3, sizeof(double)) + arena_bytes(ns, sizeof(CgState)) +
-                   3 * arena_bytes(1, sizeof(Active)) + 6 * arena_bytes(size_t(ns) + 1, sizeof(uint32_t)) +
+    size_t bytes = 8 * vn + arena_bytes((size_t(kMaxGrid) + ns) * 3, sizeof(double)) + arena_bytes(ns, sizeof(CgState)) +
+                   arena_bytes(ns, sizeof(unsigned int)) +
+                   3 * arena_bytes(1, sizeof(ListHead)) + 3 * arena_bytes(ns, sizeof(uint4)) +
                    arena_bytes(ns, sizeof(double)) + arena_bytes(1, sizeof(BatchCtl)) + 2 * arena_bytes(B->user_rows, 8);
     if (mixed) bytes += 7 * vf;
     RSG_TRY(arena_reserve(ctx, bytes));
     double *bp = arena_take<double>(ctx, n), *xp = arena_take<double>(ctx, n), *r = arena_take<double>(ctx, n),
            *z = arena_take<double>(ctx, n), *p0 = arena_take<double>(ctx, n), *p1 = arena_take<double>(ctx, n),
            *q = arena_take<double>(ctx, n), *d = arena_take<double>(ctx, n);
-    double *part = arena_take<double>(ctx, size_t(nsl) * 3);
+    Sums T = {};
+    T.part = arena_take<double>(ctx, (size_t(kMaxGrid) + ns) * 3);
+    T.ticket = arena_take<unsigned int>(ctx, ns);
     CgState *S = arena_take<CgState>(ctx, ns);
-    double *relres = arena_take<double>(ctx, ns);
+    double *relres = T.relres = arena_take<double>(ctx, ns);
     BatchCtl *ctl = arena_take<BatchCtl>(ctx, 1);
-    Active *L_all = arena_take<Active>(ctx, 1), *L_act = arena_take<Active>(ctx, 1);
-    uint32_t *la_sys = arena_take<uint32_t>(ctx, size_t(ns) + 1), *la_pre = arena_take<uint32_t>(ctx, size_t(ns) + 1);
-    uint32_t *lb_sys = arena_take<uint32_t>(ctx, size_t(ns) + 1), *lb_pre = arena_take<uint32_t>(ctx, size_t(ns) + 1);
-    Active *L_chk = arena_take<Active>(ctx, 1);  // systems that asked for a check (built by the update reduction)
-    uint32_t *lc_sys = arena_take<uint32_t>(ctx, size_t(ns) + 1), *lc_pre = arena_take<uint32_t>(ctx, size_t(ns) + 1);
+    Active L_all, L_act, L_chk;  // every system; the active ones; those that asked for a check (bk_list)
+    for (Active *l : {&L_all, &L_act, &L_chk}) {
+        l->head = arena_take<ListHead>(ctx, 1);
+        l->entry = arena_take<uint4>(ctx, ns);
+    }
     double *bu = memory == RSG_MEM_HOST ? arena_take<double>(ctx, B->user_rows) : const_cast<double *>(b);
     double *xu = memory == RSG_MEM_HOST ? arena_take<double>(ctx, B->user_rows) : x;
     float *r32 = nullptr, *z32 = nullptr, *pa = nullptr, *pb = nullptr, *q32 = nullptr, *y32 = nullptr, *d32 = nullptr;
@@ -700,23 +732,18 @@ rsg_status rsg_batch_solve(rsg_context *ctx, rsg_batch *B, const rsg_solver_conf
         h.stop_rule = RSG_STOP_TRUE_RELRES;
         std::vector<CgState> hs(ns, h);
         RSG_CHECK_CUDA(ctx, cudaMemcpyAsync(S, hs.data(), ns * sizeof(CgState), cudaMemcpyHostToDevice, sm));
-        BatchCtl c = {0, max_it / 2 + 16, 0, 1, 0};
+        BatchCtl c = {0, max_it + 16, 0, 1};  // a body makes at least one iteration of every active system
+        RSG_CHECK_CUDA(ctx, cudaMemsetAsync(T.ticket, 0, ns * sizeof(unsigned int), sm));
         RSG_CHECK_CUDA(ctx, cudaMemcpyAsync(ctl, &c, sizeof(c), cudaMemcpyHostToDevice, sm));
-        // both lists start with every system
-        std::vector<uint32_t> ids(ns), pre(size_t(ns) + 1);
-        for (uint32_t i = 0; i < ns; i++) {
-            ids[i] = i;
-            pre[i] = B->pad_begin[i] / 32;
+        // the lists start with every system
+        std::vector<uint4> entry(ns);
+        for (uint32_t i = 0; i < ns; i++)
+            entry[i] = make_uint4(i, B->pad_begin[i] / 32, B->pad_begin[i + 1] / 32, 0u);
+        const ListHead head = {ns, nsl};
+        for (const Active *l : {&L_all, &L_act, &L_chk}) {
+            RSG_CHECK_CUDA(ctx, cudaMemcpyAsync(l->head, &head, sizeof(head), cudaMemcpyHostToDevice, sm));
+            RSG_CHECK_CUDA(ctx, cudaMemcpyAsync(l->entry, entry.data(), ns * sizeof(uint4), cudaMemcpyHostToDevice, sm));
         }
-        pre[ns] = nsl;
-        Active la = {ns, nsl, la_sys, la_pre}, lb = {ns, nsl, lb_sys, lb_pre}, lc = {0, 0, lc_sys, lc_pre};
-        RSG_CHECK_CUDA(ctx, cudaMemcpyAsync(la_sys, ids.data(), ns * 4, cudaMemcpyHostToDevice, sm));
-        RSG_CHECK_CUDA(ctx, cudaMemcpyAsync(la_pre, pre.data(), (size_t(ns) + 1) * 4, cudaMemcpyHostToDevice, sm));
-        RSG_CHECK_CUDA(ctx, cudaMemcpyAsync(lb_sys, ids.data(), ns * 4, cudaMemcpyHostToDevice, sm));
-        RSG_CHECK_CUDA(ctx, cudaMemcpyAsync(lb_pre, pre.data(), (size_t(ns) + 1) * 4, cudaMemcpyHostToDevice, sm));
-        RSG_CHECK_CUDA(ctx, cudaMemcpyAsync(L_all, &la, sizeof(Active), cudaMemcpyHostToDevice, sm));
-        RSG_CHECK_CUDA(ctx, cudaMemcpyAsync(L_act, &lb, sizeof(Active), cudaMemcpyHostToDevice, sm));
-        RSG_CHECK_CUDA(ctx, cudaMemcpyAsync(L_chk, &lc, sizeof(Active), cudaMemcpyHostToDevice, sm));
         RSG_CHECK_CUDA(ctx, cudaStreamSynchronize(sm));
     }
     const BView V{B->d_slice_sys, B->d_sys_slice, nsl, ns};
@@ -725,45 +752,41 @@ rsg_status rsg_batch_solve(rsg_context *ctx, rsg_batch *B, const rsg_solver_conf
     const int g_tuned = B->tuned ? (mixed ? B->g32 : B->g64) : 0;
     const int g = g_tuned > 0
                       ? g_tuned
-                      : std::min(grid_for(ctx, (const void *)bk_dir<double, false>, kBlock, 0, (long long)nsl * 32),
+                      : std::min(grid_for(ctx,
+                                          mixed ? (const void *)bk_dir<float, true> : (const void *)bk_dir<double, false>,
+                                          kBlock, 0, (long long)nsl * 32),
                                  kMaxGrid);
     cudaEventRecord(ctx->ev[0], sm);
-    const int gr = int(ns);  // reduce kernels: one block per listed system
-    bk_init_res<<<g, kBlock, 0, sm>>>(M64, V, L_all, bp, xp, r, part, S);
-    bk_reduce<2, RED_INIT_RES><<<gr, kBlock, 0, sm>>>(V, L_all, S, part, nullptr);
-    if (mixed) {
-        bk_init_z<true><<<g, kBlock, 0, sm>>>(V, L_all, n, jac ? d : nullptr, jac ? d32 : nullptr, r, z, r32, z32, part, S);
-    } else {
-        bk_init_z<false><<<g, kBlock, 0, sm>>>(V, L_all, n, jac ? d : nullptr, nullptr, r, z, r32, z32, part, S);
-    }
-    bk_reduce<1, RED_INIT_Z><<<gr, kBlock, 0, sm>>>(V, L_all, S, part, nullptr);
+    bk_init_res<<<g, kBlock, 0, sm>>>(M64, V, L_all, bp, xp, r, T, S);
+    if (mixed)
+        bk_init_z<true><<<g, kBlock, 0, sm>>>(V, L_all, n, jac ? d : nullptr, jac ? d32 : nullptr, r, z, r32, z32, T, S);
+    else
+        bk_init_z<false><<<g, kBlock, 0, sm>>>(V, L_all, n, jac ? d : nullptr, nullptr, r, z, r32, z32, T, S);
     RSG_CHECK_CUDA(ctx, cudaGetLastError());
 
-    auto body = [&](cudaGraphConditionalHandle h, int use_cond) {
-        for (int half = 0; half < 2; half++) {
+    auto body = [&](cudaGraphConditionalHandle h, int use_cond, bool pdl) {
+        for (int it = 0; it < kBatchIterations; it++) {
             if (!mixed) {
-                double *po = half ? p1 : p0, *pn = half ? p0 : p1;
-                bk_dir<double, false><<<g, kBlock, 0, sm>>>(M64, V, L_act, z, po, pn, q, xp, nullptr, part, S);
-                bk_reduce<1, RED_DIR64><<<gr, kBlock, 0, sm>>>(V, L_act, S, part, nullptr);
-                bk_update<double, false><<<g, kBlock, 0, sm>>>(V, L_act, n, jac ? d : nullptr, pn, q, xp, r, z, part, S);
-                bk_reduce<3, RED_UPD64><<<gr, kBlock, 0, sm>>>(V, L_act, S, part, nullptr, L_chk, &ctl->arrive);
-                bk_check<false><<<g, kBlock, 0, sm>>>(M64, V, L_chk, jac ? d : nullptr, nullptr, bp, xp, nullptr, r, z,
-                                                     nullptr, nullptr, part, S);
-                bk_reduce<2, RED_CHK64><<<gr, kBlock, 0, sm>>>(V, L_chk, S, part, nullptr);
+                launch_k(sm, pdl, bk_dir<double, false>, g, kBlock, 0, M64, V, L_act, z, p0, p1, q, xp,
+                         (float *)nullptr, T, S);
+                launch_k(sm, pdl, bk_update<double, false>, g, kBlock, 0, V, L_act, n, jac ? d : (double *)nullptr, p0,
+                         p1, q, xp, r, z, T, S);
             } else {
-                float *po = half ? pb : pa, *pn = half ? pa : pb;
-                bk_dir<float, true><<<g, kBlock, 0, sm>>>(M32, V, L_act, z32, po, pn, q32, xp, y32, part, S);
-                bk_reduce<1, RED_DIR32><<<gr, kBlock, 0, sm>>>(V, L_act, S, part, nullptr);
-                bk_update<float, true><<<g, kBlock, 0, sm>>>(V, L_act, n, jac ? d32 : nullptr, pn, q32, y32, r32, z32, part,
-                                                            S);
-                bk_reduce<3, RED_UPD32><<<gr, kBlock, 0, sm>>>(V, L_act, S, part, nullptr, L_chk, &ctl->arrive);
-                bk_check<true><<<g, kBlock, 0, sm>>>(M64, V, L_chk, nullptr, jac ? d32 : nullptr, bp, xp, y32, r, z, r32,
-                                                    z32, part, S);
-                bk_reduce<2, RED_CHK32><<<gr, kBlock, 0, sm>>>(V, L_chk, S, part, nullptr);
+                launch_k(sm, pdl, bk_dir<float, true>, g, kBlock, 0, M32, V, L_act, z32, pa, pb, q32, xp, y32, T, S);
+                launch_k(sm, pdl, bk_update<float, true>, g, kBlock, 0, V, L_act, n, jac ? d32 : (float *)nullptr, pa, pb,
+                         q32, y32, r32, z32, T, S);
             }
         }
-        bk_tail<<<1, kBlock, 0, sm>>>(S, B->d_sys_slice, ns, L_act, ctl, h, use_cond);
+        launch_k(sm, pdl, bk_list, 1, kBlock, 0, S, B->d_sys_slice, L_act, L_chk);
+        if (!mixed)
+            launch_k(sm, pdl, bk_check<false>, g, kBlock, 0, M64, V, L_chk, jac ? d : (double *)nullptr, (float *)nullptr,
+                     bp, xp, (float *)nullptr, r, z, (float *)nullptr, (float *)nullptr, T, S);
+        else
+            launch_k(sm, pdl, bk_check<true>, g, kBlock, 0, M64, V, L_chk, (double *)nullptr, jac ? d32 : (float *)nullptr,
+                     bp, xp, y32, r, z, r32, z32, T, S);
+        launch_k(sm, pdl, bk_tail, 1, kBlock, 0, S, B->d_sys_slice, ns, L_act, ctl, h, use_cond);
     };
+    const bool pdl = pdl_for(B->A, mixed);
 
     rsg_status status = RSG_OK;
     if (conf->use_graph) {
@@ -788,7 +811,7 @@ rsg_status rsg_batch_solve(rsg_context *ctx, rsg_batch *B, const rsg_solver_conf
                 status = set_error(ctx, RSG_ERR_CUDA, "batch: graph capture");
                 break;
             }
-            body(h, 1);
+            body(h, 1, pdl);
             cudaGraph_t captured;
             if (cudaStreamEndCapture(sm, &captured) != cudaSuccess || cudaGraphInstantiate(&exec, graph, 0) != cudaSuccess ||
                 cudaGraphLaunch(exec, sm) != cudaSuccess) {
@@ -802,10 +825,10 @@ rsg_status rsg_batch_solve(rsg_context *ctx, rsg_batch *B, const rsg_solver_conf
         if (status != RSG_OK) return status;
         if (e != cudaSuccess) return set_error(ctx, RSG_ERR_CUDA, "batch solve: %s", cudaGetErrorString(e));
     } else {
-        const uint32_t polls = std::max<uint32_t>(1, conf->check_interval / 2);
+        const uint32_t polls = std::max<uint32_t>(1, conf->check_interval / kBatchIterations);
         int32_t *keep = reinterpret_cast<int32_t *>(ctx->pinned);
         for (;;) {
-            for (uint32_t k = 0; k < polls; k++) body(0, 0);
+            for (uint32_t k = 0; k < polls; k++) body(0, 0, pdl);
             RSG_CHECK_CUDA(ctx, cudaGetLastError());
             RSG_CHECK_CUDA(ctx, cudaMemcpyAsync(keep, &ctl->pad, sizeof(int32_t), cudaMemcpyDeviceToHost, sm));
             RSG_CHECK_CUDA(ctx, cudaStreamSynchronize(sm));
@@ -813,8 +836,7 @@ rsg_status rsg_batch_solve(rsg_context *ctx, rsg_batch *B, const rsg_solver_conf
         }
     }
     if (mixed) bk_fold<<<g, kBlock, 0, sm>>>(V, n, xp, y32, S);
-    bk_true_res<<<g, kBlock, 0, sm>>>(M64, V, L_all, bp, xp, part, S, relres);
-    bk_reduce<2, RED_TRUE><<<gr, kBlock, 0, sm>>>(V, L_all, S, part, relres);
+    bk_true_res<<<g, kBlock, 0, sm>>>(M64, V, L_all, bp, xp, T, S);
     cudaEventRecord(ctx->ev[1], sm);
     bk_gather<<<gu, kBlock, 0, sm>>>(B->user_rows, B->d_user2pad, xp, xu);
     if (memory == RSG_MEM_HOST)
