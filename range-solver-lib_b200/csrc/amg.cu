@@ -27,8 +27,10 @@
 //   with the same sweeps.  Every sweep is one pass over the level's matrix with the smoother fused
 //   into the gather; the finest level reads the matrix's FP32 SELL-32 (or CSR-stream) copy, the
 //   coarse levels their CSR with 4 lanes per row.  Levels 1..kAmgKLevels are solved by two
-//   flexible-CG steps each (K-cycle); the last smoothed level and the dense coarse solve run as one
-//   single-CTA kernel.  Each step is its own kernel, launched with programmatic dependent launch; on
+//   flexible-CG steps each (K-cycle).  With one sweep a second K-cycle level of at most kAmgClusterRows
+//   rows and all levels below it run as one thread-block cluster (amg_cluster.cu); otherwise each step is
+//   its own kernel, launched with programmatic dependent launch, the last smoothed level and the dense
+//   coarse solve one single-CTA kernel.  On
 //   request (conf.persistent > 0) the levels of at most kCoarsePersistRows rows run instead as one
 //   persistent cooperative kernel per visit, with the same bits (measured slower on B200).
 #include "amg.cuh"
@@ -1362,6 +1364,9 @@ enum CoarseOp : uint32_t {
     CP_DENSE,         // dense coarse solve: a.out = inv a.b
     CP_KC_SPMV2,      // K-cycle: v = A c, sc[o0] = c.v, sc[o1] = c.y1
     CP_KC_SPMV3,      //          ... and sc[o2] = c.y2
+    CP_KC_MV,         // K-cycle on a cluster level: v = A c
+    CP_KC_DOTS2,      //          ... sc[o0] = c.v, sc[o1] = c.y1, added as amg_cluster.cu adds them
+    CP_KC_DOTS3,      //          ... and sc[o2] = c.y2
     CP_KC_R2,         // K-cycle: r2 = a.b - a1 v1 (a1 from sc), x1 = dw r2
 };
 
@@ -1436,6 +1441,40 @@ __device__ __forceinline__ void kc_spmv_blocks(const CoarsePhase &p, double *par
     }
 }
 
+// The K-cycle dot products as the cluster kernel forms them: CTA `cta` < kAmgClusterCtas takes the rows of its
+// aggregates, thread g the cluster kernel's row group g (its 1024 threads are 256 groups of four lanes, rows
+// g, g + 256, ...), then that kernel's warps of eight groups and its block; part[3 cta + k].
+static_assert(kAmgClusterThreads == 4 * kBlock, "one thread per row group of the cluster kernel");
+__device__ __forceinline__ void kc_dots_cluster(const CoarsePhase &p, bool three, double *part, double *sh, uint32_t cta)
+{
+    const uint32_t I0 = uint32_t(uint64_t(p.nc) * cta / kAmgClusterCtas),
+                   I1 = uint32_t(uint64_t(p.nc) * (cta + 1) / kAmgClusterCtas);
+    Dot2 s[3];
+    for (uint32_t k = p.ptr[I0] + threadIdx.x; k < p.ptr[I1]; k += kBlock) {
+        const uint32_t row = p.rows[k];
+        const float c = __ldcg(p.c + row);
+        s[0].add_prod(c, __ldcg(p.v + row));
+        s[1].add_prod(c, __ldcg(p.y1 + row));
+        if (three) s[2].add_prod(c, __ldcg(p.y2 + row));
+    }
+    double v[3] = {s[0].value(), s[1].value(), s[2].value()};
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
+        for (int k = 0; k < 3; k++) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+    __syncthreads();
+    if ((threadIdx.x & 7) == 0)
+#pragma unroll
+        for (int k = 0; k < 3; k++) sh[k * 32 + (threadIdx.x >> 3)] = v[k];
+    __syncthreads();
+    if (threadIdx.x < 32)
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            const double t = warp_sum(sh[k * 32 + threadIdx.x]);
+            if (threadIdx.x == 0) part[3 * cta + k] = t;
+        }
+}
+
 __global__ void __launch_bounds__(kBlock) k_amg_coarse_persist(const CoarsePhase *prog, uint32_t n_phases,
                                                                double *part, unsigned int *bar, const CgState *st,
                                                                unsigned int *err)
@@ -1482,6 +1521,28 @@ __global__ void __launch_bounds__(kBlock) k_amg_coarse_persist(const CoarsePhase
                     p.sc[p.o0] = acc[0];
                     p.sc[p.o1] = acc[1];
                     if (op == CP_KC_SPMV3) p.sc[p.o2] = acc[2];
+                }
+            };
+            if (!grid_barrier(bar, err, last)) return;
+            continue;
+        } else if (op == CP_KC_MV) {
+            const int ln = threadIdx.x & (kLanes - 1);
+            auto gx = [&](uint32_t col) { return __ldcg(p.c + col); };
+            for (uint32_t b0 = gw * (32 / kLanes); b0 < p.n; b0 += warps * (32 / kLanes)) {
+                const uint32_t row = b0 + (threadIdx.x & 31) / kLanes;
+                const float acc = csr_row_dot(p.rp, p.ci, p.val, row, row < p.n, ln, gx);
+                if (ln == 0 && row < p.n) p.v[row] = acc;
+            }
+        } else if (op == CP_KC_DOTS2 || op == CP_KC_DOTS3) {
+            for (uint32_t c = blockIdx.x; c < kAmgClusterCtas; c += gridDim.x)
+                kc_dots_cluster(p, op == CP_KC_DOTS3, part, sh, c);
+            auto last = [&]() {
+                if (threadIdx.x < 3) {
+                    double t = 0.0;
+                    for (uint32_t c = 0; c < kAmgClusterCtas; c++) t += __ldcg(&part[3 * c + threadIdx.x]);
+                    if (threadIdx.x == 0) p.sc[p.o0] = t;
+                    else if (threadIdx.x == 1) p.sc[p.o1] = t;
+                    else if (op == CP_KC_DOTS3) p.sc[p.o2] = t;
                 }
             };
             if (!grid_barrier(bar, err, last)) return;
@@ -1702,6 +1763,10 @@ void amg_free(AmgHierarchy *H)
         l.v2.release();
         l.r2.release();
     }
+    H->cluster.blob.release();
+    H->cluster.ext.release();
+    H->cluster.place.release();
+    if (H->cluster.ext_h) cudaFreeHost(H->cluster.ext_h);
     H->coarse_inv.release();
     H->T.release();
     H->M1.release();
@@ -1784,7 +1849,9 @@ rsg_status amg_setup(rsg_context *ctx, rsg_csr *A, bool persistent)
         k_amg_dense_inverse<<<1, 512, smem, ctx->stream>>>(last.n, last.rp, last.ci, last.val, H->coarse_inv.p);
         RSG_CHECK_CUDA(ctx, cudaGetLastError());
     }
+    RSG_TRY(amg_cluster_extents(ctx, H));
     RSG_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    RSG_TRY(amg_cluster_pack(ctx, H));
     H->seconds_setup = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
     H->setup_launches = t_launches - launches0;
     RSG_TRY(build_persist(ctx, H, persistent));
@@ -1828,9 +1895,8 @@ void fine_sweep(rsg_context *ctx, const FineLaunch<RPW> &f, const SweepArgs &a, 
 }
 
 // Coarse levels run on the whole GPU: CSR with kLanes lanes per row.  (A SELL-32 copy leaves one warp
-// per 32 rows, too few warps for these levels: measured slower.  One thread-block cluster of 8 CTAs
-// running all levels of up to 32k rows with cluster barriers between steps was slower still: 8 SMs
-// lack the memory-level parallelism for the 276k-entry third level.)
+// per 32 rows, too few warps for these levels: measured slower.  The levels from a small second K-cycle
+// level on run in one thread-block cluster instead, amg_cluster.cu.)
 template <int SRC, int OUT>
 void coarse_sweep(rsg_context *ctx, const AmgLevel &l, const SweepArgs &a, const CgState *st, bool pdl)
 {
@@ -1967,6 +2033,11 @@ void solve_level(rsg_context *ctx, const AmgHierarchy *H, int l, const float *b,
         coarse_persist(ctx, H, sweeps, st);
         return;
     }
+    if (l == H->cluster.level && l > 0 && sweeps == 1 && b == F.b.p && e == F.e.p) {  // amg_cluster.cu
+        ++t_launches;
+        if (!t_dry) amg_cluster_launch(ctx, H, st, pdl);
+        return;
+    }
     if (l == H->levels - 1) {
         if (H->dense_coarsest) {
             amg_launch(ctx->stream, pdl, k_amg_dense_apply, 1, 1024, 0, F.n, (const float *)H->coarse_inv.p, b, e, st);
@@ -2066,6 +2137,14 @@ struct CoarseProgram {
         p.o0 = o0;
         p.o1 = o1;
         p.o2 = o2;
+        if (sweeps == 1 && H->cluster.level && &F == &H->L[H->cluster.level]) {  // the cluster kernel's dot products
+            p.nc = H->L[H->cluster.level + 1].n;
+            p.ptr = F.agg_ptr.p;
+            p.rows = F.agg_rows.p;
+            p.op = CP_KC_MV;
+            ph.push_back(p);
+            p.op = ndot == 2 ? CP_KC_DOTS2 : CP_KC_DOTS3;
+        }
         ph.push_back(p);
     }
     void cycle(int l, const float *b, float *out)

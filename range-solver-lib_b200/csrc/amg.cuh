@@ -68,7 +68,33 @@ struct AmgLevel {
     DevBuf<float> c1, c2, v1, v2, r2;      // K-cycle levels: the two flexible-CG steps
 };
 
+// The coarse levels that one thread-block cluster runs (amg_cluster.cu): level kAmgClusterLevel, a K-cycle
+// level, and all below it, when their packed parts fit the cluster's shared memory.
+constexpr int kAmgClusterLevel = 2;
+constexpr uint32_t kAmgClusterRows = 7168;  // the first of them has at most so many rows
+constexpr uint32_t kAmgClusterCtas = 16;
+constexpr int kAmgClusterThreads = 1024;
+struct AmgClusterMap {                 // shared-memory layout, the same in every CTA (byte offsets)
+    uint32_t nl = 0;                   // smoothed levels
+    uint32_t n[kAmgMaxLevels + 1];     // rows of each, and of the dense level after them
+    uint32_t o_ga[kAmgMaxLevels], o_gb[kAmgMaxLevels], o_bw[kAmgMaxLevels], o_e[kAmgMaxLevels];
+    uint32_t o_bown, o_v1, o_r2, o_xo, o_part, o_bd, o_ws, o_win, o_blob;
+    uint32_t stride;                   // bytes of packed data per CTA in global memory
+    float scale;
+};
+struct AmgCluster {
+    int level = 0;                     // first level, 0: not used
+    int supported = -1;
+    uint32_t smem = 0;
+    AmgClusterMap map;
+    DevBuf<uint8_t> blob;
+    DevBuf<uint32_t> ext;
+    DevBuf<uint16_t> place;            // set-up scratch
+    uint32_t *ext_h = nullptr;         // pinned
+};
+
 struct AmgHierarchy {
+    AmgCluster cluster;
     int levels = 0;                 // levels in use, the finest included
     AmgLevel L[kAmgMaxLevels];
     bool dense_coarsest = false;    // the last level is applied through coarse_inv
@@ -99,6 +125,10 @@ struct AmgHierarchy {
     uint32_t persist_len[2] = {0, 0};
     DevBuf<unsigned int> persist_bar;
 };
+
+rsg_status amg_cluster_extents(rsg_context *ctx, AmgHierarchy *H);
+rsg_status amg_cluster_pack(rsg_context *ctx, AmgHierarchy *H);
+void amg_cluster_launch(rsg_context *ctx, const AmgHierarchy *H, const CgState *st, bool pdl);
 
 void amg_free(AmgHierarchy *H);
 // (Re)builds A's hierarchy from A's current values; A owns it afterwards (freed with A).
