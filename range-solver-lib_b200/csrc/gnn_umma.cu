@@ -10,10 +10,16 @@
 //   3. all warps read the accumulator back with tcgen05.ld and apply bias, ReLU
 //      and the residual connection; the last layer also applies the output
 //      layer and writes z = M(r) in FP64.
-// W_l^T lives in shared memory as BF16 for the CTA's lifetime (persistent CTAs).
+// W_l^T lives in shared memory as BF16 for the CTA's lifetime (persistent CTAs).  A layer's CTAs stage it, and
+// load their first column indexes, while the preceding layer drains (programmatic dependent launch).
+// What bounds a layer: the load/store pipe's passes, 3.5M 128-byte neighbour rows at 219k rows and 15 entries a
+// row (8 of 12M passes; the index and weight shuffles 2.3M).  Stores into the A tile and of the output that
+// conflicted or went out 16 bytes a line, the weights staged in 2-byte stores, and four CTAs an SM with spills
+// had cost as much again: 73 us a layer, now 49; input layer 19, now 10; 4096 rows (latency) 14 and now 5.
 // Waits on the mbarrier are bounded: past kWaitLimit polls the kernel flags the
 // context's error word, waits (bounded) for its MMAs, frees its TMEM and returns.
 #include "gnn.cuh"
+#include "krylov.cuh"
 #include "spmv.cuh"
 
 namespace rsg {
@@ -25,11 +31,19 @@ constexpr int K2 = 2 * H;       // 128
 constexpr int kTileRows = 128;
 constexpr int kThreads = 256;
 constexpr uint32_t kTmemCols = 64;
+// CTAs of the layer kernel per SM.  Three leave 84 registers a thread (four: 64 and spills) and L1 for the gathers,
+// two too few loads in flight; six layers of 219k rows and their input: 365, 320 and 381 us with 4, 3 and 2.
+constexpr int kCtasPerSm = 3;
+constexpr int kCarveout = 71;  // percent: their 162 KB; the rest caches gathered rows (100: 323 us instead of 315)
 constexpr uint32_t kATileBytes = kTileRows * K2 * 2;  // 32 KB
 constexpr uint32_t kBTileBytes = H * K2 * 2;          // 16 KB
 constexpr uint32_t kLBO = 128;                        // K-adjacent core matrices
 constexpr uint32_t kSBO = (K2 / 8) * 128;             // 8-row groups: 16 core matrices of 128 B
-constexpr uint32_t kOffB = kATileBytes;
+// The layer kernel's A tile: K-adjacent core matrices 144 bytes apart instead of 128, so that the 8 lanes that
+// store one row (8 core matrices) hit 8 different bank groups.
+constexpr uint32_t kALBO = 144;
+constexpr uint32_t kASBO = (K2 / 8) * kALBO;
+constexpr uint32_t kOffB = (kTileRows / 8) * kASBO;
 constexpr uint32_t kOffBias = kOffB + kBTileBytes;
 constexpr uint32_t kOffWout = kOffBias + H * 4;
 constexpr uint32_t kOffPart = kOffWout + H * 4;
@@ -48,10 +62,15 @@ __device__ __forceinline__ uint32_t tile_off(uint32_t row, uint32_t k)
     return (row >> 3) * kSBO + (k >> 3) * kLBO + (row & 7) * 16 + (k & 7) * 2;
 }
 
-// shared-memory matrix descriptor: start address, LBO, SBO (all >> 4), version 1, no swizzle
-__device__ __forceinline__ uint64_t smem_desc(uint32_t saddr)
+__device__ __forceinline__ uint32_t a_off(uint32_t row, uint32_t k)  // the same in the layer kernel's A tile
 {
-    return uint64_t((saddr & 0x3FFFFu) >> 4) | (uint64_t(kLBO >> 4) << 16) | (uint64_t(kSBO >> 4) << 32) |
+    return (row >> 3) * kASBO + (k >> 3) * kALBO + (row & 7) * 16 + (k & 7) * 2;
+}
+
+// shared-memory matrix descriptor: start address, LBO, SBO (all >> 4), version 1, no swizzle
+__device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo = kLBO, uint32_t sbo = kSBO)
+{
+    return uint64_t((saddr & 0x3FFFFu) >> 4) | (uint64_t(lbo >> 4) << 16) | (uint64_t(sbo >> 4) << 32) |
            (uint64_t(1) << 46);
 }
 
@@ -103,18 +122,28 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi)
     return *reinterpret_cast<const uint32_t *>(&v);
 }
 
-// features and input layer, BF16 output: h0 = relu(f W_in + b_in)
-__global__ void k_gnn_input_bf16(uint32_t n, const double *__restrict__ r, const float *__restrict__ s,
-                                 const float *__restrict__ logd, const float *__restrict__ rsum,
-                                 const float *__restrict__ mean_logd, const float *__restrict__ rms,
-                                 const double *__restrict__ xyz, const float *__restrict__ P,
-                                 __nv_bfloat16 *__restrict__ h0)
+// features and input layer, BF16 output: h0 = relu(f W_in + b_in).  Bound by the store of h0: 8 lanes per row,
+// one 16-byte store each, so a warp writes whole lines; a lane keeps its 8 columns' weights in registers.  (One
+// lane per row stored 32 lines a quarter at a time: 219k rows 18.9 us.)
+__global__ void __launch_bounds__(kBlock) k_gnn_input_bf16(
+    uint32_t n, const double *__restrict__ r, const float *__restrict__ s, const float *__restrict__ logd,
+    const float *__restrict__ rsum, const float *__restrict__ mean_logd, const float *__restrict__ rms,
+    const double *__restrict__ xyz, const float *__restrict__ P, __nv_bfloat16 *__restrict__ h0)
 {
-    __shared__ float w[F * H + H];
-    for (int k = threadIdx.x; k < F * H + H; k += blockDim.x) w[k] = P[k];
-    __syncthreads();
+    const uint32_t lane = threadIdx.x & 31u, c8 = lane & 7u;
+    float w[F][8], bias[8];
+#pragma unroll
+    for (int t = 0; t < 8; t++) {
+#pragma unroll
+        for (int k = 0; k < F; k++) w[k][t] = P[k * H + c8 * 8 + t];
+        bias[t] = P[F * H + c8 * 8 + t];
+    }
+    pdl_release();
+    pdl_wait();
     const float inv = 1.0f / *rms, ml = *mean_logd;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+    for (uint32_t base = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32; base < n; base += warps * 32) {
+        const uint32_t i = min(base + lane, n - 1);  // the row whose features this lane loads
         float f[F];
         f[0] = float(r[i] * double(s[i])) * inv;
         f[1] = logd[i] - ml;
@@ -124,25 +153,29 @@ __global__ void k_gnn_input_bf16(uint32_t n, const double *__restrict__ r, const
         f[5] = xyz ? float(xyz[3 * size_t(i) + 2]) : 0.f;
         f[6] = 1.f;
         f[7] = 0.f;
-        uint4 *dst = reinterpret_cast<uint4 *>(h0 + size_t(i) * H);
-#pragma unroll 1
-        for (int c8 = 0; c8 < H / 8; c8++) {
+#pragma unroll 2
+        for (int g = 0; g < 8; g++) {  // four rows at a time
+            const uint32_t from = uint32_t(g * 4) + (lane >> 3), row = base + from;
             float o[8];
 #pragma unroll
-            for (int t = 0; t < 8; t++) {
-                const int c = c8 * 8 + t;
-                float z = w[F * H + c];
+            for (int t = 0; t < 8; t++) o[t] = bias[t];
 #pragma unroll
-                for (int k = 0; k < F; k++) z = fmaf(f[k], w[k * H + c], z);
-                o[t] = fmaxf(z, 0.f);
+            for (int k = 0; k < F; k++) {
+                const float fk = k < 6 ? __shfl_sync(0xffffffffu, f[k], int(from)) : f[k];
+#pragma unroll
+                for (int t = 0; t < 8; t++) o[t] = fmaf(fk, w[k][t], o[t]);
             }
-            dst[c8] = make_uint4(pack2(o[0], o[1]), pack2(o[2], o[3]), pack2(o[4], o[5]), pack2(o[6], o[7]));
+#pragma unroll
+            for (int t = 0; t < 8; t++) o[t] = fmaxf(o[t], 0.f);
+            if (row < n)
+                reinterpret_cast<uint4 *>(h0 + size_t(row) * H)[c8] =
+                    make_uint4(pack2(o[0], o[1]), pack2(o[2], o[3]), pack2(o[4], o[5]), pack2(o[6], o[7]));
         }
     }
 }
 
 template <bool LAST>
-__global__ void __launch_bounds__(kThreads) k_gnn_layer_umma(
+__global__ void __launch_bounds__(kThreads, kCtasPerSm) k_gnn_layer_umma(
     uint32_t n, const uint32_t *__restrict__ rp, const uint32_t *__restrict__ ci, const float *__restrict__ ew,
     const float *__restrict__ s, const __nv_bfloat16 *__restrict__ h, const float *__restrict__ W,
     const float *__restrict__ bias, const float *__restrict__ pout, const float *__restrict__ rms,
@@ -158,10 +191,15 @@ __global__ void __launch_bounds__(kThreads) k_gnn_layer_umma(
     uint32_t *tslot = reinterpret_cast<uint32_t *>(sm + kOffTmem);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
-    // B = W^T (N = 64 output columns x K = 128), BF16, K-major
-    for (int e = tid; e < K2 * H; e += kThreads) {
-        const int k = e / H, c = e % H;
-        *reinterpret_cast<__nv_bfloat16 *>(Bt + tile_off(c, k)) = __float2bfloat16_rn(W[e]);
+    // B = W^T (N = 64 output columns x K = 128), BF16, K-major: 8 values of k, one 16-byte store, at a time
+#pragma unroll
+    for (int e = tid; e < K2 / 8 * H; e += kThreads) {
+        const int k = e / H * 8, c = e % H;
+        float x[8];
+#pragma unroll
+        for (int t = 0; t < 8; t++) x[t] = W[(k + t) * H + c];
+        *reinterpret_cast<uint4 *>(Bt + tile_off(c, k)) =
+            make_uint4(pack2(x[0], x[1]), pack2(x[2], x[3]), pack2(x[4], x[5]), pack2(x[6], x[7]));
     }
     if (tid < H) {
         bs[tid] = bias[tid];
@@ -181,44 +219,48 @@ __global__ void __launch_bounds__(kThreads) k_gnn_layer_umma(
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    pdl_release();  // the next layer's CTAs stage their weights in the slots that these leave
     const uint32_t tmem = *tslot;
     const float b_out = LAST ? pout[H] : 0.f;
-    const float sc = LAST ? *rms : 0.f;
     const uint32_t tiles = (n + kTileRows - 1) / kTileRows;
     const int q = lane >> 3, kc = lane & 7;  // gather: 4 rows per warp pass, 8 lanes x 16 B per row
     const int quarter = warp & 3, half = warp >> 2;
     uint32_t phase = 0;
     bool in_flight = false, failed = false;
 
+    bool waited = false;
+    float sc = 0.f;
+
     for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
         const uint32_t r0 = tile * kTileRows;
         // 1. gather m = G h and stage [h | m] (BF16) in the A tile.  The 8 lanes of a row
         //    fetch 8 of its (column, weight) pairs at once and then 8 neighbour rows
-        //    back to back, so each lane keeps 8 independent 16-byte loads in flight.
+        //    back to back, so each lane keeps 8 independent 16-byte loads in flight.  The
+        //    next 8 pairs (of this row, or of the next pass's) are loaded behind them.
+        const uint32_t rpv = rp[min(r0 + uint32_t(warp * 16 + min(lane, 16)), n)];  // the warp's 16 rows
+        uint32_t jb = __shfl_sync(0xffffffffu, rpv, q), je = __shfl_sync(0xffffffffu, rpv, q + 1);
+        uint32_t row = r0 + uint32_t(warp * 16 + q), rown = row < n ? row : 0u;
+        uint32_t c_mine = rown;
+        float w_mine = 0.f;
+        if (jb + uint32_t(kc) < je) {  // the diagonal's weight is 0
+            c_mine = ci[jb + kc];
+            w_mine = ew[jb + kc];
+        }
+        if (!waited) {  // h of the preceding kernel from here on
+            pdl_wait();
+            waited = true;
+            if (LAST) sc = *rms;
+        }
 #pragma unroll 1
         for (int pass = 0; pass < 4; pass++) {
             const uint32_t trow = uint32_t(warp * 16 + pass * 4 + q);
-            const uint32_t row = r0 + trow;
             float acc[8];
 #pragma unroll
             for (int t = 0; t < 8; t++) acc[t] = 0.f;
-            uint4 hown = make_uint4(0u, 0u, 0u, 0u);
-            uint32_t jb = 0, je = 0;
-            if (row < n) {
-                hown = *reinterpret_cast<const uint4 *>(h + size_t(row) * H + kc * 8);
-                jb = rp[row];
-                je = rp[row + 1];
-            }
-            const uint32_t trips = __reduce_max_sync(0xffffffffu, (je - jb + 7) / 8);
-            const uint32_t rown = row < n ? row : 0u;
+            const uint4 hown =
+                row < n ? *reinterpret_cast<const uint4 *>(h + size_t(row) * H + kc * 8) : make_uint4(0u, 0u, 0u, 0u);
+            const uint32_t trips = max(__reduce_max_sync(0xffffffffu, (je - jb + 7) / 8), 1u);
             for (uint32_t it = 0; it < trips; it++) {
-                const uint32_t jj = jb + it * 8 + uint32_t(kc);
-                uint32_t c_mine = rown;
-                float w_mine = 0.f;
-                if (jj < je) {  // the diagonal's weight is 0
-                    c_mine = ci[jj];
-                    w_mine = ew[jj];
-                }
                 uint4 hv[8];
                 float wt[8];
 #pragma unroll
@@ -226,6 +268,20 @@ __global__ void __launch_bounds__(kThreads) k_gnn_layer_umma(
                     const uint32_t ct = __shfl_sync(0xffffffffu, c_mine, (lane & ~7) + t);
                     wt[t] = __shfl_sync(0xffffffffu, w_mine, (lane & ~7) + t);
                     hv[t] = *reinterpret_cast<const uint4 *>(h + size_t(ct) * H + kc * 8);
+                }
+                jb += 8;
+                if (it + 1 == trips) {  // the next pass's row
+                    const int src = min((pass + 1) * 4 + q, 15);
+                    jb = __shfl_sync(0xffffffffu, rpv, src);
+                    je = __shfl_sync(0xffffffffu, rpv, src + 1);
+                    row = r0 + uint32_t(warp * 16 + src);
+                    rown = row < n ? row : 0u;
+                }
+                c_mine = rown;
+                w_mine = 0.f;
+                if (jb + uint32_t(kc) < je) {
+                    c_mine = ci[jb + kc];
+                    w_mine = ew[jb + kc];
                 }
 #pragma unroll
                 for (int t = 0; t < 8; t++) {
@@ -235,8 +291,8 @@ __global__ void __launch_bounds__(kThreads) k_gnn_layer_umma(
                     for (int u = 0; u < 8; u++) acc[u] = fmaf(wt[t], f[u], acc[u]);
                 }
             }
-            *reinterpret_cast<uint4 *>(At + tile_off(trow, kc * 8)) = hown;
-            *reinterpret_cast<uint4 *>(At + tile_off(trow, H + kc * 8)) =
+            *reinterpret_cast<uint4 *>(At + a_off(trow, kc * 8)) = hown;
+            *reinterpret_cast<uint4 *>(At + a_off(trow, H + kc * 8)) =
                 make_uint4(pack2(acc[0], acc[1]), pack2(acc[2], acc[3]), pack2(acc[4], acc[5]),
                            pack2(acc[6], acc[7]));
         }
@@ -248,7 +304,8 @@ __global__ void __launch_bounds__(kThreads) k_gnn_layer_umma(
             const uint32_t a0 = smem_u32(At), b0 = smem_u32(Bt);
 #pragma unroll
             for (int ks = 0; ks < K2 / 16; ks++)
-                umma_bf16(tmem, smem_desc(a0 + ks * 2 * kLBO), smem_desc(b0 + ks * 2 * kLBO), ks > 0 ? 1u : 0u);
+                umma_bf16(tmem, smem_desc(a0 + ks * 2 * kALBO, kALBO, kASBO), smem_desc(b0 + ks * 2 * kLBO),
+                          ks > 0 ? 1u : 0u);
             umma_commit(bar);
         }
         in_flight = true;
@@ -261,36 +318,42 @@ __global__ void __launch_bounds__(kThreads) k_gnn_layer_umma(
         phase ^= 1u;
         tc_fence_after();
         // 3. epilogue: warp (quarter, half) reads TMEM lanes 32*quarter.., columns 32*half..
-        const uint32_t trow = uint32_t(quarter * 32 + lane), row = r0 + trow;
+        const uint32_t orow = uint32_t(quarter * 32 + lane);
         uint32_t v[32];
         tmem_ld32(tmem + (uint32_t(quarter * 32) << 16) + uint32_t(half * 32), v);
-        float o[32];
         float dot = 0.f;
 #pragma unroll
         for (int c8 = 0; c8 < 4; c8++) {
             const int cb = half * 32 + c8 * 8;
-            float hp[8];
-            unpack8(*reinterpret_cast<const uint4 *>(At + tile_off(trow, cb)), hp);
+            uint4 *own = reinterpret_cast<uint4 *>(At + a_off(orow, cb));
+            float hp[8], bc[8], o[8];
+            unpack8(*own, hp);
+            *reinterpret_cast<float4 *>(bc) = *reinterpret_cast<const float4 *>(bs + cb);
+            *reinterpret_cast<float4 *>(bc + 4) = *reinterpret_cast<const float4 *>(bs + cb + 4);
 #pragma unroll
             for (int t = 0; t < 8; t++) {
-                const int c = cb + t;
-                const float val_o = hp[t] + fmaxf(__uint_as_float(v[c8 * 8 + t]) + bs[c], 0.f);
-                o[c8 * 8 + t] = val_o;
-                dot = fmaf(val_o, wo[c], dot);
+                o[t] = hp[t] + fmaxf(__uint_as_float(v[c8 * 8 + t]) + bc[t], 0.f);
+                if (LAST) dot = fmaf(o[t], wo[cb + t], dot);
             }
+            if (!LAST) *own = make_uint4(pack2(o[0], o[1]), pack2(o[2], o[3]), pack2(o[4], o[5]), pack2(o[6], o[7]));
         }
         if constexpr (!LAST) {
-            if (row < n) {
-                uint4 *dst = reinterpret_cast<uint4 *>(h_out + size_t(row) * H + half * 32);
+            // out through the tile's h half, where each thread has replaced what it alone read: the warp's 32 rows
+            // of 64 bytes, 4 lanes a row (rows 4 apart in a quarter warp, so no bank conflicts)
+            __syncwarp();
+            const uint32_t sub = uint32_t(lane >> 2), ch = uint32_t(half * 4 + (lane & 3));
 #pragma unroll
-                for (int c8 = 0; c8 < 4; c8++)
-                    dst[c8] = make_uint4(pack2(o[c8 * 8], o[c8 * 8 + 1]), pack2(o[c8 * 8 + 2], o[c8 * 8 + 3]),
-                                         pack2(o[c8 * 8 + 4], o[c8 * 8 + 5]), pack2(o[c8 * 8 + 6], o[c8 * 8 + 7]));
+            for (int it = 0; it < 4; it++) {
+                const uint32_t t = uint32_t(quarter * 32 + it * 8) + (sub >> 1) + (sub & 1u) * 4;
+                if (r0 + t < n)
+                    reinterpret_cast<uint4 *>(h_out + size_t(r0 + t) * H)[ch] =
+                        *reinterpret_cast<const uint4 *>(At + a_off(t, ch * 8));
             }
         } else {
-            if (half == 1) part[trow] = dot;
+            if (half == 1) part[orow] = dot;
             __syncthreads();
-            if (half == 0 && row < n) z[row] = double(dot + part[trow] + b_out) * double(sc) * double(s[row]);
+            if (half == 0 && r0 + orow < n)
+                z[r0 + orow] = double(dot + part[orow] + b_out) * double(sc) * double(s[r0 + orow]);
         }
         tc_fence_before();
         __syncthreads();  // A tile, TMEM and part[] free for the next tile
@@ -314,7 +377,7 @@ bool gnn_umma_setup(rsg_context *ctx, int *grid)
     if (!attr) {
         for (const void *f : {(const void *)k_gnn_layer_umma<false>, (const void *)k_gnn_layer_umma<true>}) {
             if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kLayerSmem)) != cudaSuccess ||
-                cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, 100) != cudaSuccess)
+                cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, kCarveout) != cudaSuccess)
                 return false;
         }
         attr = true;
@@ -324,11 +387,7 @@ bool gnn_umma_setup(rsg_context *ctx, int *grid)
             cudaSuccess ||
         per_sm < 1)
         return false;
-    // Four CTAs fit an SM by shared memory and registers; CTAs beyond the resident
-    // ones wait for a slot, so a larger grid never over-commits the 512 TMEM columns
-    // (each resident CTA holds kTmemCols of them).
-    per_sm = std::min(std::max(per_sm, 4), int(512 / kTmemCols));
-    *grid = per_sm * ctx->num_sms;
+    *grid = kCtasPerSm * ctx->num_sms;
     return true;
 }
 
@@ -342,19 +401,17 @@ rsg_status gnn_forward_umma(rsg_context *ctx, rsg_learned *G, const rsg_csr *A, 
     if (!gnn_umma_setup(ctx, &gl)) return set_error(ctx, RSG_ERR_CUDA, "learned: tensor-core layer set-up");
     const uint32_t tiles = (n + kTileRows - 1) / kTileRows;
     gl = int(std::min<uint32_t>(uint32_t(gl), std::max<uint32_t>(tiles, 1)));
-    const int gi = std::min(grid_for(ctx, (const void *)k_gnn_input_bf16, kBlock, 0, n), kMaxGrid);
-    k_gnn_input_bf16<<<gi, kBlock, 0, sm>>>(n, r, G->s, G->logd, G->rsum, G->scal32, rms, xyz, G->params, G->hb[0]);
+    const int gi = std::min(grid_for(ctx, (const void *)k_gnn_input_bf16, kBlock, 0, (long long)n * 8), kMaxGrid);
+    launch_k(sm, true, k_gnn_input_bf16, gi, kBlock, 0, n, r, (const float *)G->s, (const float *)G->logd,
+           (const float *)G->rsum, (const float *)G->scal32, rms, xyz, (const float *)G->params, G->hb[0]);
     for (int l = 0; l < G->L; l++) {
         const float *W = G->params + off_layer(l), *b = W + size_t(K2) * H;
         const float *pout = G->params + off_layer(G->L);
         const __nv_bfloat16 *hin = G->hb[l & 1];
         __nv_bfloat16 *hout = G->hb[(l + 1) & 1];
-        if (l + 1 < G->L)
-            k_gnn_layer_umma<false><<<gl, kThreads, kLayerSmem, sm>>>(n, A->rp, A->ci, G->ew, G->s, hin, W, b, pout,
-                                                                     rms, hout, z, ctx->errw);
-        else
-            k_gnn_layer_umma<true><<<gl, kThreads, kLayerSmem, sm>>>(n, A->rp, A->ci, G->ew, G->s, hin, W, b, pout,
-                                                                    rms, hout, z, ctx->errw);
+        launch_k(sm, true, l + 1 < G->L ? k_gnn_layer_umma<false> : k_gnn_layer_umma<true>, gl, kThreads, kLayerSmem, n,
+               (const uint32_t *)A->rp, (const uint32_t *)A->ci, (const float *)G->ew, (const float *)G->s, hin, W, b,
+               pout, rms, hout, z, ctx->errw);
     }
     RSG_CHECK_CUDA(ctx, cudaGetLastError());
     return RSG_OK;
