@@ -701,16 +701,18 @@ rsg_status build_loop_graph(rsg_context *ctx, const CgArgs &a, const Launch &L, 
 }
 
 template <int RPW, int PK>
-rsg_status run_typed(rsg_context *ctx, const CgArgs &a, double *seconds)
+rsg_status run_typed(rsg_context *ctx, const CgArgs &a)
 {
     Launch L;
     L.s64 = a.A->use_sell ? 0 : tma_smem<double>();
     L.s32 = a.A->use_sell ? 0 : tma_smem<float>();
-    set_smem(k_cg_init_res<RPW>, tma_smem<double>());
-    set_smem(k_cg_dir<RPW>, tma_smem<double>());
-    set_smem(k_cg_check<RPW, PK>, tma_smem<double>());
-    set_smem(k_mx_dir<RPW>, tma_smem<float>());
-    set_smem(k_mx_check<RPW, PK>, tma_smem<double>());
+    if (!a.A->use_sell) {
+        set_smem(k_cg_init_res<RPW>, tma_smem<double>());
+        set_smem(k_cg_dir<RPW>, tma_smem<double>());
+        set_smem(k_cg_check<RPW, PK>, tma_smem<double>());
+        set_smem(k_mx_dir<RPW>, tma_smem<float>());
+        set_smem(k_mx_check<RPW, PK>, tma_smem<double>());
+    }
     const long long chunk_threads = (long long)a.A->n * 32 / RPW;
     (void)chunk_threads;
     L.g_spmv64 = spmv_grid(ctx, a.A, (const void *)k_cg_dir<RPW>, L.s64, RPW);
@@ -742,8 +744,6 @@ rsg_status run_typed(rsg_context *ctx, const CgArgs &a, double *seconds)
     if (persisted) {
         if (a.mixed) k_mx_fold<<<L.g_vec, kBlock, 0, ctx->stream>>>(a.A->n, a.x, a.y32, a.st);
         RSG_CHECK_CUDA(ctx, cudaEventRecord(ctx->ev[1], ctx->stream));
-        const cudaError_t e = cudaStreamSynchronize(ctx->stream);
-        if (e != cudaSuccess) return set_error(ctx, RSG_ERR_CUDA, "solve: %s", cudaGetErrorString(e));
     } else if (a.use_graph) {
         cudaGraph_t graph = nullptr;
         cudaGraphExec_t exec = nullptr;
@@ -782,13 +782,17 @@ rsg_status run_typed(rsg_context *ctx, const CgArgs &a, double *seconds)
         RSG_CHECK_CUDA(ctx, cudaEventRecord(ctx->ev[1], ctx->stream));
         RSG_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     }
-    float ms = 0.f;
-    cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[1]);
-    *seconds = ms * 1e-3;
     return RSG_OK;
 }
 
 }  // namespace
+
+double cg_seconds(rsg_context *ctx)
+{
+    float ms = 0.f;
+    cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[1]);
+    return ms * 1e-3;
+}
 
 namespace {
 
@@ -913,17 +917,17 @@ rsg_status profile_typed(rsg_context *ctx, const rsg_csr *A, int kernel, uint32_
 
 }  // namespace
 
-rsg_status cg_run(rsg_context *ctx, const CgArgs &a, double *seconds)
+rsg_status cg_run(rsg_context *ctx, const CgArgs &a)
 {
     const int rpw = pick_rpw(a.A);
     switch (a.P.kind) {
-    case 0: RSG_RPW_DISPATCH(rpw, return (run_typed<RPW, 0>(ctx, a, seconds)));
-    case 1: RSG_RPW_DISPATCH(rpw, return (run_typed<RPW, 1>(ctx, a, seconds)));
+    case 0: RSG_RPW_DISPATCH(rpw, return (run_typed<RPW, 0>(ctx, a)));
+    case 1: RSG_RPW_DISPATCH(rpw, return (run_typed<RPW, 1>(ctx, a)));
     case 3:
         if (!a.mixed || !a.amg)
             return set_error(ctx, RSG_ERR_UNSUPPORTED, "the multilevel preconditioner runs in the mixed-precision CG");
-        RSG_RPW_DISPATCH(rpw, return (run_typed<RPW, 3>(ctx, a, seconds)));
-    default: RSG_RPW_DISPATCH(rpw, return (run_typed<RPW, 2>(ctx, a, seconds)));
+        RSG_RPW_DISPATCH(rpw, return (run_typed<RPW, 3>(ctx, a)));
+    default: RSG_RPW_DISPATCH(rpw, return (run_typed<RPW, 2>(ctx, a)));
     }
     return RSG_ERR_UNSUPPORTED;
 }

@@ -27,6 +27,8 @@ struct Arena {
 
 }  // namespace rsg
 
+constexpr size_t kPinnedDoubles = 128;
+
 struct rsg_context {
     int device = 0;
     cudaStream_t stream = nullptr;
@@ -34,11 +36,18 @@ struct rsg_context {
     int num_sms = 0;
     std::string last_error;
     rsg::Arena ws;                    // per-solve workspace
-    double *pinned = nullptr;         // small pinned host buffer for readbacks (64 doubles)
+    double *pinned = nullptr;         // small pinned host buffer for readbacks (kPinnedDoubles)
     unsigned int *errw = nullptr;     // device word: set when a kernel's bounded wait ran out
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
     double *persist = nullptr;        // persistent CG loop: phase partials and barrier words (cg_persist.cu)
     int coop_graph = -1;              // a cooperative launch can be captured in a graph: -1 not probed, 0 no, 1 yes
+    struct Occupancy {
+        const void *kernel;
+        int block;
+        size_t smem;
+        int per_sm;
+    };
+    std::vector<Occupancy> occupancy; // grid_for's answers so far
 };
 
 struct rsg_csr {

@@ -36,9 +36,15 @@ rsg_status arena_reserve(rsg_context *ctx, size_t bytes)
 
 int grid_for(rsg_context *ctx, const void *kernel, int block, size_t smem, long long work_items)
 {
+    // asked of the driver once per kernel and launch shape (about 1 us each, a dozen per solve)
     int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, smem) != cudaSuccess || per_sm < 1)
-        per_sm = 1;
+    for (const rsg_context::Occupancy &o : ctx->occupancy)
+        if (o.kernel == kernel && o.block == block && o.smem == smem) per_sm = o.per_sm;
+    if (per_sm == 0) {
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, smem) != cudaSuccess || per_sm < 1)
+            per_sm = 1;
+        ctx->occupancy.push_back({kernel, block, smem, per_sm});
+    }
     long long full = (long long)per_sm * ctx->num_sms;
     long long need = (work_items + block - 1) / block;
     if (need < 1) need = 1;
@@ -65,7 +71,7 @@ rsg_status rsg_context_create(int device, rsg_context **out)
         return RSG_ERR_CUDA;
     }
     ctx->own_stream = true;
-    if (cudaMallocHost(&ctx->pinned, 64 * sizeof(double)) != cudaSuccess) {
+    if (cudaMallocHost(&ctx->pinned, kPinnedDoubles * sizeof(double)) != cudaSuccess) {
         cudaStreamDestroy(ctx->stream);
         delete ctx;
         return RSG_ERR_CUDA;

@@ -74,7 +74,7 @@ __global__ void __launch_bounds__(kBlock) k_spmv(Csr<V> M, Sell<V> S, int use_se
 }
 
 __global__ void k_jacobi(uint32_t n, const uint32_t *__restrict__ rp, const uint32_t *__restrict__ ci,
-                         const double *__restrict__ val, double *__restrict__ d)
+                         const double *__restrict__ val, double *__restrict__ d, float *__restrict__ d32)
 {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         double inv = 0.0;
@@ -85,6 +85,7 @@ __global__ void k_jacobi(uint32_t n, const uint32_t *__restrict__ rp, const uint
                 break;
             }
         d[i] = inv;
+        if (d32) d32[i] = float(inv);
     }
 }
 
@@ -359,10 +360,10 @@ rsg_status spmv32(rsg_context *ctx, const rsg_csr *A, const float *x, float *y, 
     return RSG_OK;
 }
 
-rsg_status jacobi_build(rsg_context *ctx, const rsg_csr *A, double *d)
+rsg_status jacobi_build(rsg_context *ctx, const rsg_csr *A, double *d, float *d32)
 {
     const int grid = grid_for(ctx, (const void *)k_jacobi, kBlock, 0, A->n);
-    k_jacobi<<<grid, kBlock, 0, ctx->stream>>>(A->n, A->rp, A->ci, A->val, d);
+    k_jacobi<<<grid, kBlock, 0, ctx->stream>>>(A->n, A->rp, A->ci, A->val, d, d32);
     RSG_CHECK_CUDA(ctx, cudaGetLastError());
     return RSG_OK;
 }

@@ -48,7 +48,8 @@ rsg_status csr_create_ex(rsg_context *ctx, uint32_t n, const uint32_t *rp, const
                          int32_t memory, int sell_mode, rsg_csr **out);
 // Recompute ||A||_F and the FP32 copy after the values were rewritten in place.
 rsg_status csr_refresh(rsg_context *ctx, rsg_csr *A);
-rsg_status jacobi_build(rsg_context *ctx, const rsg_csr *A, double *d);
+// Inverse diagonal, and its FP32 copy when d32 is given.
+rsg_status jacobi_build(rsg_context *ctx, const rsg_csr *A, double *d, float *d32 = nullptr);
 // Frees a matrix's multilevel preconditioner hierarchy (amg.cu).
 void amg_release(void *hierarchy);
 uint32_t block_width(uint32_t n, uint32_t block_size);

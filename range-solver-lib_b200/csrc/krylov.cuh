@@ -98,7 +98,10 @@ void launch_k(cudaStream_t stream, bool pdl, void (*k)(P...), dim3 grid, int blo
     cudaLaunchKernelEx(&cfg, k, std::forward<A>(args)...);
 }
 
-rsg_status cg_run(rsg_context *ctx, const CgArgs &a, double *seconds);
+// Runs the loop from the state *a.st.  The cooperative loops are only queued (the caller synchronises once,
+// behind what it queues after them); cg_seconds is the loop's time, valid after that.
+rsg_status cg_run(rsg_context *ctx, const CgArgs &a);
+double cg_seconds(rsg_context *ctx);
 // The CG loop as one persistent cooperative kernel (cg_persist.cu), bit for bit the graph loop's
 // results with the same grids; *ran = false when it could not be launched (nothing was).
 rsg_status cg_persist_run(rsg_context *ctx, const CgArgs &a, int g_dir, int g_upd, int g_chk, bool *ran);

@@ -19,20 +19,43 @@
 
 namespace rsg {
 
+// out[0] = ||b||; the equation scale 1e9 ||A|| / ||b|| (1 when off or undefined) and its reciprocal to out[1], out[2]:
+// what follows is queued without the host having seen them.
 __global__ void k_norm2(uint32_t n, const double *__restrict__ v, double *partials, unsigned int *ticket,
-                        double *out)
+                        double *out, double an, int scaled)
 {
     __shared__ double sh[32];
     double acc[1] = {0.0};
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
         acc[0] += v[i] * v[i];
     double tot[1];
-    if (grid_sum<1>(acc, partials, ticket, sh, tot) && threadIdx.x == 0) *out = sqrt(tot[0]);
+    if (grid_sum<1>(acc, partials, ticket, sh, tot) && threadIdx.x == 0) {
+        const double bn = sqrt(tot[0]);
+        const double s = scaled && bn != 0.0 && an != 0.0 ? 1.0e9 / fabs(bn / an) : 1.0;
+        out[0] = bn;
+        out[1] = s;
+        out[2] = 1.0 / s;
+    }
 }
 
-__global__ void k_scale(uint32_t n, const double *__restrict__ src, double *__restrict__ dst, double s)
+// y = s b, x = s x with s = sc[1]; the loop's initial state to *st (by value: no copy from pageable memory).
+__global__ void k_start(uint32_t n, const double *__restrict__ b, double *__restrict__ y, double *__restrict__ x,
+                        const double *__restrict__ sc, CgState init, CgState *st)
 {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) dst[i] = src[i] * s;
+    const double s = sc[1];
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        y[i] = b[i] * s;
+        if (s != 1.0) x[i] = x[i] * s;
+    }
+    if (st && blockIdx.x == 0 && threadIdx.x == 0) *st = init;
+}
+
+// x = x / s (sc[2] = 1 / s)
+__global__ void k_unscale(uint32_t n, double *__restrict__ x, const double *__restrict__ sc)
+{
+    if (sc[1] == 1.0) return;
+    const double s = sc[2];
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) x[i] = x[i] * s;
 }
 
 __global__ void k_to_f32(size_t n, const double *__restrict__ src, float *__restrict__ dst)
@@ -141,14 +164,26 @@ extern "C" rsg_status rsg_solve(rsg_context *ctx, rsg_csr *A, const rsg_solver_c
     double *y = arena_take<double>(ctx, n);
     double *d = arena_take<double>(ctx, size_t(n) * w);
     double *partials = arena_take<double>(ctx, size_t(4) * kMaxGrid * 32);
-    CgState *cst = arena_take<CgState>(ctx, 1);
     GmresState *gst = arena_take<GmresState>(ctx, 1);
+    // cleared with one memset: scalars and tickets, the CG state (next to them: read back together) and the
+    // direction vectors
+    const bool cg = !gmres && !learned;
     double *scal = arena_take<double>(ctx, 64);
+    CgState *cst = arena_take<CgState>(ctx, 1);
+    double *p0 = cg ? arena_take<double>(ctx, n) : nullptr, *p1 = cg ? arena_take<double>(ctx, n) : nullptr;
+    float *p32a = nullptr, *p32b = nullptr, *y32 = nullptr;
+    if (cg && mixed) {
+        p32a = arena_take<float>(ctx, n);
+        p32b = arena_take<float>(ctx, n);
+        y32 = arena_take<float>(ctx, n);
+    }
+    const size_t cleared = ctx->ws.base + ctx->ws.used - reinterpret_cast<char *>(scal);
+    float *d32 = mixed && !gmres ? arena_take<float>(ctx, size_t(n) * w) : nullptr;
     double *hist = want_hist ? arena_take<double>(ctx, hist_len) : nullptr;
     double *thist = want_hist ? arena_take<double>(ctx, hist_len) : nullptr;
     unsigned int *ticket = reinterpret_cast<unsigned int *>(scal + 32);
 
-    RSG_CHECK_CUDA(ctx, cudaMemsetAsync(scal, 0, 64 * sizeof(double), ctx->stream));
+    RSG_CHECK_CUDA(ctx, cudaMemsetAsync(scal, 0, cleared, ctx->stream));
     if (memory == RSG_MEM_HOST) {
         RSG_CHECK_CUDA(ctx, cudaMemcpyAsync(b_dev, b, size_t(n) * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
         RSG_CHECK_CUDA(ctx, cudaMemcpyAsync(x_dev, x, size_t(n) * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
@@ -161,7 +196,7 @@ extern "C" rsg_status rsg_solve(rsg_context *ctx, rsg_csr *A, const rsg_solver_c
     if (prec_type == RSG_PREC_AMG) {
         RSG_TRY(amg_setup(ctx, A, c.persistent > 0));  // rebuilt from the current values on every solve
     } else if (prec_type == RSG_PREC_JACOBI || learned) {
-        RSG_TRY(jacobi_build(ctx, A, d));
+        RSG_TRY(jacobi_build(ctx, A, d, d32));
     } else if (prec_type == RSG_PREC_BLOCK_JACOBI) {
         unsigned int *flag = ticket + 8;
         RSG_TRY(block_jacobi_build(ctx, A, w, d, flag));
@@ -173,23 +208,35 @@ extern "C" rsg_status rsg_solve(rsg_context *ctx, rsg_csr *A, const rsg_solver_c
     P.d = d;
 
     // ---- equation scaling ----
-    {
-        const int g = std::min(grid_for(ctx, (const void *)k_norm2, kBlock, 0, n), kMaxGrid);
-        k_norm2<<<g, kBlock, 0, ctx->stream>>>(n, b_dev, partials, ticket, scal);
-        RSG_CHECK_CUDA(ctx, cudaGetLastError());
-        RSG_CHECK_CUDA(ctx, cudaMemcpyAsync(ctx->pinned, scal, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-        RSG_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    }
-    const double bn = ctx->pinned[0], an = A->norm;
-    double scale = 1.0;
-    if (c.scale_equations && bn != 0.0 && an != 0.0) scale = 1.0e9 / std::abs(bn / an);
-    st_out.norm_a = an;
-    st_out.norm_b = bn;
-    st_out.equation_scale = scale;
-    const int gv = std::min(grid_for(ctx, (const void *)k_scale, kBlock, 0, n), kMaxGrid);
-    k_scale<<<gv, kBlock, 0, ctx->stream>>>(n, b_dev, y, scale);
-    if (scale != 1.0) k_scale<<<gv, kBlock, 0, ctx->stream>>>(n, x_dev, x_dev, scale);
+    const double an = A->norm;
+    CgState h;
+    std::memset(&h, 0, sizeof(h));
+    h.an = an;
+    h.cvg = c.cvg;
+    h.eps = c.eps;
+    h.rtol = c.rtol;
+    h.delta = c.reliable_delta > 0.0 && c.reliable_delta < 1.0 ? c.reliable_delta : kReliableDelta;
+    h.sigma = 1.0;
+    h.max_it = max_it;
+    h.stop_rule = c.stop_rule;
+    h.body_limit = max_it + 16;  // a body makes at least one iteration
+    h.history = hist;
+    h.trend_hist = thist;
+    h.evict_first32 = c.l2_resident_f32 ? 0 : 1;
+    h.auto_switch = c.precision == RSG_PRECISION_AUTO ? 1 : 0;
+    const CgState h_init = h;
+    const int gn = std::min(grid_for(ctx, (const void *)k_norm2, kBlock, 0, n), kMaxGrid);
+    k_norm2<<<gn, kBlock, 0, ctx->stream>>>(n, b_dev, partials, ticket, scal, an, c.scale_equations != 0);
+    const int gv = std::min(grid_for(ctx, (const void *)k_start, kBlock, 0, n), kMaxGrid);
+    k_start<<<gv, kBlock, 0, ctx->stream>>>(n, b_dev, y, x_dev, scal, h_init, cg ? cst : nullptr);
     RSG_CHECK_CUDA(ctx, cudaGetLastError());
+    // scalars and state, in pinned memory after the next synchronisation
+    auto read_back = [&]() {
+        return cudaMemcpyAsync(ctx->pinned, scal, 64 * sizeof(double) + sizeof(CgState), cudaMemcpyDeviceToHost,
+                               ctx->stream);
+    };
+    static_assert(64 * sizeof(double) + sizeof(CgState) <= kPinnedDoubles * sizeof(double), "pinned readback");
+    static_assert(64 * sizeof(double) % 256 == 0, "the state follows the scalars");
 
     if (c.learned_initial_guess) {
         // x0 = M(b): the network's estimate of A^{-1} b (M is positively homogeneous,
@@ -197,7 +244,9 @@ extern "C" rsg_status rsg_solve(rsg_context *ctx, rsg_csr *A, const rsg_solver_c
         RSG_TRY(gnn_forward(ctx, G, A, y, x_dev, nullptr, false, true));
     }
 
-    double solve_seconds = 0.0;
+    double solve_seconds = 0.0, first_seconds = 0.0;
+    int32_t switched = 0;                // precision AUTO: iterations and updates before the switch to FP64
+    uint32_t cg_used = 0, cg_outer = 0;
     rsg_status solve_status = RSG_OK;
     if (learned && !gmres) {
         FcgResult fr;
@@ -218,27 +267,21 @@ extern "C" rsg_status rsg_solve(rsg_context *ctx, rsg_csr *A, const rsg_solver_c
         a.st = cst;
         a.r = arena_take<double>(ctx, n);
         a.z = arena_take<double>(ctx, n);
-        a.p0 = arena_take<double>(ctx, n);
-        a.p1 = arena_take<double>(ctx, n);
+        a.p0 = p0;
+        a.p1 = p1;
         a.q = arena_take<double>(ctx, n);
         a.mixed = mixed;
         a.use_graph = c.use_graph != 0;
         a.persistent = c.persistent;
         a.check_interval = std::max<uint32_t>(2, c.check_interval);
-        RSG_CHECK_CUDA(ctx, cudaMemsetAsync(a.p0, 0, size_t(n) * sizeof(double), ctx->stream));
-        RSG_CHECK_CUDA(ctx, cudaMemsetAsync(a.p1, 0, size_t(n) * sizeof(double), ctx->stream));
         if (mixed) {
             a.r32 = arena_take<float>(ctx, n);
             a.z32 = arena_take<float>(ctx, n);
-            a.p32a = arena_take<float>(ctx, n);
-            a.p32b = arena_take<float>(ctx, n);
+            a.p32a = p32a;
+            a.p32b = p32b;
             a.q32 = arena_take<float>(ctx, n);
-            a.y32 = arena_take<float>(ctx, n);
-            float *d32 = arena_take<float>(ctx, size_t(n) * w);
-            RSG_CHECK_CUDA(ctx, cudaMemsetAsync(a.p32a, 0, size_t(n) * sizeof(float), ctx->stream));
-            RSG_CHECK_CUDA(ctx, cudaMemsetAsync(a.p32b, 0, size_t(n) * sizeof(float), ctx->stream));
-            RSG_CHECK_CUDA(ctx, cudaMemsetAsync(a.y32, 0, size_t(n) * sizeof(float), ctx->stream));
-            if (prec_type == RSG_PREC_JACOBI || prec_type == RSG_PREC_BLOCK_JACOBI)
+            a.y32 = y32;
+            if (prec_type == RSG_PREC_BLOCK_JACOBI)
                 k_to_f32<<<gv, kBlock, 0, ctx->stream>>>(size_t(n) * w, d, d32);
             P.d32 = d32;
         }
@@ -249,31 +292,19 @@ extern "C" rsg_status rsg_solve(rsg_context *ctx, rsg_csr *A, const rsg_solver_c
             a.P.d32 = amg_finest_weights(a.amg);  // omega / a_ii: the V-cycle's first smoothing step
             a.amg_x0 = amg_finest_x0(a.amg);
         }
-        CgState h;
-        std::memset(&h, 0, sizeof(h));
-        h.an = an;
-        h.cvg = c.cvg;
-        h.eps = c.eps;
-        h.rtol = c.rtol;
-        h.delta = c.reliable_delta > 0.0 && c.reliable_delta < 1.0 ? c.reliable_delta : kReliableDelta;
-        h.sigma = 1.0;
-        h.max_it = max_it;
-        h.stop_rule = c.stop_rule;
-        h.body_limit = max_it + 16;  // a body makes at least one iteration
-        h.history = hist;
-        h.trend_hist = thist;
-        h.evict_first32 = c.l2_resident_f32 ? 0 : 1;
-        h.auto_switch = c.precision == RSG_PRECISION_AUTO ? 1 : 0;
-        const CgState h_init = h;
-        RSG_CHECK_CUDA(ctx, cudaMemcpyAsync(cst, &h, sizeof(h), cudaMemcpyHostToDevice, ctx->stream));
-        RSG_TRY(cg_run(ctx, a, &solve_seconds));
-        RSG_CHECK_CUDA(ctx, cudaMemcpyAsync(&h, cst, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
-        RSG_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-        uint32_t logged = h.it, outer = h.n_updates;
+        RSG_TRY(cg_run(ctx, a));
+        uint32_t used = 0, outer = 0;
+        if (h_init.auto_switch) {
+            RSG_CHECK_CUDA(ctx, read_back());
+            RSG_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+            std::memcpy(&h, ctx->pinned + 64, sizeof(h));
+            first_seconds = cg_seconds(ctx);
+        }
         if (h.switched) {
             // precision AUTO: the FP32 recurrence drifted -- continue in FP64 from the folded x with the
             // iterations left (fresh directions; the history continues where it stopped)
-            const uint32_t used = h.it;
+            used = h.it;
+            outer = h.n_updates;
             CgArgs a64 = a;
             a64.mixed = false;
             CgState h2 = h_init;
@@ -285,28 +316,11 @@ extern "C" rsg_status rsg_solve(rsg_context *ctx, rsg_csr *A, const rsg_solver_c
             RSG_CHECK_CUDA(ctx, cudaMemsetAsync(a64.p0, 0, size_t(n) * sizeof(double), ctx->stream));
             RSG_CHECK_CUDA(ctx, cudaMemsetAsync(a64.p1, 0, size_t(n) * sizeof(double), ctx->stream));
             RSG_CHECK_CUDA(ctx, cudaMemcpyAsync(cst, &h2, sizeof(h2), cudaMemcpyHostToDevice, ctx->stream));
-            double s2 = 0.0;
-            RSG_TRY(cg_run(ctx, a64, &s2));
-            solve_seconds += s2;
-            RSG_CHECK_CUDA(ctx, cudaMemcpyAsync(&h, cst, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
-            RSG_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-            st_out.fp64_iterations = h.it;
-            logged = used + h.it;
-            outer += h.n_updates;
+            RSG_TRY(cg_run(ctx, a64));
         }
-        st_out.iterations = logged;
-        st_out.outer = outer;
-        st_out.error = h.error;
-        st_out.trend = h.trend;
-        st_out.converged = h.converged;
-        solve_status = h.ticket[7] ? RSG_ERR_TIMEOUT : rsg_status(h.status);
-        if (want_hist) {
-            h.it = logged;
-            std::vector<double> e(h.it), t(h.it);
-            cudaMemcpy(e.data(), hist, h.it * sizeof(double), cudaMemcpyDeviceToHost);
-            cudaMemcpy(t.data(), thist, h.it * sizeof(double), cudaMemcpyDeviceToHost);
-            write_log(c, "Conjugate Gradient", h.it, e.data(), t.data(), h.converged != 0);
-        }
+        switched = h.switched;
+        cg_used = used;
+        cg_outer = outer;
     } else {
         GmresArgs a = {};
         a.A = A;
@@ -359,18 +373,35 @@ extern "C" rsg_status rsg_solve(rsg_context *ctx, rsg_csr *A, const rsg_solver_c
         }
     }
 
-    // ---- unscale, true residual, download ----
-    if (scale != 1.0) k_scale<<<gv, kBlock, 0, ctx->stream>>>(n, x_dev, x_dev, 1.0 / scale);
-    {
-        unsigned int *t2 = ticket + 4;
-        RSG_TRY(true_residual(ctx, A, b_dev, x_dev, partials, t2, scal + 8));
-        RSG_CHECK_CUDA(ctx, cudaMemcpyAsync(ctx->pinned, scal + 8, 3 * sizeof(double), cudaMemcpyDeviceToHost,
-                                            ctx->stream));
-    }
+    // ---- unscale, true residual, download: one synchronisation for these and a queued loop ----
+    k_unscale<<<gv, kBlock, 0, ctx->stream>>>(n, x_dev, scal);
+    RSG_TRY(true_residual(ctx, A, b_dev, x_dev, partials, ticket + 4, scal + 8));
+    RSG_CHECK_CUDA(ctx, read_back());
     if (memory == RSG_MEM_HOST)
         RSG_CHECK_CUDA(ctx, cudaMemcpyAsync(x, x_dev, size_t(n) * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
     RSG_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    st_out.true_relres = ctx->pinned[2];
+    st_out.norm_a = an;
+    st_out.norm_b = ctx->pinned[0];
+    st_out.equation_scale = ctx->pinned[1];
+    st_out.true_relres = ctx->pinned[10];
+    if (cg) {
+        std::memcpy(&h, ctx->pinned + 64, sizeof(h));
+        solve_seconds = switched ? first_seconds + cg_seconds(ctx) : cg_seconds(ctx);
+        if (switched) st_out.fp64_iterations = h.it;
+        st_out.iterations = cg_used + h.it;
+        st_out.outer = cg_outer + h.n_updates;
+        st_out.error = h.error;
+        st_out.trend = h.trend;
+        st_out.converged = h.converged;
+        solve_status = h.ticket[7] ? RSG_ERR_TIMEOUT : rsg_status(h.status);
+        if (want_hist) {
+            const uint32_t logged = st_out.iterations;
+            std::vector<double> e(logged), t(logged);
+            cudaMemcpy(e.data(), hist, logged * sizeof(double), cudaMemcpyDeviceToHost);
+            cudaMemcpy(t.data(), thist, logged * sizeof(double), cudaMemcpyDeviceToHost);
+            write_log(c, "Conjugate Gradient", logged, e.data(), t.data(), h.converged != 0);
+        }
+    }
     st_out.seconds_solve = solve_seconds;
     st_out.seconds_setup =
         std::chrono::duration<double>(std::chrono::steady_clock::now() - t_start).count() - solve_seconds;
