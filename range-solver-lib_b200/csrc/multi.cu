@@ -69,7 +69,10 @@ __device__ __forceinline__ double2 ld2(const double *__restrict__ base, size_t i
 }
 
 // acc = sum over the row's entries (CSR order) of a_rc * g(c); g returns this
-// lane's column pair of the gathered row c.  All 32 lanes must call it.
+// lane's column pair of the gathered row c.  All 32 lanes must call it.  A trip's gathers are
+// issued together (an entry past the row's end gathers row 0 and is not added) and the next trip's
+// entries are loaded behind them; one entry at a time behind a branch, 60^3 with k = 8 took 38.1 ms a solve
+// instead of 33.9.
 template <int K, class G>
 __device__ __forceinline__ double2 row_product(const MView &M, uint32_t row, bool valid, G &g)
 {
@@ -81,11 +84,11 @@ __device__ __forceinline__ double2 row_product(const MView &M, uint32_t row, boo
         je = __ldg(&M.rp[row + 1]);
     }
     const uint32_t trips = __reduce_max_sync(0xffffffffu, (je - jb + LPR - 1) / LPR);
-    double2 acc = make_double2(0.0, 0.0);
-    for (uint32_t t = 0; t < trips; t++) {
+    uint32_t c_mine = 0;
+    double v_mine = 0.0;
+    auto load = [&](uint32_t t) {  // the lane's entry of trip t
         const uint32_t e = jb + t * LPR + uint32_t(li);
-        uint32_t c_mine = 0;
-        double v_mine = 0.0;
+        c_mine = 0;
         if (e < je) {
             if (M.use_sell) {
                 const uint32_t k = e - jb, row0 = row & ~31u;
@@ -98,16 +101,24 @@ __device__ __forceinline__ double2 row_product(const MView &M, uint32_t row, boo
                 v_mine = __ldg(&M.val[e]);
             }
         }
+    };
+    if (trips) load(0);
+    double2 acc = make_double2(0.0, 0.0);
+    for (uint32_t t = 0; t < trips; t++) {
+        double2 x[LPR];
+        double v[LPR];
 #pragma unroll
-        for (int u = 0; u < LPR; u++) {
-            const uint32_t c = __shfl_sync(0xffffffffu, c_mine, g0 + u);
-            const double v = __shfl_sync(0xffffffffu, v_mine, g0 + u);
-            if (jb + t * LPR + uint32_t(u) < je) {
-                const double2 x = g(c);
-                acc.x = __dadd_rn(acc.x, __dmul_rn(v, x.x));
-                acc.y = __dadd_rn(acc.y, __dmul_rn(v, x.y));
-            }
+        for (int u = 0; u < LPR; u++) {  // all gathers of the trip, then the next trip's entries, then the sums
+            v[u] = __shfl_sync(0xffffffffu, v_mine, g0 + u);
+            x[u] = g(__shfl_sync(0xffffffffu, c_mine, g0 + u));
         }
+        if (t + 1 < trips) load(t + 1);
+#pragma unroll
+        for (int u = 0; u < LPR; u++)
+            if (jb + t * LPR + uint32_t(u) < je) {
+                acc.x = __dadd_rn(acc.x, __dmul_rn(v[u], x[u].x));
+                acc.y = __dadd_rn(acc.y, __dmul_rn(v[u], x[u].y));
+            }
     }
     return acc;
 }
@@ -218,11 +229,11 @@ __device__ __forceinline__ void each_column(MrState *st, F f)
         const uint32_t row = grp_ * Map<K>::RPW + uint32_t(lane_ / Map<K>::LPR);                               \
         const bool valid = row < (n);
 
-// r = b - A x, z = D r; per column ||b||^2, ||r||^2, r^T z
+// r = b - A x (z = D r); per column ||b||^2, ||r||^2, r^T z
 template <int K>
 __global__ void __launch_bounds__(kBlock) k_mr_init(MView M, const double *__restrict__ d, const double *__restrict__ b,
                                                     const double *__restrict__ x, double *__restrict__ r,
-                                                    double *__restrict__ z, double *partials, MrState *st)
+                                                    double *partials, MrState *st)
 {
     __shared__ double sh[8 * 3 * K];
     __shared__ double tot[3 * K];
@@ -238,7 +249,6 @@ __global__ void __launch_bounds__(kBlock) k_mr_init(MView M, const double *__res
             const double2 rv = make_double2(bv.x - ax.x, bv.y - ax.y);
             const double2 zv = make_double2(di * rv.x, di * rv.y);
             reinterpret_cast<double2 *>(r)[idx] = rv;
-            reinterpret_cast<double2 *>(z)[idx] = zv;
             acc[0].x += bv.x * bv.x;
             acc[0].y += bv.y * bv.y;
             acc[1].x += rv.x * rv.x;
@@ -271,31 +281,50 @@ __global__ void __launch_bounds__(kBlock) k_mr_init(MView M, const double *__res
         });
 }
 
-// p = z + beta p_old (own row, and gathered on the fly), q = A p; per column p^T q -> alpha
+// p = z + beta p with z = D r, in place; a finished column's p stays.  Streaming, as k_mr_update.  A pass of its own:
+// formed where k_mr_dir gathers it, p cost that kernel two gathers per entry, which bound it (the load/store
+// pipe's passes), a second p and a stored z.  60^3, k = 8: 33.9 -> 29.4 ms; 45^3, k = 16: 20.3 (22.1) -> 18.0;
+// 30^3, k = 8, where the launch weighs most: 6.4-6.7 before, 6.5.
 template <int K>
-__global__ void __launch_bounds__(kBlock) k_mr_dir(MView M, const double *__restrict__ z,
-                                                   const double *__restrict__ po, double *__restrict__ pn,
-                                                   double *__restrict__ q, double *partials, MrState *st)
+__global__ void __launch_bounds__(kBlock) k_mr_p(uint32_t n, const double *__restrict__ d, const double *__restrict__ r,
+                                                 double *__restrict__ p, const MrState *st)
+{
+    pdl_wait();
+    pdl_release();
+    if (st->all_done) return;
+    const int li = (threadIdx.x & 31) % Map<K>::LPR;
+    const int j0 = 2 * li, j1 = 2 * li + 1;
+    const bool a0 = j0 < int(st->k) && !st->col[j0].done, a1 = j1 < int(st->k) && !st->col[j1].done;
+    const double bx = a0 ? st->col[j0].beta : 0.0, by = a1 ? st->col[j1].beta : 0.0;
+    const size_t total = size_t(n) * (K / 2);
+    for (size_t e = blockIdx.x * size_t(blockDim.x) + threadIdx.x; e < total; e += size_t(gridDim.x) * blockDim.x) {
+        const double2 rv = ld2(r, e);
+        double2 pv = reinterpret_cast<const double2 *>(p)[e];
+        const double di = d ? d[e / (K / 2)] : 1.0;
+        if (a0) pv.x = fma(bx, pv.x, di * rv.x);
+        if (a1) pv.y = fma(by, pv.y, di * rv.y);
+        reinterpret_cast<double2 *>(p)[e] = pv;
+    }
+}
+
+// q = A p; per column p^T q -> alpha
+template <int K>
+__global__ void __launch_bounds__(kBlock) k_mr_dir(MView M, const double *__restrict__ p, double *__restrict__ q,
+                                                   double *partials, MrState *st)
 {
     __shared__ double sh[8 * K];
     __shared__ double tot[K];
+    pdl_wait();
+    pdl_release();
     if (st->all_done) return;
     const int li = (threadIdx.x & 31) % Map<K>::LPR;
-    const double bx = 2 * li < int(st->k) ? st->col[2 * li].beta : 0.0;
-    const double by = 2 * li + 1 < int(st->k) ? st->col[2 * li + 1].beta : 0.0;
-    auto gp = [&](uint32_t c) {
-        const size_t idx = size_t(c) * (K / 2) + li;
-        const double2 zv = ld2(z, idx), pv = ld2(po, idx);
-        return make_double2(fma(bx, pv.x, zv.x), fma(by, pv.y, zv.y));
-    };
+    auto gp = [&](uint32_t c) { return ld2(p, size_t(c) * (K / 2) + li); };
     double2 acc[1] = {make_double2(0, 0)};
     MR_FOR_ROWS(K, M.n, row, valid)
         const double2 qv = row_product<K>(M, row, valid, gp);
         if (valid) {
-            const size_t idx = size_t(row) * (K / 2) + li;
             const double2 pv = gp(row);
-            reinterpret_cast<double2 *>(pn)[idx] = pv;
-            reinterpret_cast<double2 *>(q)[idx] = qv;
+            reinterpret_cast<double2 *>(q)[size_t(row) * (K / 2) + li] = qv;
             acc[0].x += pv.x * qv.x;
             acc[0].y += pv.y * qv.y;
         }
@@ -317,16 +346,18 @@ __global__ void __launch_bounds__(kBlock) k_mr_dir(MView M, const double *__rest
         });
 }
 
-// x += alpha p, r -= alpha q, z = D r for the active columns; r^T z, ||r||^2 -> beta, stop tests.
+// x += alpha p, r -= alpha q for the active columns; r^T z (z = D r), ||r||^2 -> beta, stop tests.
 // Streaming: one thread per 16-byte column pair of a row.
 template <int K>
 __global__ void __launch_bounds__(kBlock) k_mr_update(uint32_t n, const double *__restrict__ d,
                                                       const double *__restrict__ p, const double *__restrict__ q,
                                                       double *__restrict__ x, double *__restrict__ r,
-                                                      double *__restrict__ z, double *partials, MrState *st)
+                                                      double *partials, MrState *st)
 {
     __shared__ double sh[8 * 2 * K];
     __shared__ double tot[2 * K];
+    pdl_wait();
+    pdl_release();
     const int li = (threadIdx.x & 31) % Map<K>::LPR;
     const int j0 = 2 * li, j1 = 2 * li + 1;
     const bool a0 = j0 < int(st->k) && !st->col[j0].done, a1 = j1 < int(st->k) && !st->col[j1].done;
@@ -337,23 +368,19 @@ __global__ void __launch_bounds__(kBlock) k_mr_update(uint32_t n, const double *
         const double2 pv = ld2(p, e), qv = ld2(q, e);
         double2 xv = reinterpret_cast<const double2 *>(x)[e];
         double2 rv = reinterpret_cast<const double2 *>(r)[e];
-        double2 zv = reinterpret_cast<const double2 *>(z)[e];
         const double di = d ? d[e / (K / 2)] : 1.0;
         if (a0) {
             xv.x = fma(al0, pv.x, xv.x);
             rv.x = fma(-al0, qv.x, rv.x);
-            zv.x = di * rv.x;
         }
         if (a1) {
             xv.y = fma(al1, pv.y, xv.y);
             rv.y = fma(-al1, qv.y, rv.y);
-            zv.y = di * rv.y;
         }
         reinterpret_cast<double2 *>(x)[e] = xv;
         reinterpret_cast<double2 *>(r)[e] = rv;
-        reinterpret_cast<double2 *>(z)[e] = zv;
-        acc[0].x += rv.x * zv.x;
-        acc[0].y += rv.y * zv.y;
+        acc[0].x += rv.x * (di * rv.x);
+        acc[0].y += rv.y * (di * rv.y);
         acc[1].x += rv.x * rv.x;
         acc[1].y += rv.y * rv.y;
     }
@@ -380,11 +407,12 @@ __global__ void __launch_bounds__(kBlock) k_mr_update(uint32_t n, const double *
 template <int K>
 __global__ void __launch_bounds__(kBlock) k_mr_check(MView M, const double *__restrict__ d,
                                                      const double *__restrict__ b, const double *__restrict__ x,
-                                                     double *__restrict__ r, double *__restrict__ z, double *partials,
-                                                     MrState *st)
+                                                     double *__restrict__ r, double *partials, MrState *st)
 {
     __shared__ double sh[8 * 2 * K];
     __shared__ double tot[2 * K];
+    pdl_wait();
+    pdl_release();
     if (!st->any_check) return;
     const int li = (threadIdx.x & 31) % Map<K>::LPR;
     const bool c0 = 2 * li < int(st->k) && st->col[2 * li].need_check;
@@ -397,20 +425,12 @@ __global__ void __launch_bounds__(kBlock) k_mr_check(MView M, const double *__re
             const size_t idx = size_t(row) * (K / 2) + li;
             const double2 bv = ld2(b, idx);
             double2 rv = reinterpret_cast<const double2 *>(r)[idx];
-            double2 zv = reinterpret_cast<const double2 *>(z)[idx];
             const double di = d ? d[row] : 1.0;
-            if (c0) {
-                rv.x = bv.x - ax.x;
-                zv.x = di * rv.x;
-            }
-            if (c1) {
-                rv.y = bv.y - ax.y;
-                zv.y = di * rv.y;
-            }
+            if (c0) rv.x = bv.x - ax.x;
+            if (c1) rv.y = bv.y - ax.y;
             reinterpret_cast<double2 *>(r)[idx] = rv;
-            reinterpret_cast<double2 *>(z)[idx] = zv;
-            acc[0].x += rv.x * zv.x;
-            acc[0].y += rv.y * zv.y;
+            acc[0].x += rv.x * (di * rv.x);
+            acc[0].y += rv.y * (di * rv.y);
             acc[1].x += rv.x * rv.x;
             acc[1].y += rv.y * rv.y;
         }
@@ -468,6 +488,7 @@ __global__ void __launch_bounds__(kBlock) k_mr_true(MView M, const double *__res
 
 __global__ void k_mr_tail(MrState *st, cudaGraphConditionalHandle h, int use_cond)
 {
+    pdl_wait();
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     const uint32_t bc = ++st->body_count;
     if (!st->all_done && bc >= st->body_limit) {
@@ -480,7 +501,7 @@ __global__ void k_mr_tail(MrState *st, cudaGraphConditionalHandle h, int use_con
 struct MrArgs {
     MView M;
     const double *d, *b;
-    double *x, *r, *z, *p[2], *q, *partials;
+    double *x, *r, *p, *q, *partials;
     MrState *st;
     int g;
 };
@@ -488,14 +509,15 @@ struct MrArgs {
 template <int K>
 void mr_body(rsg_context *ctx, const MrArgs &a, cudaGraphConditionalHandle h, int use_cond)
 {
+    cudaStream_t sm = ctx->stream;
     for (int half = 0; half < 2; half++) {
-        const double *po = a.p[half];
-        double *pn = a.p[half ^ 1];
-        k_mr_dir<K><<<a.g, kBlock, 0, ctx->stream>>>(a.M, a.z, po, pn, a.q, a.partials, a.st);
-        k_mr_update<K><<<a.g, kBlock, 0, ctx->stream>>>(a.M.n, a.d, pn, a.q, a.x, a.r, a.z, a.partials, a.st);
-        k_mr_check<K><<<a.g, kBlock, 0, ctx->stream>>>(a.M, a.d, a.b, a.x, a.r, a.z, a.partials, a.st);
+        launch_k(sm, true, k_mr_p<K>, a.g, kBlock, 0, a.M.n, a.d, (const double *)a.r, a.p, (const MrState *)a.st);
+        launch_k(sm, true, k_mr_dir<K>, a.g, kBlock, 0, a.M, (const double *)a.p, a.q, a.partials, a.st);
+        launch_k(sm, true, k_mr_update<K>, a.g, kBlock, 0, a.M.n, a.d, (const double *)a.p, (const double *)a.q, a.x,
+                 a.r, a.partials, a.st);
+        launch_k(sm, true, k_mr_check<K>, a.g, kBlock, 0, a.M, a.d, a.b, (const double *)a.x, a.r, a.partials, a.st);
     }
-    k_mr_tail<<<1, 32, 0, ctx->stream>>>(a.st, h, use_cond);
+    launch_k(sm, true, k_mr_tail, 1, 32, 0, a.st, h, use_cond);
 }
 
 template <int K>
@@ -507,7 +529,7 @@ rsg_status mr_run(rsg_context *ctx, MrArgs &a, bool use_graph, double *seconds)
     if (K >= 8) a.M.use_sell = 0;
     a.g = g;
     cudaEventRecord(ctx->ev[0], ctx->stream);
-    k_mr_init<K><<<g, kBlock, 0, ctx->stream>>>(a.M, a.d, a.b, a.x, a.r, a.z, a.partials, a.st);
+    k_mr_init<K><<<g, kBlock, 0, ctx->stream>>>(a.M, a.d, a.b, a.x, a.r, a.partials, a.st);
     RSG_CHECK_CUDA(ctx, cudaGetLastError());
     rsg_status s = RSG_OK;
     if (use_graph) {
@@ -593,7 +615,7 @@ extern "C" rsg_status rsg_solve_multi(rsg_context *ctx, rsg_csr *A, const rsg_so
     const uint32_t n = A->n;
     const uint32_t K = k <= 2 ? 2 : k <= 4 ? 4 : k <= 8 ? 8 : 16;
     const size_t vk = arena_bytes(size_t(n) * K, sizeof(double));
-    size_t bytes = 7 * vk + arena_bytes(n, sizeof(double)) + arena_bytes(size_t(kMaxGrid) * 3 * K, sizeof(double)) +
+    size_t bytes = 5 * vk + arena_bytes(n, sizeof(double)) + arena_bytes(size_t(kMaxGrid) * 3 * K, sizeof(double)) +
                    arena_bytes(1, sizeof(MrState)) + 4096;
     if (memory == RSG_MEM_HOST) bytes += 2 * arena_bytes(size_t(n) * k, sizeof(double));
     RSG_TRY(arena_reserve(ctx, bytes));
@@ -601,9 +623,7 @@ extern "C" rsg_status rsg_solve_multi(rsg_context *ctx, rsg_csr *A, const rsg_so
     double *bi = arena_take<double>(ctx, size_t(n) * K);
     a.x = arena_take<double>(ctx, size_t(n) * K);
     a.r = arena_take<double>(ctx, size_t(n) * K);
-    a.z = arena_take<double>(ctx, size_t(n) * K);
-    a.p[0] = arena_take<double>(ctx, size_t(n) * K);
-    a.p[1] = arena_take<double>(ctx, size_t(n) * K);
+    a.p = arena_take<double>(ctx, size_t(n) * K);
     a.q = arena_take<double>(ctx, size_t(n) * K);
     double *d = arena_take<double>(ctx, n);
     a.partials = arena_take<double>(ctx, size_t(kMaxGrid) * 3 * K);
@@ -625,7 +645,7 @@ extern "C" rsg_status rsg_solve_multi(rsg_context *ctx, rsg_csr *A, const rsg_so
     const int gp = std::min(grid_for(ctx, (const void *)k_mr_pack, kBlock, 0, (long long)n * K), kMaxGrid);
     k_mr_pack<<<gp, kBlock, 0, ctx->stream>>>(n, k, K, Bsrc, n, bi);
     k_mr_pack<<<gp, kBlock, 0, ctx->stream>>>(n, k, K, Xsrc, n, a.x);
-    RSG_CHECK_CUDA(ctx, cudaMemsetAsync(a.p[0], 0, size_t(n) * K * 8, ctx->stream));
+    RSG_CHECK_CUDA(ctx, cudaMemsetAsync(a.p, 0, size_t(n) * K * 8, ctx->stream));
     RSG_CHECK_CUDA(ctx, cudaMemsetAsync(a.partials, 0, 8, ctx->stream));
     MrState h;
     std::memset(&h, 0, sizeof(h));
