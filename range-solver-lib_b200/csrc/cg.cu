@@ -154,14 +154,12 @@ __global__ void __launch_bounds__(kBlock) k_cg_prec(uint32_t n, uint32_t w, cons
     }
 }
 
-template <int RPW>
-__global__ void __launch_bounds__(kBlock) k_cg_dir(Csr<double> M, Sell<double> S, int use_sell, const double *__restrict__ z,
-                                                   double *p0, double *p1, double *__restrict__ q, double *partials,
-                                                   CgState *st)
+// p = z + beta p_old, formed where it is gathered and stored for the own rows, q = A p, p^T q -> alpha; rows(gx, epi)
+// runs over the matrix.
+template <class ROWS>
+__device__ __forceinline__ void cg_dir(const double *__restrict__ z, double *p0, double *p1, double *__restrict__ q,
+                                       double *partials, CgState *st, ROWS rows)
 {
-    pdl_wait();
-    pdl_release();
-    extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ double sh[32];
     if (st->done || st->need_check) return;
     const double *__restrict__ p_old = st->pcur ? p1 : p0;
@@ -175,7 +173,7 @@ __global__ void __launch_bounds__(kBlock) k_cg_dir(Csr<double> M, Sell<double> S
         q[row] = v;
         acc[0] += p * v;
     };
-    for_rows_any<double, RPW>(M, S, use_sell != 0, gx, epi, smem_raw, &st->ticket[7], true);
+    rows(gx, epi);
     state_step<1>(st, acc, partials, 0, sh, [](CgState *s, const double *tot) {
         const double pq = clamp_pq(tot[0], s->eps);
         s->pq = pq;
@@ -183,6 +181,64 @@ __global__ void __launch_bounds__(kBlock) k_cg_dir(Csr<double> M, Sell<double> S
         s->alpha = s->rho / pq;
         s->pcur ^= 1u;
     });
+}
+
+// The CSR stream (matrices without a SELL-32 copy).
+template <int RPW>
+__global__ void __launch_bounds__(kBlock) k_cg_dir(Csr<double> M, const double *__restrict__ z, double *p0, double *p1,
+                                                   double *__restrict__ q, double *partials, CgState *st)
+{
+    pdl_wait();
+    pdl_release();
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    cg_dir(z, p0, p1, q, partials, st, [&](auto &gx, auto &epi) {
+        for_rows_tma<double, RPW>(M, gx, epi, smem_raw, &st->ticket[7], true);
+    });
+}
+
+// SELL-32, bound by the matrix's bytes from memory or, where it stays there, from L2.  One 32-byte load per lane and
+// four entries (two of 16 bytes touch every line twice).  BLOCKS per SM: with five (48 registers) more loads are in
+// flight per warp, six hold 7104 slices at once instead of 5920.
+template <int CACHE, int BLOCKS>
+__global__ void __launch_bounds__(kBlock, BLOCKS) k_cg_dir_sell(Sell<double> S, const double *__restrict__ z, double *p0,
+                                                                double *p1, double *__restrict__ q, double *partials,
+                                                                CgState *st)
+{
+    pdl_wait();
+    pdl_release();
+    cg_dir(z, p0, p1, q, partials, st, [&](auto &gx, auto &epi) {
+        for_rows_sell_v<double, CACHE>(S, gx, epi, blockIdx.x, gridDim.x);
+    });
+}
+
+using DirSell = void (*)(Sell<double>, const double *, double *, double *, double *, double *, CgState *);
+
+// Which of them for A, and its grid.  Caches: what an iteration reads again has to share L2 with the matrix -- the
+// six vectors, then the offsets, then the values, as far as they fit kL2Keep, half of the 126 MB (either die's half
+// also holds lines of the other's memory).  FP64 solves, everything out of L2 first / offsets kept / all kept, ms:
+// 60^3 (53 MB in all) 9.7 / - / 9.0; the beam of 64 x 32 x 32 (28 MB with the offsets, 120 in all) 39.0 / 36.6 with
+// 16-byte loads / 40.7; 80^3 (42 MB) 21.2 / 20.1 with 16-byte loads / 21.8; 100^3 (80 MB) 39.0 / 46.4 / 46.9.
+// Blocks: six where they save a third of the rounds over the slices (60^3: one instead of two, 9.7 against 10.6; the
+// beam 39.0 against 45.3), else five (80^3 21.2 -> 19.3, 100^3 39.0 -> 38.3).  Streaming 16-byte loads before: 9.8,
+// 40.3, 22.4 and 41.8.
+constexpr size_t kL2Keep = size_t(60) << 20;
+template <int CACHE>
+DirSell pick_blocks(rsg_context *ctx, const rsg_csr *A, int *grid)
+{
+    constexpr uint32_t wpb = kBlock / 32;
+    const int g5 = grid_for(ctx, (const void *)k_cg_dir_sell<CACHE, 5>, kBlock, 0, (long long)A->n_slices * 32);
+    const int g6 = grid_for(ctx, (const void *)k_cg_dir_sell<CACHE, 6>, kBlock, 0, (long long)A->n_slices * 32);
+    const uint32_t r5 = (A->n_slices + g5 * wpb - 1) / (g5 * wpb), r6 = (A->n_slices + g6 * wpb - 1) / (g6 * wpb);
+    const DirSell k = 3 * r6 <= 2 * r5 ? k_cg_dir_sell<CACHE, 6> : k_cg_dir_sell<CACHE, 5>;
+    *grid = spmv_grid(ctx, A, (const void *)k, 0, 32);
+    return k;
+}
+DirSell pick_dir_sell(rsg_context *ctx, const rsg_csr *A, int *grid)
+{
+    const size_t vec = size_t(6) * A->n * sizeof(double), off = A->sell_len * (A->soff ? 2 : 4);
+    if (vec + off + A->sell_len * sizeof(double) <= kL2Keep) return pick_blocks<kSellKeep>(ctx, A, grid);
+    if (vec + off <= kL2Keep) return pick_blocks<kSellKeepOffsets>(ctx, A, grid);
+    return pick_blocks<kSellOut>(ctx, A, grid);
 }
 
 template <int PK>
@@ -579,6 +635,7 @@ struct Launch {
     int g_spmv64, g_spmv32, g_vec;
     int g_dir64, g_dir32, g_upd64, g_upd32;  // the loop's kernels: autotuned shapes or the defaults
     size_t s64, s32;
+    DirSell dir_sell = nullptr;              // the FP64 direction kernel of a SELL-32 matrix
 };
 
 template <int RPW, int PK>
@@ -626,8 +683,10 @@ void launch_body(rsg_context *ctx, const CgArgs &a, const Launch &L, cudaGraphCo
     const Csr<float> M32 = view<float>(a.A, true);
     for (int it = 0; it < iterations; it++) {
         if (!a.mixed) {
-            launch_k(st, pdl, k_cg_dir<RPW>, L.g_dir64, kBlock, L.s64, M64, S64, us, a.z, a.p0, a.p1, a.q, a.partials,
-                     a.st);
+            if (us)
+                launch_k(st, pdl, L.dir_sell, L.g_dir64, kBlock, 0, S64, a.z, a.p0, a.p1, a.q, a.partials, a.st);
+            else
+                launch_k(st, pdl, k_cg_dir<RPW>, L.g_dir64, kBlock, L.s64, M64, a.z, a.p0, a.p1, a.q, a.partials, a.st);
             launch_k(st, pdl, k_cg_update<PK>, L.g_upd64, kBlock, 0, n, a.P.w, a.P.d, a.p0, a.p1, a.q, a.x, a.r, a.z,
                      a.partials, a.st);
         } else {
@@ -715,7 +774,11 @@ rsg_status run_typed(rsg_context *ctx, const CgArgs &a)
     }
     const long long chunk_threads = (long long)a.A->n * 32 / RPW;
     (void)chunk_threads;
-    L.g_spmv64 = spmv_grid(ctx, a.A, (const void *)k_cg_dir<RPW>, L.s64, RPW);
+    // (the residual's and the checks' grid)
+    L.g_spmv64 = spmv_grid(ctx, a.A, a.A->use_sell ? (const void *)k_cg_init_res<RPW> : (const void *)k_cg_dir<RPW>,
+                           L.s64, RPW);
+    int g_dir64 = L.g_spmv64;
+    if (a.A->use_sell) L.dir_sell = pick_dir_sell(ctx, a.A, &g_dir64);
     L.g_spmv32 = spmv_grid(ctx, a.A, (const void *)k_mx_dir<RPW>, L.s32, RPW);
     // the update's grid: a block for every 256 pairs (FP64) or quadruples (FP32) of rows, at most three an SM --
     // every block adds a ticket and partials (220k rows, us per iteration: FP64 20.6 with 8 blocks an SM, 20.2
@@ -723,7 +786,7 @@ rsg_status run_typed(rsg_context *ctx, const CgArgs &a)
     L.g_vec = std::min(grid_for(ctx, (const void *)k_cg_update<PK>, kBlock, 0, a.A->n / (a.mixed ? 4 : 2)),
                        kUpdateBlocksPerSm * ctx->num_sms);
     const rsg_csr::Tune &T = a.A->tune;
-    L.g_dir64 = T.valid && T.g_dir64 > 0 ? T.g_dir64 : L.g_spmv64;
+    L.g_dir64 = T.valid && T.g_dir64 > 0 ? T.g_dir64 : g_dir64;
     L.g_dir32 = T.valid && T.g_dir32 > 0 ? T.g_dir32 : L.g_spmv32;
     L.g_upd64 = T.valid && T.g_upd64 > 0 ? T.g_upd64 : L.g_vec;
     L.g_upd32 = T.valid && T.g_upd32 > 0 ? T.g_upd32 : L.g_vec;
@@ -849,7 +912,10 @@ rsg_status profile_typed(rsg_context *ctx, const rsg_csr *A, int kernel, uint32_
     (void)ct;
     // the solve loop's launch shapes: autotuned when A carries them, else the built-in defaults
     const rsg_csr::Tune &T = A->tune;
-    const int g64 = T.valid && T.g_dir64 > 0 ? T.g_dir64 : spmv_grid(ctx, A, (const void *)k_cg_dir<RPW>, s64, RPW);
+    int g64 = 0;
+    const DirSell dir_sell = A->use_sell ? pick_dir_sell(ctx, A, &g64) : nullptr;
+    if (!dir_sell) g64 = spmv_grid(ctx, A, (const void *)k_cg_dir<RPW>, s64, RPW);
+    if (T.valid && T.g_dir64 > 0) g64 = T.g_dir64;
     const int g32 = T.valid && T.g_dir32 > 0 ? T.g_dir32 : spmv_grid(ctx, A, (const void *)k_mx_dir<RPW>, s32, RPW);
     const int gv = std::min(grid_for(ctx, (const void *)k_cg_update<1>, kBlock, 0, n), kMaxGrid);
     const int gv64 = T.valid && T.g_upd64 > 0 ? T.g_upd64 : gv;
@@ -859,8 +925,10 @@ rsg_status profile_typed(rsg_context *ctx, const rsg_csr *A, int kernel, uint32_
     auto launch = [&]() {
         switch (kernel) {
         case RSG_KERNEL_CG_DIR_FP64:
-            k_cg_dir<RPW><<<g64, kBlock, s64, ctx->stream>>>(M64, S64, us, v64[0], v64[1], v64[2], v64[3], partials,
-                                                             st);
+            if (dir_sell)
+                dir_sell<<<g64, kBlock, 0, ctx->stream>>>(S64, v64[0], v64[1], v64[2], v64[3], partials, st);
+            else
+                k_cg_dir<RPW><<<g64, kBlock, s64, ctx->stream>>>(M64, v64[0], v64[1], v64[2], v64[3], partials, st);
             break;
         case RSG_KERNEL_CG_DIR_MIXED:
             k_mx_dir<RPW><<<g32, kBlock, s32, ctx->stream>>>(M32, S32, us, v32[0], v32[1], v32[2], v32[3], v64[0],

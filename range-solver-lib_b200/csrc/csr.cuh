@@ -34,11 +34,18 @@ constexpr int kMaxGrid = 16384;     // upper bound on grid size of reduction ker
 // 32-row slices / chunks).  A sweep over the 1M-row heat matrix on B200 measured
 // this at 71% of HBM bandwidth for the FP64 SpMV, ahead of one-slice-per-warp
 // grids (whose many block-level reductions stall on barriers), two slices per
-// warp, and register-capped variants.
+// warp, and register-capped variants.  With SELL-32 every warp gets the same number of
+// slices or one less: 80^3 (16.2k slices, 7104 resident warps) has 2.3 slices a warp, and
+// the third round of a full grid ran on 28% of them (FP64 solve 22.4 -> 21.8 ms, mixed
+// 17.5 -> 17.1; 100^3 mixed 30.4 -> 29.9).
 inline int spmv_grid(rsg_context *ctx, const rsg_csr *A, const void *kernel, size_t smem, int rpw)
 {
     const long long threads = A->use_sell ? (long long)A->n_slices * 32 : (long long)A->n * 32 / rpw;
-    return std::min(grid_for(ctx, kernel, kBlock, smem, threads), kMaxGrid);
+    const int full = std::min(grid_for(ctx, kernel, kBlock, smem, threads), kMaxGrid);
+    if (!A->use_sell) return full;
+    constexpr uint32_t wpb = kBlock / 32;
+    const uint32_t rounds = (A->n_slices + uint32_t(full) * wpb - 1) / (uint32_t(full) * wpb);
+    return std::max(1, int((A->n_slices + rounds * wpb - 1) / (rounds * wpb)));
 }
 
 rsg_status spmv64(rsg_context *ctx, const rsg_csr *A, const double *x, double *y, bool off16);

@@ -395,8 +395,22 @@ struct Sell {
 __device__ __forceinline__ double row_acc(double acc, double v, double x) { return __dadd_rn(acc, __dmul_rn(v, x)); }
 __device__ __forceinline__ float row_acc(float acc, float v, float x) { return fmaf(v, x, acc); }
 
+// How a pass over a SELL-32 matrix uses the caches: as streaming loads; or, for the FP64 direction kernel
+// (cg.cu), with 32-byte loads: values and offsets past L1 and first out of L2, only the offsets kept in L2, or both.
+enum { kSellStream = 0, kSellOut, kSellKeepOffsets, kSellKeep };
+
+template <int CACHE = kSellStream>
 __device__ __forceinline__ void ld4(const double *p, double (&v)[4])
 {
+    if constexpr (CACHE == kSellKeep) {
+        asm("ld.global.nc.v4.f64 {%0,%1,%2,%3}, [%4];" : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3]) : "l"(p));
+        return;
+    } else if constexpr (CACHE != kSellStream) {
+        asm("ld.global.nc.L1::no_allocate.L2::evict_first.v4.f64 {%0,%1,%2,%3}, [%4];"
+            : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3])
+            : "l"(p));
+        return;
+    }
     const double2 a = __ldcs(reinterpret_cast<const double2 *>(p));
     const double2 b = __ldcs(reinterpret_cast<const double2 *>(p) + 1);
     v[0] = a.x;
@@ -404,6 +418,7 @@ __device__ __forceinline__ void ld4(const double *p, double (&v)[4])
     v[2] = b.x;
     v[3] = b.y;
 }
+template <int CACHE = kSellStream>
 __device__ __forceinline__ void ld4(const float *p, float (&v)[4])
 {
     const float4 a = __ldcs(reinterpret_cast<const float4 *>(p));
@@ -415,7 +430,7 @@ __device__ __forceinline__ void ld4(const float *p, float (&v)[4])
 
 // The rows of virtual block vb of a grid of vgrid blocks (a persistent kernel runs several virtual
 // blocks per CTA with the same row assignment, and so the same sums, as a grid of vgrid blocks).
-template <typename V, class GX, class EPI>
+template <typename V, int CACHE = kSellStream, class GX, class EPI>
 __device__ __forceinline__ void for_rows_sell_v(const Sell<V> &M, GX &gx, EPI &epi, uint32_t vb, uint32_t vgrid)
 {
     const int lane = threadIdx.x & 31;
@@ -431,16 +446,18 @@ __device__ __forceinline__ void for_rows_sell_v(const Sell<V> &M, GX &gx, EPI &e
         for (uint32_t g = 0; g < g4; g++) {
             const size_t e = base + size_t(g) * 128u;
             V v[4];
-            ld4(M.val + e, v);
+            ld4<CACHE>(M.val + e, v);
             uint32_t c[4];
             if (M.off) {
-                const short4 o = __ldcs(reinterpret_cast<const short4 *>(M.off + e));
+                const short4 *po = reinterpret_cast<const short4 *>(M.off + e);
+                const short4 o = CACHE >= kSellKeepOffsets ? __ldg(po) : __ldcs(po);
                 c[0] = uint32_t(int(row0) + o.x);
                 c[1] = uint32_t(int(row0) + o.y);
                 c[2] = uint32_t(int(row0) + o.z);
                 c[3] = uint32_t(int(row0) + o.w);
             } else {
-                const uint4 o = __ldcs(reinterpret_cast<const uint4 *>(M.col + e));
+                const uint4 *po = reinterpret_cast<const uint4 *>(M.col + e);
+                const uint4 o = CACHE >= kSellKeepOffsets ? __ldg(po) : __ldcs(po);
                 c[0] = o.x;
                 c[1] = o.y;
                 c[2] = o.z;
