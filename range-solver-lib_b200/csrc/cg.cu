@@ -219,8 +219,8 @@ using DirSell = void (*)(Sell<double>, const double *, double *, double *, doubl
 // 60^3 (53 MB in all) 9.7 / - / 9.0; the beam of 64 x 32 x 32 (28 MB with the offsets, 120 in all) 39.0 / 36.6 with
 // 16-byte loads / 40.7; 80^3 (42 MB) 21.2 / 20.1 with 16-byte loads / 21.8; 100^3 (80 MB) 39.0 / 46.4 / 46.9.
 // Blocks: six where they save a third of the rounds over the slices (60^3: one instead of two, 9.7 against 10.6; the
-// beam 39.0 against 45.3), else five (80^3 21.2 -> 19.3, 100^3 39.0 -> 38.3).  Streaming 16-byte loads before: 9.8,
-// 40.3, 22.4 and 41.8.
+// beam 39.0 against 45.3), else five (80^3 21.2 -> 19.3, 100^3 39.0 -> 38.3).  Both rules: 60^3 9.2, the beam 36.0,
+// 80^3 18.4, 100^3 38.8-39.6; streaming 16-byte loads before them 9.8, 40.3, 22.4 and 41.8.
 constexpr size_t kL2Keep = size_t(60) << 20;
 template <int CACHE>
 DirSell pick_blocks(rsg_context *ctx, const rsg_csr *A, int *grid)
