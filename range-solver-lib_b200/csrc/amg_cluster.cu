@@ -132,8 +132,9 @@ __global__ void __launch_bounds__(256) k_cl_extent(ClSrcs s, uint32_t *ext)
     }
 }
 
-// Exclusive scan of one value per thread of a block of 512 (sc: 512 words).
-__device__ __forceinline__ uint32_t scan_tile(uint32_t v, uint32_t *sc)
+// Running exclusive scan over tiles of one value per thread of a block of 512 (sc: 512 words).  `carry`, the sum of
+// the tiles before this one, is each thread's own: nothing but sc is shared, and it may be written again on return.
+__device__ __forceinline__ uint32_t scan_tile(uint32_t v, uint32_t *sc, uint32_t &carry)
 {
     sc[threadIdx.x] = v;
     __syncthreads();
@@ -143,13 +144,16 @@ __device__ __forceinline__ uint32_t scan_tile(uint32_t v, uint32_t *sc)
         sc[threadIdx.x] += x;
         __syncthreads();
     }
-    return sc[threadIdx.x] - v;
+    const uint32_t at = carry + sc[threadIdx.x] - v;
+    carry += sc[511];
+    __syncthreads();
+    return at;
 }
 
 __global__ void __launch_bounds__(512) k_cl_pack(ClSrcs s, AmgClusterMap m, const uint32_t *ext, uint8_t *blob)
 {
     __shared__ ClHead h;
-    __shared__ uint32_t sc[512], carry;
+    __shared__ uint32_t sc[512];
     uint8_t *out = blob + size_t(blockIdx.x) * m.stride;
     if (threadIdx.x == 0) {
         cl_layout(m, blockIdx.x, ext, h);
@@ -178,20 +182,17 @@ __global__ void __launch_bounds__(512) k_cl_pack(ClSrcs s, AmgClusterMap m, cons
         for (uint32_t i = threadIdx.x; i < d.hi - d.lo; i += blockDim.x) place[i] = 0xffffu;
         __syncthreads();
         for (uint32_t k = threadIdx.x; k < d.nr; k += blockDim.x) place[L.rows[k0 + k] - d.lo] = uint16_t(k);
-        if (threadIdx.x == 0) carry = 0;
         __syncthreads();
+        uint32_t carry = 0;
         for (uint32_t t0 = 0; t0 < d.hi - d.lo; t0 += blockDim.x) {
             const uint32_t i = t0 + threadIdx.x;
             const uint16_t k = i < d.hi - d.lo ? place[i] : uint16_t(0xffffu);
             const uint32_t mine = k != 0xffffu;
-            const uint32_t at = carry + scan_tile(mine, sc);
+            const uint32_t at = scan_tile(mine, sc, carry);
             if (mine) perm[at] = k;
-            __syncthreads();
-            if (threadIdx.x == blockDim.x - 1) carry = at + mine;
-            __syncthreads();
         }
         // row pointers: a running scan over tiles of 512 rows
-        if (threadIdx.x == 0) carry = 0;
+        carry = 0;
         for (uint32_t t0 = 0; t0 < d.nr; t0 += blockDim.x) {
             const uint32_t k = t0 + threadIdx.x;
             uint32_t len = 0, r = 0;
@@ -201,7 +202,7 @@ __global__ void __launch_bounds__(512) k_cl_pack(ClSrcs s, AmgClusterMap m, cons
                 row[k] = uint16_t(r - d.lo);
                 dw[k] = L.dw[r];
             }
-            const uint32_t at = carry + scan_tile(len, sc);
+            const uint32_t at = scan_tile(len, sc, carry);
             if (k < d.nr) {
                 rptr[k] = uint16_t(at);
                 for (uint32_t i = 0; i < len; i++) {
@@ -209,12 +210,8 @@ __global__ void __launch_bounds__(512) k_cl_pack(ClSrcs s, AmgClusterMap m, cons
                     col[at + i] = uint16_t(L.ci[L.rp[r] + i] - d.lo);
                 }
             }
-            __syncthreads();
-            if (threadIdx.x == blockDim.x - 1) carry = at + len;
-            __syncthreads();
         }
         if (threadIdx.x == 0) rptr[d.nr] = uint16_t(carry);
-        __syncthreads();
         if (j + 1 == m.nl) {
             float *inv = reinterpret_cast<float *>(out + h.o_inv);
             for (uint32_t i = threadIdx.x; i < d.nI * L.nc; i += blockDim.x) inv[i] = s.inv[size_t(d.I0) * L.nc + i];
