@@ -18,10 +18,12 @@
 #include "csr.cuh"
 
 #include <algorithm>
+#include <atomic>
 #include <cstdlib>
 #include <cstring>
 
 struct rsg_assembly {
+    uint64_t id = 0;           // its own among all plans ever made; a matrix made from it carries it (rsg_csr::plan)
     uint32_t n_nodes = 0, n_tets = 0, n_tris = 0, dofs = 1, n_free = 0;
     uint64_t nnz = 0;
     double *xyz = nullptr;
@@ -752,7 +754,9 @@ rsg_status create_plan(rsg_context *ctx, uint32_t n_nodes, const double *xyz, ui
     std::string err;
     if (!build_assembly_plan(n_nodes, n_tets, tets, n_tris, tris, book, dofs, n_free, H, err))
         return set_error(ctx, RSG_ERR_INVALID_ARG, "assembly_create: %s", err.c_str());
+    static std::atomic<uint64_t> plans{0};
     auto *p = new rsg_assembly;
+    p->id = ++plans;
     p->n_nodes = n_nodes;
     p->n_tets = n_tets;
     p->n_tris = n_tris;
@@ -894,6 +898,7 @@ rsg_status assemble_into(rsg_context *ctx, rsg_assembly *p, rsg_csr **A, Launch 
     cudaError_t e = cudaGetLastError();
     rsg_status s = e == cudaSuccess ? RSG_OK : set_error(ctx, RSG_ERR_CUDA, "assemble: %s", cudaGetErrorString(e));
     if (s == RSG_OK) s = rsg_csr_create(ctx, p->n_free, p->rp, p->ci, tmp, RSG_MEM_DEVICE, A);
+    if (s == RSG_OK) (*A)->plan = p->id;
     cudaStreamSynchronize(ctx->stream);
     cudaFree(tmp);
     return s;
@@ -998,13 +1003,13 @@ rsg_status rsg_assemble_heat(rsg_context *ctx, rsg_assembly *p, const double *k_
     RSG_CHECK_CUDA(ctx, cudaFuncSetAttribute(local_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              int(heat_local_smem(kLocalRowMax))));
     const int grid = std::min(grid_for(ctx, (const void *)local_kernel, kBlock, smem, p->n_free), kMaxGrid);
-    if (!*A)
+    // The kernel lays the copies out by the plan's rows, so it writes them only into a matrix that was made from
+    // this plan; one of another pattern with the same counts (a renumbered mesh) has other slices.
+    if (!*A || (*A)->plan != p->id)
         return assemble_into(ctx, p, A, [&](double *val) {
             local_kernel<<<grid, kBlock, smem, ctx->stream>>>(p->n_free, rows, p->rp, h, HeatOut{val, b_device});
         });
     rsg_csr *M = *A;
-    if (M->n != p->n_free || M->nnz != p->nnz)
-        return set_error(ctx, RSG_ERR_INVALID_ARG, "assemble: matrix does not match the plan's pattern");
     RSG_TRY(arena_reserve(ctx, arena_bytes(32, sizeof(double)) + arena_bytes(size_t(grid), sizeof(double))));
     double *scal = arena_take<double>(ctx, 32);
     HeatOut o{M->val, b_device};

@@ -63,6 +63,7 @@ struct rsg_csr {
     uint32_t max_warp_nnz = 0;        // longest 32-row chunk
     uint32_t band = 0;                // largest |column - row|
     bool has_off16 = false;
+    uint64_t plan = 0;                // assembly plan that it was made from (rsg_assembly::id), 0: none
     // SELL-32 copy (slice = 32 rows = one warp; element k of lane l at
     // slice_ptr[s] + (k/4)*128 + 4l + k%4, rows padded to a multiple of 4)
     bool use_sell = false;
