@@ -732,7 +732,7 @@ rsg_status rsg_batch_solve(rsg_context *ctx, rsg_batch *B, const rsg_solver_conf
         h.stop_rule = RSG_STOP_TRUE_RELRES;
         std::vector<CgState> hs(ns, h);
         RSG_CHECK_CUDA(ctx, cudaMemcpyAsync(S, hs.data(), ns * sizeof(CgState), cudaMemcpyHostToDevice, sm));
-        BatchCtl c = {0, max_it + 16, 0, 1};  // a body makes at least one iteration of every active system
+        BatchCtl c = {0, body_limit_for(max_it), 0, 1};
         RSG_CHECK_CUDA(ctx, cudaMemsetAsync(T.ticket, 0, ns * sizeof(unsigned int), sm));
         RSG_CHECK_CUDA(ctx, cudaMemcpyAsync(ctl, &c, sizeof(c), cudaMemcpyHostToDevice, sm));
         // the lists start with every system

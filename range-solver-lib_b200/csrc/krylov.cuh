@@ -43,6 +43,10 @@ struct CgState {
 };
 constexpr uint32_t kStateWords = uint32_t(offsetof(CgState, ticket) / sizeof(uint32_t));
 
+// The loops' limit of bodies for max_it iterations (a body makes at least one); saturates, since a caller may mean
+// "no cap" by the largest max_it.
+inline uint32_t body_limit_for(uint32_t max_it) { return max_it > UINT32_MAX - 16 ? UINT32_MAX : max_it + 16; }
+
 struct AmgHierarchy;
 
 struct Precond {

@@ -219,7 +219,7 @@ extern "C" rsg_status rsg_solve(rsg_context *ctx, rsg_csr *A, const rsg_solver_c
     h.sigma = 1.0;
     h.max_it = max_it;
     h.stop_rule = c.stop_rule;
-    h.body_limit = max_it + 16;  // a body makes at least one iteration
+    h.body_limit = body_limit_for(max_it);
     h.history = hist;
     h.trend_hist = thist;
     h.evict_first32 = c.l2_resident_f32 ? 0 : 1;
@@ -310,7 +310,7 @@ extern "C" rsg_status rsg_solve(rsg_context *ctx, rsg_csr *A, const rsg_solver_c
             CgState h2 = h_init;
             h2.auto_switch = 0;
             h2.max_it = max_it > used ? max_it - used : 1;
-            h2.body_limit = h2.max_it + 16;
+            h2.body_limit = body_limit_for(h2.max_it);
             h2.history = hist ? hist + used : nullptr;
             h2.trend_hist = thist ? thist + used : nullptr;
             RSG_CHECK_CUDA(ctx, cudaMemsetAsync(a64.p0, 0, size_t(n) * sizeof(double), ctx->stream));
