@@ -12,7 +12,10 @@
 // holds P w as k_gm_correct leaves them, and inv[k + 1] = 1 / ||w|| multiplies
 // whatever is read from those slots, so an inner step is two launches and V is
 // never rewritten.  (The learned preconditioner needs v_k itself: there k_gm_vz
-// normalises the slot in place and inv stays 1.)
+// normalises the slot in place and inv stays 1.)  In FP32 without a preconditioner
+// a slot of Z is also scaled by a power of two, next to 1 / the norm of the slot
+// before: the product's row sums, taken before inv is applied, would be ~ ||A||^2,
+// past FP32's range from entries of 1e19 on and with lost bits below 1e-17.
 //   cycle end    back substitution (:554-567), x += sum_j z_j y_j (:570-578)
 // Z is stored, so a variable preconditioner (flexible GMRES) needs no change.
 // Each cycle is one captured CUDA graph; the host polls the device state once
@@ -143,7 +146,7 @@ __global__ void __launch_bounds__(kBlock) k_gm_vz(uint32_t n, size_t ld, uint32_
     if (st->done || st->inner_done) return;
     const double s = (k == 0) ? st->beta : wnorm[k];
     T *v = V + size_t(k) * ld, *z = Z + size_t(k) * ld;
-    if (blockIdx.x == 0 && threadIdx.x == 0) inv[k] = 1.0;
+    if (blockIdx.x == 0 && threadIdx.x == 0) inv[k] = inv[kVInv + k] = 1.0;
     const uint32_t G = PK == 2 ? w_ : 1, ng = n / G;
     for (uint32_t gi = blockIdx.x * blockDim.x + threadIdx.x; gi < ng; gi += gridDim.x * blockDim.x) {
         T vl[kMaxBlock];
@@ -282,9 +285,9 @@ __global__ void __launch_bounds__(kBlock) k_gm_step(Sell<T> S, uint32_t n, size_
         if (i <= k) {
             const double sum = warp_sum(acc[j]);
             if (lane == 0) {
-                const double h = sum * inv[i];  // v_i = inv_i (slot i)
+                const double h = sum * inv[kVInv + i];  // v_i = inv_i (slot i)
                 H[size_t(i) * m + k] = h;
-                hv[i] = h * inv[i];             // the factor of slot i in w -= h_i v_i
+                hv[i] = h * inv[kVInv + i];             // the factor of slot i in w -= h_i v_i
             }
         }
     }
@@ -310,6 +313,8 @@ __global__ void __launch_bounds__(kBlock) k_gm_correct(uint32_t n, size_t ld, ui
     __shared__ double hv[kMaxRestart + 1];
     __shared__ double hc[kMaxRestart + 1], cc[kMaxRestart], ss[kMaxRestart];
     if (st->done || st->inner_done) return;
+    constexpr bool kScaleZ = PK == 0 && sizeof(T) == 4;
+    const T zs = kScaleZ ? T(st->zscale) : T(1);
     for (uint32_t i = threadIdx.x; i <= k; i += blockDim.x) hv[i] = hv_g[i];
     __syncthreads();
     double acc[1] = {0.0};
@@ -355,7 +360,7 @@ __global__ void __launch_bounds__(kBlock) k_gm_correct(uint32_t n, size_t ld, ui
             for (int e = 0; e < N; e++) {
                 w[e] = T(val[e]);
                 acc[0] += double(w[e]) * double(w[e]);
-                z[e] = PK == 1 ? T(d[size_t(p) * N + e]) * w[e] : w[e];
+                z[e] = PK == 1 ? T(d[size_t(p) * N + e]) * w[e] : kScaleZ ? zs * w[e] : w[e];
             }
             P::st(wv + size_t(p) * N, w);
             if (zn) P::st(zn + size_t(p) * N, z);
@@ -365,7 +370,7 @@ __global__ void __launch_bounds__(kBlock) k_gm_correct(uint32_t n, size_t ld, ui
             const T w = row_value(j);
             wv[j] = w;
             acc[0] += double(w) * double(w);
-            if (zn) zn[j] = PK == 1 ? T(d[j]) * w : w;
+            if (zn) zn[j] = PK == 1 ? T(d[j]) * w : kScaleZ ? zs * w : w;
         }
     } else {
         const uint32_t G = w_, ng = n / G;
@@ -401,7 +406,10 @@ __global__ void __launch_bounds__(kBlock) k_gm_correct(uint32_t n, size_t ld, ui
         // v_{k+1} = w / h_{k+1,k}: its scale is kept in inv, h_{k+1,k} itself is rotated away
         const double hn = sqrt(tot[0]);
         wnorm[k + 1] = hn;
-        inv[k + 1] = hn == 0.0 ? 0.0 : 1.0 / hn;
+        const double s = hn == 0.0 ? 0.0 : 1.0 / hn;
+        inv[kVInv + k + 1] = s;
+        inv[k + 1] = kScaleZ ? s / double(zs) : s;
+        if (kScaleZ) st->zscale = zscale_for(hn);
         for (uint32_t i = 1; i <= k; i++) {
             const double hsave = hc[i - 1], hi = hc[i];
             hc[i - 1] = cc[i - 1] * hsave + ss[i - 1] * hi;
@@ -518,7 +526,8 @@ size_t gmres_workspace_bytes(uint32_t n, uint32_t m, bool mixed, uint32_t w)
 {
     const size_t vn = arena_bytes(n, sizeof(double));
     const size_t vt = arena_bytes(size_t(m + 1) * gmres_ld(n), mixed ? sizeof(float) : sizeof(double));
-    return 2 * vt + vn + arena_bytes(size_t(m + 1) * m, sizeof(double)) + 7 * arena_bytes(m + 2, sizeof(double)) +
+    return 2 * vt + vn + arena_bytes(size_t(m + 1) * m, sizeof(double)) + 6 * arena_bytes(m + 2, sizeof(double)) +
+           arena_bytes(kVInv + m + 2, sizeof(double)) +
            (mixed ? arena_bytes(size_t(n) * w, sizeof(float)) : 0);
 }
 
@@ -540,7 +549,7 @@ rsg_status gmres_carve(rsg_context *ctx, GmresArgs &a, uint32_t n, uint32_t m)
     a.y = arena_take<double>(ctx, m + 2);
     a.hv = arena_take<double>(ctx, m + 2);
     a.wnorm = arena_take<double>(ctx, m + 2);
-    a.inv = arena_take<double>(ctx, m + 2);
+    a.inv = arena_take<double>(ctx, kVInv + m + 2);
     if (!a.inv) return set_error(ctx, RSG_ERR_OUT_OF_MEMORY, "GMRES workspace");
     return RSG_OK;
 }

@@ -351,6 +351,7 @@ extern "C" rsg_status rsg_solve(rsg_context *ctx, rsg_csr *A, const rsg_solver_c
         h.rtol = c.rtol;
         h.max_outer = max_it;
         h.m = m;
+        h.zscale = zscale_for(an / std::sqrt(double(n)));
         h.stop_rule = c.stop_rule;
         h.history = hist;
         h.trend_hist = thist;
