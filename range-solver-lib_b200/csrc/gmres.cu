@@ -323,9 +323,33 @@ __global__ void __launch_bounds__(kBlock) k_gm_correct(uint32_t n, size_t ld, ui
         for (uint32_t i = 0; i <= k; i++) value -= hv[i] * double(V[size_t(i) * ld + j]);
         return T(value);
     };
-    const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+    constexpr int N = P::N;
+    // val -= sum_i hv_i v_i for the N rows at vp of slot 0
+    auto project = [&](const T *vp, double (&val)[N]) {
+        uint32_t i = 0;
+        for (; i + 8 <= k + 1; i += 8) {
+            T a[8][N];
+#pragma unroll
+            for (int u = 0; u < 8; u++) P::ld(vp + size_t(i + u) * ld, a[u]);
+#pragma unroll
+            for (int u = 0; u < 8; u++)
+#pragma unroll
+                for (int e = 0; e < N; e++) val[e] -= hv[i + u] * double(a[u][e]);
+        }
+        if (i <= k) {  // the last one to seven vectors, loaded together
+            T a[7][N];
+#pragma unroll
+            for (int u = 0; u < 7; u++)
+                if (i + u <= k) P::ld(vp + size_t(i + u) * ld, a[u]);
+#pragma unroll
+            for (int u = 0; u < 7; u++)
+                if (i + u <= k)
+#pragma unroll
+                    for (int e = 0; e < N; e++) val[e] -= hv[i + u] * double(a[u][e]);
+        }
+    };
     if (PK < 2) {
-        constexpr int N = P::N;
+        const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
         const uint32_t np = n / N;
         for (uint32_t p = tid; p < np; p += stride) {
             T w[N];
@@ -333,28 +357,7 @@ __global__ void __launch_bounds__(kBlock) k_gm_correct(uint32_t n, size_t ld, ui
             double val[N];
 #pragma unroll
             for (int e = 0; e < N; e++) val[e] = double(w[e]);
-            const T *vp = V + size_t(p) * N;
-            uint32_t i = 0;
-            for (; i + 8 <= k + 1; i += 8) {
-                T a[8][N];
-#pragma unroll
-                for (int u = 0; u < 8; u++) P::ld(vp + size_t(i + u) * ld, a[u]);
-#pragma unroll
-                for (int u = 0; u < 8; u++)
-#pragma unroll
-                    for (int e = 0; e < N; e++) val[e] -= hv[i + u] * double(a[u][e]);
-            }
-            if (i <= k) {  // the last one to seven vectors, loaded together
-                T a[7][N];
-#pragma unroll
-                for (int u = 0; u < 7; u++)
-                    if (i + u <= k) P::ld(vp + size_t(i + u) * ld, a[u]);
-#pragma unroll
-                for (int u = 0; u < 7; u++)
-                    if (i + u <= k)
-#pragma unroll
-                        for (int e = 0; e < N; e++) val[e] -= hv[i + u] * double(a[u][e]);
-            }
+            project(V + size_t(p) * N, val);
             T z[N];
 #pragma unroll
             for (int e = 0; e < N; e++) {
@@ -373,22 +376,45 @@ __global__ void __launch_bounds__(kBlock) k_gm_correct(uint32_t n, size_t ld, ui
             if (zn) zn[j] = PK == 1 ? T(d[j]) * w : kScaleZ ? zs * w : w;
         }
     } else {
-        const uint32_t G = w_, ng = n / G;
-        for (uint32_t gi = tid; gi < ng; gi += stride) {
-            T wl[kMaxBlock];
-            for (uint32_t j = 0; j < G; j++) {
-                const uint32_t r = gi * G + j;
-                wl[j] = row_value(r);
-                wv[r] = wl[j];
-                acc[0] += double(wl[j]) * double(wl[j]);
+        // Blocks of G rows: tiles of whole blocks and whole packs, w as above and through shared memory, then a row of
+        // its block's inverse per thread.  A thread per block of rows, strided and one vector at a time, left 209k
+        // rows at 60.5 us a step with G = 3 and 110.5 with G = 8, FP64, m = 30: now 50.3 and 54.2 (mixed 46.6 and
+        // 83.0: 42.6 and 45.4); with m = 100 and G = 8 it was slower than a launch per operation had been.
+        __shared__ __align__(16) T ws[PK == 2 ? kBlock * N : 1];
+        const uint32_t G = w_, rows = kBlock / G * G * N;
+        for (uint64_t t0 = uint64_t(blockIdx.x) * rows; t0 < n; t0 += uint64_t(gridDim.x) * rows) {
+            const uint32_t cnt = uint32_t(min(uint64_t(rows), n - t0)), own = threadIdx.x * N;
+            if (own + N <= cnt) {
+                T w[N];
+                P::ld(wv + t0 + own, w);
+                double val[N];
+#pragma unroll
+                for (int e = 0; e < N; e++) val[e] = double(w[e]);
+                project(V + t0 + own, val);
+#pragma unroll
+                for (int e = 0; e < N; e++) {
+                    w[e] = T(val[e]);
+                    acc[0] += double(w[e]) * double(w[e]);
+                }
+                P::st(wv + t0 + own, w);
+                P::st(ws + own, w);
+            } else if (own < cnt) {
+                for (uint32_t j = own; j < cnt; j++) {
+                    const T w = row_value(uint32_t(t0) + j);
+                    wv[t0 + j] = ws[j] = w;
+                    acc[0] += double(w) * double(w);
+                }
             }
+            __syncthreads();
             if (zn)
-                for (uint32_t j = 0; j < G; j++) {
-                    const D *row = d + (size_t(gi) * G + j) * G;
+                for (uint32_t j = threadIdx.x; j < cnt; j += kBlock) {
+                    const D *row = d + (size_t(t0) + j) * G;
+                    const T *wl = ws + j / G * G;
                     T z = T(0);
                     for (uint32_t l = 0; l < G; l++) z += T(row[l]) * wl[l];
-                    zn[size_t(gi) * G + j] = z;
+                    zn[t0 + j] = z;
                 }
+            __syncthreads();
         }
     }
     double tot[1];
@@ -598,7 +624,7 @@ rsg_status run_typed(rsg_context *ctx, const GmresArgs &a, double *seconds)
     const int g_res = spmv_grid(ctx, a.A, (const void *)k_gm_residual<RPW>, s64, RPW);
     const int g_vec = std::min(grid_for(ctx, (const void *)k_gm_update<double>, kBlock, 0, n), kMaxGrid);
     const int g_cor = std::min(grid_for(ctx, (const void *)k_gm_correct<PK, double, double>, kBlock, 0,
-                                        PK < 2 ? (long long)n / (a.mixed ? 4 : 2) : n),
+                                        (long long)n / (a.mixed ? 4 : 2)),
                                kMaxGrid);
     // k_gm_step: every block takes the same number of tiles (the fewest that one wave of blocks allows),
     // since each block adds a ticket and (k + 1) partials.  226,981 rows = 887 tiles, 740 resident
