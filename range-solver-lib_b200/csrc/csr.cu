@@ -234,9 +234,15 @@ static void free_csr(rsg_csr *A)
 }
 
 // Build the SELL-32 copy when its padding costs at most 25% over the CSR (or always when forced); up to
-// kPersistRows rows, where an iteration is latency and not bytes, at most 100%: the loops that keep the
-// whole iteration on the SMs need the slices (567-row heat cube, slices padded to 1.3x: 17.6 -> 3.4 us per
-// CG iteration).
+// kPersistRows rows, where the copy stays in L2, at most 100%: the loops that keep the whole iteration on the SMs
+// need the slices (567-row heat cube, slices padded to 1.3x: 17.6 -> 3.4 us per CG iteration).  The other solvers
+// on ragged 27-point grids, CSR -> padded copy, us per iteration:
+//   rows, padding       graph CG FP64 / mixed        block-Jacobi CG FP64   GMRES FP64     multilevel
+//   512, 1.67           16.3 -> 16.4, 16.3 -> 16.6   16.9 -> 17.3           19.6 -> 17.8   46.6 -> 47.4
+//   8000, 1.49          14.2 -> 14.8, 15.4 -> 14.8   15.5 -> 16.0           17.8 -> 16.8   468 -> 462
+//   64000, 1.98         16.9 -> 14.7, 17.7 -> 16.1   18.0 -> 15.2           24.8 -> 23.1   314 -> 317
+//   125000, 1.46        27.6 -> 17.6, 27.6 -> 18.2   29.8 -> 19.1           38.8 -> 28.8   937 -> 904
+// (rsg_solve_multi, 4 columns at 29791 rows 26.2 -> 27.4, keeps to 25%.)
 static rsg_status build_sell(rsg_context *ctx, rsg_csr *A, bool force)
 {
     A->n_slices = (A->n + 31u) / 32u;
