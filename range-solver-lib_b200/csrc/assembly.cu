@@ -34,7 +34,7 @@ struct rsg_assembly {
     uint32_t *adj_ptr = nullptr, *adj_elem = nullptr;
     uint8_t *adj_loc = nullptr;
     uint16_t *adj_off = nullptr;
-    // heat plans: the (row, adjacent tet) pairs and the coordinates as k_asm_heat reads them (pack_heat_plan)
+    // heat plans, instead of xyz and adj_*: the (row, adjacent tet) pairs (AsmPair) and the coordinates by fours
     uint4 *pair = nullptr;
     uint32_t *pair_ptr = nullptr;
     double4 *xyz4 = nullptr;
@@ -88,14 +88,10 @@ __device__ __forceinline__ uint32_t node_of(const uint4 t, int k)
 }
 
 // ---- heat ----
-// What a thread reads for one (row, adjacent tet) pair: 16 bytes, stored in slices of 32 rows -- pair t of
-// lane l of slice s at pair[(pair_ptr[s] + t) * 32 + l], padded with tet RSG_EOD -- so that a warp's reads
-// are one contiguous 512 bytes.  Two forms:
-//   wide   {tet, local index m of the row's node, offsets of the tet's four nodes in the row as 16 bits
-//          each (0xffff: a fixed node)}; the node numbers come from the tet array;
-//   near   for rows of at most 32 entries whose neighbour nodes are numbered within 32767 of the row's:
-//          {tet, m | offsets as 6 bits each (63: a fixed node), node numbers less the row node's as
-//          16 bits each}, which saves the tet array's scattered 16 bytes per pair and a dependent load.
+// A thread reads its (row, adjacent tet) pairs as AsmPair (assembly_plan.h), a warp's as one contiguous 512 bytes.
+// The host packs them while it builds the plan: packed on the device out of the unpacked arrays, a plan of 10^3 /
+// 40^3 / 100^3 hexes took 1.2 / 16.6 / 344 ms to make (1.0 / 14.9 / 332 before there were pairs) and held both, 0.7 GB
+// at 100^3; packed by the host 0.7 / 14.3 / 321.
 
 __device__ __forceinline__ double4 ld_node(const double4 *p)
 {
@@ -309,76 +305,6 @@ __global__ void __launch_bounds__(kBlock, 3) k_asm_heat_local(uint32_t n_free, u
     if (!o.val32) return;
     double tot[1];
     if (grid_sum<1>(nrm, o.partials, o.ticket, sh, tot) && threadIdx.x == 0) *o.norm = sqrt(tot[0]);
-}
-
-// Pairs per 32-row slice (the longest adjacency of its rows) and the packed pairs themselves.
-__global__ void k_pair_len(uint32_t n_free, uint32_t n_slices, const uint32_t *__restrict__ row_node,
-                           const uint32_t *__restrict__ adj_ptr, uint32_t *__restrict__ len)
-{
-    for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < n_slices; s += gridDim.x * blockDim.x) {
-        uint32_t m = 0;
-        for (uint32_t r = s * 32u; r < min(n_free, s * 32u + 32u); r++)
-            m = max(m, adj_ptr[row_node[r] + 1] - adj_ptr[row_node[r]]);
-        len[s] = m;
-    }
-}
-
-// near (in: the near form is allowed by the row lengths; out: still 1 if every node number fits).
-__global__ void k_pair_near(uint32_t n_free, const uint32_t *__restrict__ row_node,
-                            const uint32_t *__restrict__ adj_ptr, const uint32_t *__restrict__ adj_elem,
-                            const uint4 *__restrict__ tets, uint32_t *near)
-{
-    bool ok = true;
-    for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < n_free; r += gridDim.x * blockDim.x) {
-        const uint32_t a = row_node[r];
-        for (uint32_t t = adj_ptr[a]; t < adj_ptr[a + 1]; t++)
-            for (int n = 0; n < 4; n++) {
-                const long long d = (long long)node_of(tets[adj_elem[t]], n) - (long long)a;
-                ok = ok && d >= -32768 && d <= 32767;
-            }
-    }
-    if (!ok) *near = 0u;
-}
-
-__global__ void k_pair_fill(uint32_t n_free, uint32_t n_slices, const uint32_t *__restrict__ row_node,
-                            const uint32_t *__restrict__ adj_ptr, const uint32_t *__restrict__ adj_elem,
-                            const uint8_t *__restrict__ adj_loc, const ushort4 *__restrict__ adj_off,
-                            const uint4 *__restrict__ tets, const uint32_t *__restrict__ pair_ptr,
-                            uint4 *__restrict__ pair, int near)
-{
-    for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < n_slices * 32u; r += gridDim.x * blockDim.x) {
-        const uint32_t s = r >> 5, t0 = pair_ptr[s], nt = pair_ptr[s + 1] - t0;
-        const uint32_t a = r < n_free ? row_node[r] : 0u;
-        const uint32_t beg = adj_ptr[a], cnt = r < n_free ? adj_ptr[a + 1] - beg : 0u;
-        for (uint32_t t = 0; t < nt; t++) {
-            uint4 v = make_uint4(RSG_EOD, 0u, 0u, 0u);
-            if (t < cnt) {
-                const ushort4 o4 = adj_off[beg + t];
-                const uint32_t off[4] = {o4.x, o4.y, o4.z, o4.w};
-                v.x = adj_elem[beg + t];
-                v.y = adj_loc[beg + t];
-                if (near) {
-                    uint32_t d[4];
-                    for (int n = 0; n < 4; n++) {
-                        v.y |= (off[n] == kNoEntry ? 63u : off[n]) << (2 + 6 * n);
-                        d[n] = (node_of(tets[v.x], n) - a) & 0xffffu;
-                    }
-                    v.z = d[0] | d[1] << 16;
-                    v.w = d[2] | d[3] << 16;
-                } else {
-                    v.z = off[0] | off[1] << 16;
-                    v.w = off[2] | off[3] << 16;
-                }
-            }
-            pair[size_t(t0 + t) * 32 + (r & 31u)] = v;
-        }
-    }
-}
-
-__global__ void k_xyz4(uint32_t n_nodes, const double *__restrict__ xyz, double4 *__restrict__ out)
-{
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_nodes; i += gridDim.x * blockDim.x)
-        out[i] = make_double4(xyz[3 * size_t(i)], xyz[3 * size_t(i) + 1], xyz[3 * size_t(i) + 2], 0.0);
 }
 
 // Row (3n+j) of the 12x6 strain-displacement matrix Be (strain order xx yy zz yz xz xy).
@@ -743,7 +669,7 @@ void free_plan(rsg_assembly *p)
 
 rsg_status create_plan(rsg_context *ctx, uint32_t n_nodes, const double *xyz, uint32_t n_tets, const uint32_t *tets,
                        uint32_t n_tris, const uint32_t *tris, const uint32_t *book, uint32_t dofs, uint32_t n_free,
-                       rsg_assembly **out)
+                       int kind, rsg_assembly **out)
 {
     if (!ctx || !out || !xyz || !tets || !book || n_nodes == 0 || n_tets == 0 || n_free == 0 ||
         (n_tris && !tris))
@@ -752,11 +678,13 @@ rsg_status create_plan(rsg_context *ctx, uint32_t n_nodes, const double *xyz, ui
     RSG_CHECK_CUDA(ctx, cudaSetDevice(ctx->device));
     AsmPlanHost H;
     std::string err;
-    if (!build_assembly_plan(n_nodes, n_tets, tets, n_tris, tris, book, dofs, n_free, H, err))
+    const bool heat = kind == kPlanHeat;
+    if (!build_assembly_plan(n_nodes, n_tets, tets, n_tris, tris, book, dofs, n_free, heat, H, err))
         return set_error(ctx, RSG_ERR_INVALID_ARG, "assembly_create: %s", err.c_str());
     static std::atomic<uint64_t> plans{0};
     auto *p = new rsg_assembly;
     p->id = ++plans;
+    p->kind = kind;
     p->n_nodes = n_nodes;
     p->n_tets = n_tets;
     p->n_tris = n_tris;
@@ -768,7 +696,22 @@ rsg_status create_plan(rsg_context *ctx, uint32_t n_nodes, const double *xyz, ui
     auto chk = [&](rsg_status r) {
         if (s == RSG_OK) s = r;
     };
-    chk(upload(ctx, &p->xyz, xyz, size_t(n_nodes) * 3));
+    std::vector<double> xyz4;
+    if (heat) {
+        xyz4.resize(size_t(n_nodes) * 4);
+        for (size_t i = 0; i < n_nodes; i++)
+            for (int k = 0; k < 3; k++) xyz4[4 * i + k] = xyz[3 * i + k];
+        p->near = H.near;
+        chk(upload(ctx, &p->xyz4, reinterpret_cast<const double4 *>(xyz4.data()), n_nodes));
+        chk(upload(ctx, &p->pair, reinterpret_cast<const uint4 *>(H.pair.get()), size_t(H.pair_ptr.back()) * 32));
+        chk(upload(ctx, &p->pair_ptr, H.pair_ptr.data(), H.pair_ptr.size()));
+    } else {
+        chk(upload(ctx, &p->xyz, xyz, size_t(n_nodes) * 3));
+        chk(upload(ctx, &p->adj_ptr, H.adj_ptr.data(), H.adj_ptr.size()));
+        chk(upload(ctx, &p->adj_elem, H.adj_elem.data(), H.adj_elem.size()));
+        chk(upload(ctx, &p->adj_loc, H.adj_loc.data(), H.adj_loc.size()));
+        chk(upload(ctx, &p->adj_off, H.adj_off.data(), H.adj_off.size()));
+    }
     chk(upload(ctx, &p->tets, tets, size_t(n_tets) * 4));
     chk(upload(ctx, &p->tris, n_tris ? tris : nullptr, size_t(n_tris) * 3));
     chk(upload(ctx, &p->book, book, size_t(n_nodes) * dofs));
@@ -776,10 +719,6 @@ rsg_status create_plan(rsg_context *ctx, uint32_t n_nodes, const double *xyz, ui
     chk(upload(ctx, &p->row_comp, H.row_comp.data(), H.row_comp.size()));
     chk(upload(ctx, &p->rp, H.rp.data(), H.rp.size()));
     chk(upload(ctx, &p->ci, H.ci.data(), H.ci.size()));
-    chk(upload(ctx, &p->adj_ptr, H.adj_ptr.data(), H.adj_ptr.size()));
-    chk(upload(ctx, &p->adj_elem, H.adj_elem.data(), H.adj_elem.size()));
-    chk(upload(ctx, &p->adj_loc, H.adj_loc.data(), H.adj_loc.size()));
-    chk(upload(ctx, &p->adj_off, H.adj_off.data(), H.adj_off.size()));
     chk(upload(ctx, &p->tadj_ptr, H.tadj_ptr.data(), H.tadj_ptr.size()));
     chk(upload(ctx, &p->tadj_tri, H.tadj_tri.empty() ? nullptr : H.tadj_tri.data(), H.tadj_tri.size()));
     chk(upload(ctx, &p->node_mask, H.node_mask.data(), H.node_mask.size()));
@@ -792,55 +731,6 @@ rsg_status create_plan(rsg_context *ctx, uint32_t n_nodes, const double *xyz, ui
         return s;
     }
     *out = p;
-    return RSG_OK;
-}
-
-// The pairs and coordinates of a heat plan in the layout of k_asm_heat; the arrays they replace are freed.
-rsg_status pack_heat_plan(rsg_context *ctx, rsg_assembly *p)
-{
-    const uint32_t n_slices = (p->n_free + 31u) / 32u;
-    const int gs = int(std::min<uint32_t>((n_slices + kBlock - 1) / kBlock, 4096u));
-    RSG_TRY(upload<uint32_t>(ctx, &p->pair_ptr, nullptr, size_t(n_slices) + 1));
-    const int gr = int(std::min<uint32_t>((n_slices * 32u + kBlock - 1) / kBlock, 65535u));
-    const uint4 *tets = reinterpret_cast<const uint4 *>(p->tets);
-    k_pair_len<<<gs, kBlock, 0, ctx->stream>>>(p->n_free, n_slices, p->row_node, p->adj_ptr, p->pair_ptr);
-    std::vector<uint32_t> ptr(size_t(n_slices) + 1);  // the last word is the near flag on its way here
-    const uint32_t near0 = p->max_row <= 32 ? 1u : 0u;
-    RSG_CHECK_CUDA(ctx, cudaMemcpyAsync(p->pair_ptr + n_slices, &near0, sizeof(near0), cudaMemcpyHostToDevice,
-                                        ctx->stream));
-    k_pair_near<<<gr, kBlock, 0, ctx->stream>>>(p->n_free, p->row_node, p->adj_ptr, p->adj_elem, tets,
-                                                p->pair_ptr + n_slices);
-    RSG_CHECK_CUDA(ctx, cudaMemcpyAsync(ptr.data(), p->pair_ptr, ptr.size() * sizeof(uint32_t), cudaMemcpyDeviceToHost,
-                                        ctx->stream));
-    RSG_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    p->near = ptr[n_slices] != 0;
-    uint64_t total = 0;
-    for (uint32_t s = 0; s <= n_slices; s++) {
-        const uint32_t len = s < n_slices ? ptr[s] : 0u;
-        ptr[s] = uint32_t(total);
-        total += len;
-    }
-    if (total > 0xffffffffull) return set_error(ctx, RSG_ERR_UNSUPPORTED, "assembly_create: too many row-tet pairs");
-    RSG_CHECK_CUDA(ctx, cudaMemcpyAsync(p->pair_ptr, ptr.data(), ptr.size() * sizeof(uint32_t), cudaMemcpyHostToDevice,
-                                        ctx->stream));
-    RSG_TRY(upload<uint4>(ctx, &p->pair, nullptr, size_t(total) * 32));
-    RSG_TRY(upload<double4>(ctx, &p->xyz4, nullptr, p->n_nodes));
-    k_pair_fill<<<gr, kBlock, 0, ctx->stream>>>(p->n_free, n_slices, p->row_node, p->adj_ptr, p->adj_elem, p->adj_loc,
-                                                reinterpret_cast<const ushort4 *>(p->adj_off), tets, p->pair_ptr,
-                                                p->pair, p->near ? 1 : 0);
-    k_xyz4<<<int(std::min<uint32_t>((p->n_nodes + kBlock - 1) / kBlock, 65535u)), kBlock, 0, ctx->stream>>>(
-        p->n_nodes, p->xyz, p->xyz4);
-    RSG_CHECK_CUDA(ctx, cudaGetLastError());
-    RSG_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    cudaFree(p->adj_ptr);
-    cudaFree(p->adj_elem);
-    cudaFree(p->adj_loc);
-    cudaFree(p->adj_off);
-    cudaFree(p->xyz);
-    p->adj_ptr = p->adj_elem = nullptr;
-    p->adj_loc = nullptr;
-    p->adj_off = nullptr;
-    p->xyz = nullptr;
     return RSG_OK;
 }
 
@@ -914,24 +804,14 @@ extern "C" {
 rsg_status rsg_assembly_create_heat(rsg_context *ctx, uint32_t n_nodes, const double *xyz, uint32_t n_tets,
                                     const uint32_t *tets, const uint32_t *book, uint32_t n_free, rsg_assembly **out)
 {
-    rsg_status s = create_plan(ctx, n_nodes, xyz, n_tets, tets, 0, nullptr, book, 1, n_free, out);
-    if (s != RSG_OK) return s;
-    (*out)->kind = kPlanHeat;
-    s = pack_heat_plan(ctx, *out);
-    if (s != RSG_OK) {
-        free_plan(*out);
-        *out = nullptr;
-    }
-    return s;
+    return create_plan(ctx, n_nodes, xyz, n_tets, tets, 0, nullptr, book, 1, n_free, kPlanHeat, out);
 }
 
 rsg_status rsg_assembly_create_stress(rsg_context *ctx, uint32_t n_nodes, const double *xyz, uint32_t n_tets,
                                       const uint32_t *tets, uint32_t n_tris, const uint32_t *tris,
                                       const uint32_t *book, uint32_t n_free, rsg_assembly **out)
 {
-    const rsg_status s = create_plan(ctx, n_nodes, xyz, n_tets, tets, n_tris, tris, book, 3, n_free, out);
-    if (s == RSG_OK) (*out)->kind = kPlanStress;
-    return s;
+    return create_plan(ctx, n_nodes, xyz, n_tets, tets, n_tris, tris, book, 3, n_free, kPlanStress, out);
 }
 
 rsg_status rsg_assembly_create_magnetostatics(rsg_context *ctx, uint32_t n_nodes, const double *xyz,
@@ -952,9 +832,7 @@ rsg_status rsg_assembly_create_magnetostatics(rsg_context *ctx, uint32_t n_nodes
             return set_error(ctx, RSG_ERR_INVALID_ARG,
                              "assembly_create_magnetostatics: node %u: components must sit at 3*position + c", nd);
     }
-    const rsg_status s = create_plan(ctx, n_nodes, xyz, n_tets, tets, 0, nullptr, book, 3, n_free, out);
-    if (s == RSG_OK) (*out)->kind = kPlanMagnetostatics;
-    return s;
+    return create_plan(ctx, n_nodes, xyz, n_tets, tets, 0, nullptr, book, 3, n_free, kPlanMagnetostatics, out);
 }
 
 void rsg_assembly_destroy(rsg_context *ctx, rsg_assembly *plan)

@@ -35,16 +35,57 @@ void neighbours(const AsmPlanHost &P, const uint32_t *tets, uint32_t a, std::vec
     std::sort(nb.begin(), nb.end());
     nb.erase(std::unique(nb.begin(), nb.end()), nb.end());
 }
+
+// Columns and pairs of the rows of a plan with one component per node (row_node, rp, adj_* and near are there).
+void fill_pairs(AsmPlanHost &P, const uint32_t *tets, const uint32_t *book)
+{
+    const int64_t slices = int64_t(P.pair_ptr.size()) - 1;
+#pragma omp parallel
+    {
+        std::vector<uint32_t> nb;
+#pragma omp for schedule(dynamic, 4)
+        for (int64_t s = 0; s < slices; s++)
+            for (uint32_t l = 0; l < 32; l++) {
+                AsmPair *out = P.pair.get() + size_t(P.pair_ptr[s]) * 32 + l;
+                const uint32_t len = P.pair_ptr[s + 1] - P.pair_ptr[s], r = uint32_t(s) * 32 + l;
+                uint32_t t = 0;
+                if (r < P.n_free) {
+                    const uint32_t a = P.row_node[r], beg = P.adj_ptr[a], cnt = P.adj_ptr[a + 1] - beg;
+                    neighbours(P, tets, a, nb);
+                    for (size_t k = 0; k < nb.size(); k++) P.ci[P.rp[r] + k] = book[nb[k]];
+                    for (; t < cnt; t++) {
+                        const uint32_t e = P.adj_elem[beg + t], *tv = tets + 4 * size_t(e);
+                        uint32_t off[4], d[4];
+                        for (int k = 0; k < 4; k++) {
+                            off[k] = P.node_mask[tv[k]]
+                                         ? uint32_t(std::lower_bound(nb.begin(), nb.end(), tv[k]) - nb.begin())
+                                         : 0xffffu;
+                            d[k] = (tv[k] - a) & 0xffffu;
+                        }
+                        AsmPair v = {e, P.adj_loc[beg + t], off[0] | off[1] << 16, off[2] | off[3] << 16};
+                        if (P.near) {
+                            for (int k = 0; k < 4; k++) v.y |= (off[k] == 0xffffu ? 63u : off[k]) << (2 + 6 * k);
+                            v.z = d[0] | d[1] << 16;
+                            v.w = d[2] | d[3] << 16;
+                        }
+                        out[size_t(t) * 32] = v;
+                    }
+                }
+                for (; t < len; t++) out[size_t(t) * 32] = AsmPair{kEod, 0, 0, 0};
+            }
+    }
+}
 }  // namespace
 
 bool build_assembly_plan(uint32_t n_nodes, uint32_t n_tets, const uint32_t *tets, uint32_t n_tris,
-                         const uint32_t *tris, const uint32_t *book, uint32_t dofs, uint32_t n_free,
+                         const uint32_t *tris, const uint32_t *book, uint32_t dofs, uint32_t n_free, bool pack_pairs,
                          AsmPlanHost &P, std::string &err)
 {
     if (dofs != 1 && dofs != 3) {
         err = "dofs per node must be 1 or 3";
         return false;
     }
+    pack_pairs = pack_pairs && dofs == 1;
     P = AsmPlanHost();
     P.n_nodes = n_nodes;
     P.n_tets = n_tets;
@@ -115,11 +156,11 @@ bool build_assembly_plan(uint32_t n_nodes, uint32_t n_tets, const uint32_t *tets
 
     // pass 1: row lengths (columns of a node's rows = free comps of its neighbours)
     std::vector<uint32_t> node_len(n_nodes, 0);
-    bool too_long = false;
+    bool too_long = false, far = false;
 #pragma omp parallel
     {
         std::vector<uint32_t> nb;
-#pragma omp for schedule(dynamic, 1024) reduction(|| : too_long)
+#pragma omp for schedule(dynamic, 1024) reduction(|| : too_long, far)
         for (int64_t a = 0; a < int64_t(n_nodes); a++) {
             if (!P.node_mask[a]) continue;
             neighbours(P, tets, uint32_t(a), nb);
@@ -127,6 +168,13 @@ bool build_assembly_plan(uint32_t n_nodes, uint32_t n_tets, const uint32_t *tets
             for (uint32_t b : nb) len += popc(P.node_mask[b]);
             node_len[a] = len;
             if (len >= 0xffffu) too_long = true;
+            if (len > 32) far = true;
+            if (pack_pairs)
+                for (uint32_t t = P.adj_ptr[a]; t < P.adj_ptr[a + 1] && !far; t++)
+                    for (int k = 0; k < 4; k++) {
+                        const int64_t d = int64_t(tets[4 * size_t(P.adj_elem[t]) + k]) - a;
+                        far = far || d < -32768 || d > 32767;
+                    }
         }
     }
     if (too_long) {
@@ -143,6 +191,26 @@ bool build_assembly_plan(uint32_t n_nodes, uint32_t n_tets, const uint32_t *tets
         P.rp[r + 1] = uint32_t(e);
     }
     P.ci.resize(P.rp[n_free]);
+    if (pack_pairs) {
+        const uint32_t slices = uint32_t((uint64_t(n_free) + 31) / 32);
+        P.near = !far;
+        P.pair_ptr.assign(size_t(slices) + 1, 0);
+        uint64_t total = 0;
+        for (uint32_t s = 0; s < slices; s++) {
+            uint32_t len = 0;
+            for (uint64_t r = uint64_t(s) * 32; r < std::min<uint64_t>(n_free, uint64_t(s) * 32 + 32); r++)
+                len = std::max(len, P.adj_ptr[P.row_node[r] + 1] - P.adj_ptr[P.row_node[r]]);
+            total += len;
+            if (total > 0xffffffffull) {
+                err = "too many row-tet pairs";
+                return false;
+            }
+            P.pair_ptr[s + 1] = uint32_t(total);
+        }
+        P.pair.reset(new AsmPair[size_t(total) * 32]);  // not initialised: every thread touches its slices first
+        fill_pairs(P, tets, book);
+        return true;
+    }
     P.adj_off.assign(size_t(n_tets) * 4 * 4, 0xffffu);
 
     // pass 2: columns and the scatter map
