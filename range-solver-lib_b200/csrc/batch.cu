@@ -788,41 +788,15 @@ rsg_status rsg_batch_solve(rsg_context *ctx, rsg_batch *B, const rsg_solver_conf
     };
     const bool pdl = pdl_for(B->A, mixed);
 
-    rsg_status status = RSG_OK;
     if (conf->use_graph) {
         cudaGraph_t graph = nullptr;
         cudaGraphExec_t exec = nullptr;
-        RSG_CHECK_CUDA(ctx, cudaGraphCreate(&graph, 0));
-        do {
-            cudaGraphConditionalHandle h;
-            if (cudaGraphConditionalHandleCreate(&h, graph, 1, cudaGraphCondAssignDefault) != cudaSuccess) {
-                status = set_error(ctx, RSG_ERR_CUDA, "batch: conditional handle");
-                break;
-            }
-            cudaGraphNodeParams cp = {};
-            cp.type = cudaGraphNodeTypeConditional;
-            cp.conditional.handle = h;
-            cp.conditional.type = cudaGraphCondTypeWhile;
-            cp.conditional.size = 1;
-            cudaGraphNode_t node;
-            if (cudaGraphAddNode(&node, graph, nullptr, 0, &cp) != cudaSuccess ||
-                cudaStreamBeginCaptureToGraph(sm, cp.conditional.phGraph_out[0], nullptr, nullptr, 0,
-                                              cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
-                status = set_error(ctx, RSG_ERR_CUDA, "batch: graph capture");
-                break;
-            }
-            body(h, 1, pdl);
-            cudaGraph_t captured;
-            if (cudaStreamEndCapture(sm, &captured) != cudaSuccess || cudaGraphInstantiate(&exec, graph, 0) != cudaSuccess ||
-                cudaGraphLaunch(exec, sm) != cudaSuccess) {
-                status = set_error(ctx, RSG_ERR_CUDA, "batch: graph launch");
-                break;
-            }
-        } while (0);
-        cudaError_t e = cudaStreamSynchronize(sm);
-        if (exec) cudaGraphExecDestroy(exec);
+        RSG_TRY(while_graph(ctx, pdl, [&](cudaGraphConditionalHandle h, bool with_pdl) { body(h, 1, with_pdl); }, &graph,
+                            &exec));
+        cudaError_t e = cudaGraphLaunch(exec, sm);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(sm);
+        cudaGraphExecDestroy(exec);
         cudaGraphDestroy(graph);
-        if (status != RSG_OK) return status;
         if (e != cudaSuccess) return set_error(ctx, RSG_ERR_CUDA, "batch solve: %s", cudaGetErrorString(e));
     } else {
         const uint32_t polls = std::max<uint32_t>(1, conf->check_interval / kBatchIterations);

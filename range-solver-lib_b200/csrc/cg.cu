@@ -608,13 +608,13 @@ void set_smem(K k, size_t smem)
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
 }
 
-bool pdl_forced_off()
+}  // namespace
+
+bool pdl_allowed()
 {
     const char *v = std::getenv("RSG_NO_PDL");  // RSG_NO_PDL=1: never (A/B timing)
-    return v && v[0] == '1';
+    return !(v && v[0] == '1');
 }
-
-}  // namespace
 
 // Programmatic dependent launch overlaps the launch of each loop kernel (two or three
 // per iteration) with its predecessor's tail: 2-4% per iteration at 64k rows, neutral
@@ -623,7 +623,7 @@ bool pdl_forced_off()
 // precision.
 bool pdl_for(const rsg_csr *A, bool mixed)
 {
-    if (pdl_forced_off()) return false;
+    if (!pdl_allowed()) return false;
     const int32_t t = mixed ? A->tune.pdl32 : A->tune.pdl64;
     if (A->tune.valid && t >= 0) return t != 0;
     return pdl_default(A);
@@ -705,60 +705,6 @@ void launch_body(rsg_context *ctx, const CgArgs &a, const Launch &L, cudaGraphCo
     launch_k(st, pdl, k_tail, 1, 32, 0, a.st, h, use_cond);
 }
 
-// The solve loop as a graph: one while node whose body is kBodyIterations CG iterations (launch_body)
-// captured from the stream.  On failure nothing is left allocated.
-template <int RPW, int PK>
-rsg_status build_loop_graph(rsg_context *ctx, const CgArgs &a, const Launch &L, bool pdl, cudaGraph_t *graph_out,
-                            cudaGraphExec_t *exec_out)
-{
-    *graph_out = nullptr;
-    *exec_out = nullptr;
-    cudaGraph_t graph = nullptr;
-    RSG_CHECK_CUDA(ctx, cudaGraphCreate(&graph, 0));
-    rsg_status s = RSG_OK;
-    cudaGraphExec_t exec = nullptr;
-    do {
-        cudaGraphConditionalHandle h;
-        if (cudaGraphConditionalHandleCreate(&h, graph, 1, cudaGraphCondAssignDefault) != cudaSuccess) {
-            s = set_error(ctx, RSG_ERR_CUDA, "cudaGraphConditionalHandleCreate failed");
-            break;
-        }
-        cudaGraphNodeParams cp = {};
-        cp.type = cudaGraphNodeTypeConditional;
-        cp.conditional.handle = h;
-        cp.conditional.type = cudaGraphCondTypeWhile;
-        cp.conditional.size = 1;
-        cudaGraphNode_t node;
-        if (cudaGraphAddNode(&node, graph, nullptr, 0, &cp) != cudaSuccess) {
-            s = set_error(ctx, RSG_ERR_CUDA, "adding the while node failed");
-            break;
-        }
-        cudaGraph_t body = cp.conditional.phGraph_out[0];
-        if (cudaStreamBeginCaptureToGraph(ctx->stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal) !=
-            cudaSuccess) {
-            s = set_error(ctx, RSG_ERR_CUDA, "capture into the loop body failed");
-            break;
-        }
-        launch_body<RPW, PK>(ctx, a, L, h, 1, pdl, PK == 3 ? 2 : kBodyIterations);
-        cudaGraph_t captured = nullptr;
-        cudaError_t e = cudaStreamEndCapture(ctx->stream, &captured);
-        if (e != cudaSuccess) {
-            s = set_error(ctx, RSG_ERR_CUDA, "end capture: %s", cudaGetErrorString(e));
-            break;
-        }
-        e = cudaGraphInstantiate(&exec, graph, 0);
-        if (e != cudaSuccess) s = set_error(ctx, RSG_ERR_CUDA, "graph instantiate: %s", cudaGetErrorString(e));
-    } while (0);
-    if (s != RSG_OK) {
-        if (exec) cudaGraphExecDestroy(exec);
-        cudaGraphDestroy(graph);
-        return s;
-    }
-    *graph_out = graph;
-    *exec_out = exec;
-    return RSG_OK;
-}
-
 template <int RPW, int PK>
 rsg_status run_typed(rsg_context *ctx, const CgArgs &a)
 {
@@ -810,12 +756,10 @@ rsg_status run_typed(rsg_context *ctx, const CgArgs &a)
     } else if (a.use_graph) {
         cudaGraph_t graph = nullptr;
         cudaGraphExec_t exec = nullptr;
-        const bool pdl = pdl_for(a.A, a.mixed);
-        rsg_status s = build_loop_graph<RPW, PK>(ctx, a, L, pdl, &graph, &exec);
-        if (s != RSG_OK && pdl) {  // the driver refused the programmatic edges: rebuild without them
-            (void)cudaGetLastError();
-            s = build_loop_graph<RPW, PK>(ctx, a, L, false, &graph, &exec);
-        }
+        // the solve loop: one while node whose body is kBodyIterations CG iterations
+        rsg_status s = while_graph(ctx, pdl_for(a.A, a.mixed), [&](cudaGraphConditionalHandle h, bool pdl) {
+            launch_body<RPW, PK>(ctx, a, L, h, 1, pdl, PK == 3 ? 2 : kBodyIterations);
+        }, &graph, &exec);
         if (s == RSG_OK) {
             cudaError_t e = cudaGraphLaunch(exec, ctx->stream);
             if (e != cudaSuccess) s = set_error(ctx, RSG_ERR_CUDA, "graph launch: %s", cudaGetErrorString(e));

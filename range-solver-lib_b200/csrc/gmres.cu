@@ -636,7 +636,7 @@ rsg_status run_typed(rsg_context *ctx, const GmresArgs &a, double *seconds)
 
     // One captured graph per cycle; with the learned preconditioner a second graph
     // (Jacobi z_k) is captured as the fallback.
-    auto capture = [&](rsg_learned *G, bool pdl, cudaGraph_t *graph, cudaGraphExec_t *exec) -> rsg_status {
+    auto capture = [&](rsg_learned *G, bool pdl, bool gnn_pdl, cudaGraph_t *graph, cudaGraphExec_t *exec) -> rsg_status {
         if (G) RSG_TRY(gnn_prepare(ctx, G, a.A, false));  // no allocation inside the capture
         RSG_CHECK_CUDA(ctx, cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
         cudaStream_t st = ctx->stream;
@@ -664,7 +664,7 @@ rsg_status run_typed(rsg_context *ctx, const GmresArgs &a, double *seconds)
                 launch_k(st, pdl, k_gm_vz<PK, double, double>, g_vec, kBlock, 0, n, ld, a.P.w, a.P.d, a.ro, a.wnorm,
                          a.V, a.Z, a.inv, a.st, k);
             if (G) {  // flexible GMRES: z_k = M(v_k) from the network (Z is stored, src/rmatrixsolver.cpp:446)
-                const rsg_status gs = gnn_forward(ctx, G, a.A, a.V + size_t(k) * ld, z, nullptr, false, true);
+                const rsg_status gs = gnn_forward(ctx, G, a.A, a.V + size_t(k) * ld, z, nullptr, false, true, gnn_pdl);
                 if (gs != RSG_OK) {
                     cudaGraph_t dummy = nullptr;
                     cudaStreamEndCapture(ctx->stream, &dummy);
@@ -701,10 +701,10 @@ rsg_status run_typed(rsg_context *ctx, const GmresArgs &a, double *seconds)
     // driver refuses the programmatic edges) plain launches
     auto capture_any = [&](rsg_learned *G, cudaGraph_t *graph, cudaGraphExec_t *exec) -> rsg_status {
         const bool pdl = pdl_for(a.A, a.mixed);
-        rsg_status r = capture(G, pdl, graph, exec);
-        if (r != RSG_OK && r != RSG_ERR_OUT_OF_MEMORY && pdl) {
+        rsg_status r = capture(G, pdl, true, graph, exec);
+        if (r != RSG_OK && r != RSG_ERR_OUT_OF_MEMORY && (pdl || (G && pdl_allowed()))) {
             (void)cudaGetLastError();
-            r = capture(G, false, graph, exec);
+            r = capture(G, false, false, graph, exec);
         }
         return r;
     };

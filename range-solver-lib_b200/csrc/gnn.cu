@@ -666,7 +666,7 @@ rsg_status gnn_prepare(rsg_context *ctx, rsg_learned *G, const rsg_csr *A, bool 
 
 // Forward pass: z = M(r).  train -> keep every activation for the backward pass.
 rsg_status gnn_forward(rsg_context *ctx, rsg_learned *G, const rsg_csr *A, const double *r, double *z,
-                       const double *xyz, bool train, bool tensor_cores)
+                       const double *xyz, bool train, bool tensor_cores, bool pdl)
 {
     RSG_TRY(gnn_prepare(ctx, G, A, train));
     const uint32_t n = A->n;
@@ -676,7 +676,7 @@ rsg_status gnn_forward(rsg_context *ctx, rsg_learned *G, const rsg_csr *A, const
     float *rms = G->scal32 + 1;
     const int gv = std::min(grid_for(ctx, (const void *)k_gnn_rms, kBlock, 0, n), kMaxGrid);
     k_gnn_rms<<<gv, kBlock, 0, sm>>>(n, r, G->s, partials, ticket, rms);
-    if (!train && tensor_cores) return gnn_forward_umma(ctx, G, A, r, z, xyz, rms);
+    if (!train && tensor_cores) return gnn_forward_umma(ctx, G, A, r, z, xyz, rms, pdl);
     const int gi = std::min(grid_for(ctx, (const void *)k_gnn_input, kBlock, 0, n), kMaxGrid);
     float *h0 = G->h[0];
     k_gnn_input<<<gi, kBlock, 0, sm>>>(n, r, G->s, G->logd, G->rsum, G->scal32, rms, xyz, G->params,

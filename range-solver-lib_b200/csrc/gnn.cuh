@@ -43,12 +43,13 @@ struct rsg_learned {
 namespace rsg {
 void gnn_free_buffers(rsg_learned *G);
 rsg_status gnn_prepare(rsg_context *ctx, rsg_learned *G, const rsg_csr *A, bool train);
+// pdl: the tensor-core layers with programmatic dependent launch (unless RSG_NO_PDL=1).
 rsg_status gnn_forward(rsg_context *ctx, rsg_learned *G, const rsg_csr *A, const double *r, double *z,
-                       const double *xyz, bool train, bool tensor_cores);
+                       const double *xyz, bool train, bool tensor_cores, bool pdl = true);
 rsg_status gnn_loss_grad(rsg_context *ctx, rsg_learned *G, const rsg_csr *A, const double *r, const double *xyz,
                          bool tensor_cores, double *loss);
 rsg_status gnn_forward_umma(rsg_context *ctx, rsg_learned *G, const rsg_csr *A, const double *r, double *z,
-                            const double *xyz, const float *rms);
+                            const double *xyz, const float *rms, bool pdl);
 bool gnn_umma_setup(rsg_context *ctx, int *grid);
 // Training layers on the tensor cores (tcgen05, BF16 operands, FP32 accumulation; gnn_umma.cu):
 // h_out = h + relu([h, m] W + b); the data backward (dz = g [z + b > 0] to dz, g_prev = g + (dz W^T)[:, :H],

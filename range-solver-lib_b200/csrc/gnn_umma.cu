@@ -393,23 +393,24 @@ bool gnn_umma_setup(rsg_context *ctx, int *grid)
 
 // z = M(r) through the BF16 tensor-core layers; h buffers hb[0], hb[1] (n x 64 BF16 each).
 rsg_status gnn_forward_umma(rsg_context *ctx, rsg_learned *G, const rsg_csr *A, const double *r, double *z,
-                            const double *xyz, const float *rms)
+                            const double *xyz, const float *rms, bool pdl)
 {
     const uint32_t n = A->n;
+    pdl = pdl && pdl_allowed();
     cudaStream_t sm = ctx->stream;
     int gl = 0;
     if (!gnn_umma_setup(ctx, &gl)) return set_error(ctx, RSG_ERR_CUDA, "learned: tensor-core layer set-up");
     const uint32_t tiles = (n + kTileRows - 1) / kTileRows;
     gl = int(std::min<uint32_t>(uint32_t(gl), std::max<uint32_t>(tiles, 1)));
     const int gi = std::min(grid_for(ctx, (const void *)k_gnn_input_bf16, kBlock, 0, (long long)n * 8), kMaxGrid);
-    launch_k(sm, true, k_gnn_input_bf16, gi, kBlock, 0, n, r, (const float *)G->s, (const float *)G->logd,
+    launch_k(sm, pdl, k_gnn_input_bf16, gi, kBlock, 0, n, r, (const float *)G->s, (const float *)G->logd,
            (const float *)G->rsum, (const float *)G->scal32, rms, xyz, (const float *)G->params, G->hb[0]);
     for (int l = 0; l < G->L; l++) {
         const float *W = G->params + off_layer(l), *b = W + size_t(K2) * H;
         const float *pout = G->params + off_layer(G->L);
         const __nv_bfloat16 *hin = G->hb[l & 1];
         __nv_bfloat16 *hout = G->hb[(l + 1) & 1];
-        launch_k(sm, true, l + 1 < G->L ? k_gnn_layer_umma<false> : k_gnn_layer_umma<true>, gl, kThreads, kLayerSmem, n,
+        launch_k(sm, pdl, l + 1 < G->L ? k_gnn_layer_umma<false> : k_gnn_layer_umma<true>, gl, kThreads, kLayerSmem, n,
                (const uint32_t *)A->rp, (const uint32_t *)A->ci, (const float *)G->ew, (const float *)G->s, hin, W, b,
                pout, rms, hout, z, ctx->errw);
     }

@@ -82,6 +82,7 @@ rsg_status autotune_run(rsg_context *ctx, rsg_csr *A, const char *cache_path);
 constexpr uint32_t kPdlDefaultRows = 262144;
 inline bool pdl_default(const rsg_csr *A) { return A->n <= kPdlDefaultRows; }
 bool pdl_for(const rsg_csr *A, bool mixed);
+bool pdl_allowed();  // not switched off by RSG_NO_PDL=1
 
 // Launch of a loop kernel; pdl adds the programmatic stream serialization attribute
 // (captured into a graph as a programmatic edge), so the kernel's blocks are scheduled
@@ -100,6 +101,56 @@ void launch_k(cudaStream_t stream, bool pdl, void (*k)(P...), dim3 grid, int blo
     cfg.attrs = &at;
     cfg.numAttrs = pdl ? 1 : 0;
     cudaLaunchKernelEx(&cfg, k, std::forward<A>(args)...);
+}
+
+// A graph of one while node whose body is what body(handle, pdl) launches on the context's stream; with plain
+// launches if the driver refuses the programmatic edges.  On failure nothing is left allocated.
+template <class BODY>
+rsg_status while_graph(rsg_context *ctx, bool pdl, BODY body, cudaGraph_t *graph_out, cudaGraphExec_t *exec_out)
+{
+    *graph_out = nullptr;
+    *exec_out = nullptr;
+    cudaGraph_t graph = nullptr;
+    RSG_CHECK_CUDA(ctx, cudaGraphCreate(&graph, 0));
+    rsg_status s = RSG_OK;
+    cudaGraphExec_t exec = nullptr;
+    do {
+        cudaGraphConditionalHandle h;
+        if (cudaGraphConditionalHandleCreate(&h, graph, 1, cudaGraphCondAssignDefault) != cudaSuccess) {
+            s = set_error(ctx, RSG_ERR_CUDA, "cudaGraphConditionalHandleCreate failed");
+            break;
+        }
+        cudaGraphNodeParams cp = {};
+        cp.type = cudaGraphNodeTypeConditional;
+        cp.conditional.handle = h;
+        cp.conditional.type = cudaGraphCondTypeWhile;
+        cp.conditional.size = 1;
+        cudaGraphNode_t node;
+        if (cudaGraphAddNode(&node, graph, nullptr, 0, &cp) != cudaSuccess) {
+            s = set_error(ctx, RSG_ERR_CUDA, "adding the while node failed");
+            break;
+        }
+        if (cudaStreamBeginCaptureToGraph(ctx->stream, cp.conditional.phGraph_out[0], nullptr, nullptr, 0,
+                                          cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
+            s = set_error(ctx, RSG_ERR_CUDA, "capture into the loop body failed");
+            break;
+        }
+        body(h, pdl);
+        cudaGraph_t captured = nullptr;
+        cudaError_t e = cudaStreamEndCapture(ctx->stream, &captured);
+        if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);
+        if (e != cudaSuccess) s = set_error(ctx, RSG_ERR_CUDA, "loop graph: %s", cudaGetErrorString(e));
+    } while (0);
+    if (s != RSG_OK) {
+        if (exec) cudaGraphExecDestroy(exec);
+        cudaGraphDestroy(graph);
+        if (!pdl) return s;
+        (void)cudaGetLastError();
+        return while_graph(ctx, false, body, graph_out, exec_out);
+    }
+    *graph_out = graph;
+    *exec_out = exec;
+    return RSG_OK;
 }
 
 // Runs the loop from the state *a.st.  The cooperative loops are only queued (the caller synchronises once,

@@ -507,17 +507,17 @@ struct MrArgs {
 };
 
 template <int K>
-void mr_body(rsg_context *ctx, const MrArgs &a, cudaGraphConditionalHandle h, int use_cond)
+void mr_body(rsg_context *ctx, const MrArgs &a, cudaGraphConditionalHandle h, int use_cond, bool pdl)
 {
     cudaStream_t sm = ctx->stream;
     for (int half = 0; half < 2; half++) {
-        launch_k(sm, true, k_mr_p<K>, a.g, kBlock, 0, a.M.n, a.d, (const double *)a.r, a.p, (const MrState *)a.st);
-        launch_k(sm, true, k_mr_dir<K>, a.g, kBlock, 0, a.M, (const double *)a.p, a.q, a.partials, a.st);
-        launch_k(sm, true, k_mr_update<K>, a.g, kBlock, 0, a.M.n, a.d, (const double *)a.p, (const double *)a.q, a.x,
+        launch_k(sm, pdl, k_mr_p<K>, a.g, kBlock, 0, a.M.n, a.d, (const double *)a.r, a.p, (const MrState *)a.st);
+        launch_k(sm, pdl, k_mr_dir<K>, a.g, kBlock, 0, a.M, (const double *)a.p, a.q, a.partials, a.st);
+        launch_k(sm, pdl, k_mr_update<K>, a.g, kBlock, 0, a.M.n, a.d, (const double *)a.p, (const double *)a.q, a.x,
                  a.r, a.partials, a.st);
-        launch_k(sm, true, k_mr_check<K>, a.g, kBlock, 0, a.M, a.d, a.b, (const double *)a.x, a.r, a.partials, a.st);
+        launch_k(sm, pdl, k_mr_check<K>, a.g, kBlock, 0, a.M, a.d, a.b, (const double *)a.x, a.r, a.partials, a.st);
     }
-    launch_k(sm, true, k_mr_tail, 1, 32, 0, a.st, h, use_cond);
+    launch_k(sm, pdl, k_mr_tail, 1, 32, 0, a.st, h, use_cond);
 }
 
 template <int K>
@@ -535,46 +535,22 @@ rsg_status mr_run(rsg_context *ctx, MrArgs &a, bool use_graph, double *seconds)
     if (use_graph) {
         cudaGraph_t graph = nullptr;
         cudaGraphExec_t exec = nullptr;
-        cudaGraphConditionalHandle h;
-        RSG_CHECK_CUDA(ctx, cudaGraphCreate(&graph, 0));
-        do {
-            if (cudaGraphConditionalHandleCreate(&h, graph, 1, cudaGraphCondAssignDefault) != cudaSuccess) {
-                s = set_error(ctx, RSG_ERR_CUDA, "multi-RHS: conditional handle");
-                break;
-            }
-            cudaGraphNodeParams cp = {};
-            cp.type = cudaGraphNodeTypeConditional;
-            cp.conditional.handle = h;
-            cp.conditional.type = cudaGraphCondTypeWhile;
-            cp.conditional.size = 1;
-            cudaGraphNode_t node;
-            if (cudaGraphAddNode(&node, graph, nullptr, 0, &cp) != cudaSuccess) {
-                s = set_error(ctx, RSG_ERR_CUDA, "multi-RHS: while node");
-                break;
-            }
-            if (cudaStreamBeginCaptureToGraph(ctx->stream, cp.conditional.phGraph_out[0], nullptr, nullptr, 0,
-                                              cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
-                s = set_error(ctx, RSG_ERR_CUDA, "multi-RHS: capture");
-                break;
-            }
-            mr_body<K>(ctx, a, h, 1);
-            cudaGraph_t captured = nullptr;
-            cudaError_t e = cudaStreamEndCapture(ctx->stream, &captured);
-            if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);
-            if (e == cudaSuccess) e = cudaGraphLaunch(exec, ctx->stream);
-            if (e != cudaSuccess) s = set_error(ctx, RSG_ERR_CUDA, "multi-RHS graph: %s", cudaGetErrorString(e));
-        } while (0);
+        s = while_graph(ctx, pdl_allowed(), [&](cudaGraphConditionalHandle h, bool pdl) { mr_body<K>(ctx, a, h, 1, pdl); },
+                        &graph, &exec);
+        if (s != RSG_OK) return s;
+        const cudaError_t e = cudaGraphLaunch(exec, ctx->stream);
+        if (e != cudaSuccess) s = set_error(ctx, RSG_ERR_CUDA, "multi-RHS graph: %s", cudaGetErrorString(e));
         if (s == RSG_OK) {
             cudaError_t e = cudaStreamSynchronize(ctx->stream);
             if (e != cudaSuccess) s = set_error(ctx, RSG_ERR_CUDA, "multi-RHS solve: %s", cudaGetErrorString(e));
         }
-        if (exec) cudaGraphExecDestroy(exec);
+        cudaGraphExecDestroy(exec);
         cudaGraphDestroy(graph);
         if (s != RSG_OK) return s;
     } else {
         int32_t *done_h = reinterpret_cast<int32_t *>(ctx->pinned);
         for (uint64_t b = 0;; b++) {
-            for (int k = 0; k < 8; k++) mr_body<K>(ctx, a, 0, 0);
+            for (int k = 0; k < 8; k++) mr_body<K>(ctx, a, 0, 0, pdl_allowed());
             RSG_CHECK_CUDA(ctx, cudaGetLastError());
             RSG_CHECK_CUDA(ctx, cudaMemcpyAsync(done_h, &a.st->all_done, sizeof(int32_t), cudaMemcpyDeviceToHost,
                                                 ctx->stream));
