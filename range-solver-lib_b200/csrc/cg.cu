@@ -638,6 +638,16 @@ struct Launch {
     DirSell dir_sell = nullptr;              // the FP64 direction kernel of a SELL-32 matrix
 };
 
+// The update's default grid: a block for every 256 pairs (FP64) or quadruples (FP32) of rows, at most three an SM --
+// every block adds a ticket and partials (220k rows, us per iteration: FP64 20.6 with 8 blocks an SM, 20.2 with 3,
+// 21.7 with 2; FP32 20.8 with a block per 256 rows, 18.2 with 296 blocks)
+template <int PK>
+int update_grid(rsg_context *ctx, uint32_t n, bool mixed)
+{
+    return std::min(grid_for(ctx, (const void *)k_cg_update<PK>, kBlock, 0, n / (mixed ? 4 : 2)),
+                    kUpdateBlocksPerSm * ctx->num_sms);
+}
+
 template <int RPW, int PK>
 void launch_init(rsg_context *ctx, const CgArgs &a, const Launch &L)
 {
@@ -726,11 +736,7 @@ rsg_status run_typed(rsg_context *ctx, const CgArgs &a)
     int g_dir64 = L.g_spmv64;
     if (a.A->use_sell) L.dir_sell = pick_dir_sell(ctx, a.A, &g_dir64);
     L.g_spmv32 = spmv_grid(ctx, a.A, (const void *)k_mx_dir<RPW>, L.s32, RPW);
-    // the update's grid: a block for every 256 pairs (FP64) or quadruples (FP32) of rows, at most three an SM --
-    // every block adds a ticket and partials (220k rows, us per iteration: FP64 20.6 with 8 blocks an SM, 20.2
-    // with 3, 21.7 with 2; FP32 20.8 with a block per 256 rows, 18.2 with 296 blocks)
-    L.g_vec = std::min(grid_for(ctx, (const void *)k_cg_update<PK>, kBlock, 0, a.A->n / (a.mixed ? 4 : 2)),
-                       kUpdateBlocksPerSm * ctx->num_sms);
+    L.g_vec = update_grid<PK>(ctx, a.A->n, a.mixed);
     const rsg_csr::Tune &T = a.A->tune;
     L.g_dir64 = T.valid && T.g_dir64 > 0 ? T.g_dir64 : g_dir64;
     L.g_dir32 = T.valid && T.g_dir32 > 0 ? T.g_dir32 : L.g_spmv32;
@@ -861,9 +867,8 @@ rsg_status profile_typed(rsg_context *ctx, const rsg_csr *A, int kernel, uint32_
     if (!dir_sell) g64 = spmv_grid(ctx, A, (const void *)k_cg_dir<RPW>, s64, RPW);
     if (T.valid && T.g_dir64 > 0) g64 = T.g_dir64;
     const int g32 = T.valid && T.g_dir32 > 0 ? T.g_dir32 : spmv_grid(ctx, A, (const void *)k_mx_dir<RPW>, s32, RPW);
-    const int gv = std::min(grid_for(ctx, (const void *)k_cg_update<1>, kBlock, 0, n), kMaxGrid);
-    const int gv64 = T.valid && T.g_upd64 > 0 ? T.g_upd64 : gv;
-    const int gv32 = T.valid && T.g_upd32 > 0 ? T.g_upd32 : gv;
+    const int gv64 = T.valid && T.g_upd64 > 0 ? T.g_upd64 : update_grid<1>(ctx, n, false);
+    const int gv32 = T.valid && T.g_upd32 > 0 ? T.g_upd32 : update_grid<1>(ctx, n, true);
     const Csr<double> M64 = view<double>(A, true);
     const Csr<float> M32 = view<float>(A, true);
     auto launch = [&]() {

@@ -1,0 +1,52 @@
+"""Which kernels a call launches, and with which grids: several loops give one result bit for bit, so that only the
+launches show whether the one meant for a size ran.  Seen through torch's profiler; skipped where it sees none."""
+import json
+
+import numpy as np
+import pytest
+
+import rsg
+from oracle import oracle as O
+from rsg import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture
+def launches(ctx, torch_cuda, tmp_path):
+    torch = torch_cuda
+
+    def run(f):
+        torch.cuda.synchronize()
+        with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA], acc_events=True) as prof:
+            f()
+            ctx.sync()
+            torch.cuda.synchronize()
+        path = tmp_path / "trace.json"
+        prof.export_chrome_trace(str(path))
+        events = json.loads(path.read_text())["traceEvents"]
+        got = [(e["name"], tuple(e["args"]["grid"])) for e in events if e.get("cat") == "kernel"]
+        if not got:
+            pytest.skip("the profiler sees no kernels here")
+        return got
+
+    return run
+
+
+def named(got, name):
+    return [(n, g) for n, g in got if name in n]
+
+
+def heat(n_hex):
+    return O.assemble_heat(W.heat_cube(n_hex, sigma=1.2, seed=4, source="random"))
+
+
+@pytest.mark.parametrize("precision,kernel,kid", [("fp64", "k_cg_update<", 2),
+                                                  ("mixed", "k_mx_update<", 3)])
+def test_profiled_update_has_the_loops_grid(ctx, launches, precision, kernel, kid):
+    A, b = heat(60)  # 215,940 rows: more than three blocks an SM with one thread per row
+    M = ctx.matrix(A.rp, A.ci, A.val)
+    conf = rsg.make_conf(n_outer=4, stop_rule="true", rtol=1e-10, precision=precision, use_graph=False)
+    loop = {g for _, g in named(launches(lambda: ctx.solve(M, b, conf=conf)), kernel)}
+    prof = {g for _, g in named(launches(lambda: ctx.profile_kernel(M, kid, reps=2)), kernel)}
+    assert len(loop) == 1 and loop == prof
