@@ -750,12 +750,15 @@ rsg_status run_typed(rsg_context *ctx, const CgArgs &a)
     const bool persist_ok = a.use_graph && (PK == 0 || PK == 1) && a.A->use_sell && a.persistent >= 0 &&
                             (a.persistent > 0 || a.A->n <= kPersistRows);
     bool persisted = false;
-    if (persist_ok)
-        RSG_TRY(cg_resident_run(ctx, a, a.mixed ? L.g_dir32 : L.g_dir64, a.mixed ? L.g_upd32 : L.g_upd64, L.g_spmv64,
-                                &persisted));
-    if (persist_ok && !persisted)
-        RSG_TRY(cg_persist_run(ctx, a, a.mixed ? L.g_dir32 : L.g_dir64, a.mixed ? L.g_upd32 : L.g_upd64, L.g_spmv64,
-                               &persisted));
+    const int gd = a.mixed ? L.g_dir32 : L.g_dir64, gu = a.mixed ? L.g_upd32 : L.g_upd64;
+    const int gd0 = a.mixed ? L.g_spmv32 : g_dir64;
+    if (persist_ok) RSG_TRY(cg_resident_run(ctx, a, gd, gu, L.g_spmv64, &persisted));
+    // Tuned grids stand for the graph loop's sums in the resident one (cg_resident.cu) and may be too small for that;
+    // they are launch shapes, though, and no reason to give it up (8.4k rows, FP64 5.6 us an iteration against 12.8): it
+    // takes the default grids then.  Not while the tuner times them.
+    if (persist_ok && !persisted && T.valid && !T.trial && (gd != gd0 || gu != L.g_vec))
+        RSG_TRY(cg_resident_run(ctx, a, gd0, L.g_vec, L.g_spmv64, &persisted));
+    if (persist_ok && !persisted) RSG_TRY(cg_persist_run(ctx, a, gd, gu, L.g_spmv64, &persisted));
     if (persisted) {
         if (a.mixed) k_mx_fold<<<L.g_vec, kBlock, 0, ctx->stream>>>(a.A->n, a.x, a.y32, a.st);
         RSG_CHECK_CUDA(ctx, cudaEventRecord(ctx->ev[1], ctx->stream));

@@ -80,6 +80,7 @@ struct rsg_csr {
     struct Tune {
         bool valid = false;
         bool from_cache = false;
+        bool trial = false;           // being timed by the tuner: the loops run with these shapes as they are
         int32_t rpw = 0;              // CSR-stream rows per warp chunk (<= the largest that fits)
         int32_t g_dir64 = 0, g_dir32 = 0, g_upd64 = 0, g_upd32 = 0;
         int32_t pdl64 = -1, pdl32 = -1;  // programmatic dependent launch in the CG loop: 1/0, -1 size default

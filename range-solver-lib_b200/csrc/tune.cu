@@ -160,7 +160,7 @@ rsg_status autotune_run(rsg_context *ctx, rsg_csr *A, const char *cache_path)
     for (const Layout &L : layouts) {
         A->use_sell = L.sell;
         A->tune = rsg_csr::Tune();
-        A->tune.valid = true;
+        A->tune.valid = A->tune.trial = true;
         A->tune.rpw = L.sell ? 0 : L.rpw;
         const long long dir_items = L.sell ? (long long)A->n_slices * 32 : (long long)n * 32 / pick_rpw(A);
         rsg_csr::Tune t = A->tune;
@@ -225,6 +225,7 @@ rsg_status autotune_run(rsg_context *ctx, rsg_csr *A, const char *cache_path)
     }
     A->use_sell = best_sell;
     best.valid = true;
+    best.trial = false;
     best.candidates = B.count;
     best.it64_default = def64;
     best.it32_default = def32;

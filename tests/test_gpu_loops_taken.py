@@ -50,3 +50,22 @@ def test_profiled_update_has_the_loops_grid(ctx, launches, precision, kernel, ki
     loop = {g for _, g in named(launches(lambda: ctx.solve(M, b, conf=conf)), kernel)}
     prof = {g for _, g in named(launches(lambda: ctx.profile_kernel(M, kid, reps=2)), kernel)}
     assert len(loop) == 1 and loop == prof
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_small_tuned_grids_keep_the_resident_loop(ctx, launches, tmp_path, precision):
+    # a tuning cache of one block per kernel: shapes that the resident loop's sums cannot stand for
+    A, b = heat(20)
+    path = tmp_path / "tune.txt"
+    M = ctx.matrix(A.rp, A.ci, A.val)
+    ctx.autotune(M, str(path))
+    key = path.read_text().split(" : ")[0]
+    path.write_text(key + " : sell=1 rpw=0 dir64=1 dir32=1 upd64=1 upd32=1 pdl64=-1 pdl32=-1 it_us=1.000,1.000\n")
+    T = ctx.matrix(A.rp, A.ci, A.val)
+    assert ctx.autotune(T, str(path))["from_cache"] == 1
+    conf = rsg.make_conf(n_outer=20000, stop_rule="true", rtol=1e-10, precision=precision)
+    U = ctx.matrix(A.rp, A.ci, A.val)
+    x, s = ctx.solve(U, b, conf=conf)
+    y, t = ctx.solve(T, b, conf=conf)
+    assert t.iterations == s.iterations and np.array_equal(x, y)
+    assert named(launches(lambda: ctx.solve(T, b, conf=conf)), "k_cg_resident")
