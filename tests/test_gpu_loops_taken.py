@@ -69,3 +69,32 @@ def test_small_tuned_grids_keep_the_resident_loop(ctx, launches, tmp_path, preci
     y, t = ctx.solve(T, b, conf=conf)
     assert t.iterations == s.iterations and np.array_equal(x, y)
     assert named(launches(lambda: ctx.solve(T, b, conf=conf)), "k_cg_resident")
+
+
+@pytest.mark.parametrize("precision,n_hex,transport", [(p, n, t) for n, f, m in [
+    (4, "true", "true"), (8, "true", "true"), (20, "true", "true"), (27, "false", "true"), (41, "false", "false"),
+    (54, None, None)] for p, t in (("fp64", f), ("mixed", m))])
+def test_small_systems_take_the_resident_loop(ctx, launches, precision, n_hex, transport):
+    # 75 to 70,560 rows: one cluster (true), as far as its shared memory holds the matrix, or one block per SM
+    # (false); 160,325 rows: neither
+    A, b = heat(n_hex)
+    M = ctx.matrix(A.rp, A.ci, A.val)
+    conf = rsg.make_conf(n_outer=20000, stop_rule="true", rtol=1e-10, precision=precision)
+    loop = named(launches(lambda: ctx.solve(M, b, conf=conf)), "k_cg_resident<")
+    assert [n.split("k_cg_resident<")[1].split(">")[0].split(", ")[2] for n, _ in loop] == [transport] * bool(transport)
+    graph = rsg.make_conf(n_outer=20000, stop_rule="true", rtol=1e-10, precision=precision, persistent=-1)
+    assert not named(launches(lambda: ctx.solve(M, b, conf=graph)), "k_cg_resident<")
+
+
+@pytest.mark.parametrize("n_hex,cluster", [(14, False), (24, True), (45, True), (74, True), (86, False)])
+def test_coarse_levels_take_the_cluster(ctx, launches, n_hex, cluster):
+    A, b = heat(n_hex)
+    M = ctx.matrix(A.rp, A.ci, A.val)
+    info = ctx.amg_setup(M)
+    assert (len(info["rows"]) > 3 and info["rows"][2] <= 7168) == cluster
+    conf = rsg.make_conf(n_outer=2, stop_rule="true", rtol=1e-10, precision="mixed", use_graph=False)
+    got = launches(lambda: ctx.solve(M, b, conf=conf, prec=rsg.PREC_AMG))
+    visits = named(got, "k_amg_cluster")
+    assert bool(visits) == cluster and all(g == (16, 1, 1) for _, g in visits)
+    # two visits a cycle in place of the dozen launches or more that each takes without the cluster
+    assert (info["cycle_launches"][0] <= 14) == (cluster or len(info["rows"]) <= 3)
