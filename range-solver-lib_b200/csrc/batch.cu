@@ -9,10 +9,12 @@
 // own CG state (the same CgState and transitions as the single-system solver:
 // stop on FP64 true relative residual, FP64 or mixed precision with reliable
 // updates).  Per iteration two kernels (direction + SpMV, update) run over the
-// slices of the active systems: every block takes a contiguous range of the
-// list's slices, so most blocks work for one system, and adds up its part of
-// each system it touches; the last block to finish a system's part (a ticket per
-// system) adds the blocks' sums in block order and advances that system's state.
+// active systems' slices in chunks of one per warp, counted from a system's first
+// slice: every block takes a contiguous range of the list's chunks, so most blocks
+// work for one system, and adds up each chunk; the last block to finish with a
+// system (a ticket per system) adds the chunks' sums in their order and advances
+// that system's state.  So a system's sums do not depend on the grid, nor on the
+// systems beside it.
 // A system whose update asks for a residual check waits (the next directions and
 // updates skip it) until the check that ends each body of kBatchIterations
 // iterations, an FP64 SpMV over the systems that asked.  The loop is one CUDA
@@ -51,6 +53,8 @@ struct BatchCtl {
 };
 
 constexpr int kBatchIterations = 4;
+constexpr uint32_t kChunk = kWarpsPerBlock;  // slices of a chunk
+constexpr uint32_t kHold = 32;               // chunks that a block holds the warps' sums of
 
 struct BView {
     const uint32_t *slice_sys;
@@ -63,12 +67,18 @@ struct BView {
 // instead of a binary search through a chain of them.
 struct ListHead {
     uint32_t n_sys;     // number of listed systems
-    uint32_t n_slices;  // their slices in total
+    uint32_t n_chunks;  // their chunks in total
 };
 struct Active {
     ListHead *head;
-    uint4 *entry;  // per listed system: id, first and last + 1 of its slices in the list, its first slice less the former
+    uint4 *entry;  // per listed system, list_entry
 };
+// {system | (slices of its last chunk - 1) << 29, first and last + 1 of its chunks in the list, its first slice}
+__host__ __device__ __forceinline__ uint4 list_entry(uint32_t sys, uint32_t at, uint32_t first, uint32_t slices)
+{
+    return make_uint4(sys | (slices - 1) % kChunk << 29, at, at + (slices + kChunk - 1) / kChunk, first);
+}
+constexpr uint32_t kSysMask = (1u << 29) - 1;
 
 // Block-wide (blockDim.x == kBlock): lists in order the systems of `in` (0..n_in when it has no entries)
 // that keep(system) accepts.  Every thread calls it; keep must give the same answer on both of its calls.
@@ -81,10 +91,10 @@ __device__ __forceinline__ void build_list(uint32_t n_in, const uint4 *in, const
     const uint32_t i0 = min(n_in, t * per), i1 = min(n_in, i0 + per);
     uint32_t ns = 0, nsl = 0;
     for (uint32_t i = i0; i < i1; i++) {
-        const uint32_t sys = in ? in[i].x : i;
+        const uint32_t sys = in ? in[i].x & kSysMask : i;
         if (keep(sys)) {
             ns++;
-            nsl += sys_slice[sys + 1] - sys_slice[sys];
+            nsl += (sys_slice[sys + 1] - sys_slice[sys] + kChunk - 1) / kChunk;
         }
     }
     // exclusive scans over the block
@@ -110,11 +120,12 @@ __device__ __forceinline__ void build_list(uint32_t n_in, const uint4 *in, const
     if (t == blockDim.x - 1) *out.head = ListHead{a, b};
     uint32_t o = a - ns, pre = b - nsl;
     for (uint32_t i = i0; i < i1; i++) {
-        const uint32_t sys = in ? in[i].x : i;
+        const uint32_t sys = in ? in[i].x & kSysMask : i;
         if (keep(sys)) {
-            const uint32_t first = sys_slice[sys], len = sys_slice[sys + 1] - first;
-            out.entry[o++] = make_uint4(sys, pre, pre + len, first - pre);
-            pre += len;
+            const uint32_t first = sys_slice[sys];
+            const uint4 e = list_entry(sys, pre, first, sys_slice[sys + 1] - first);
+            out.entry[o++] = e;
+            pre = e.z;
         }
     }
     __syncthreads();
@@ -201,32 +212,33 @@ __device__ __forceinline__ void finalize(CgState *st, const double (&acc)[NV], d
 }
 
 
-// The blocks' loop over the listed systems' slices.  Block j takes slices [j per, (j + 1) per) of the list;
-// systems that `skip(st)` rejects are jumped over as a whole.  For every visited slice one warp runs
-// `body(s, st, v)`, which returns the lane's contributions; at the end of a system's stretch the block adds
-// them up.  A system that lies in one block is finished there; otherwise the block stores its sums in slot
-// (block + list position) -- consecutive for a system's blocks, and no two (block, system) pairs share one,
-// as either grows along the list -- and the last block to take the system's ticket adds the slots.  Sums and
-// transition used to be kernels of their own after every phase, with the check in every iteration: 24 uneven
-// cubes (0.39M rows), six and a half launches an iteration, mixed 14.2, FP64 13.4 ms a solve; now 11.0 and
-// 10.5 (29 us an iteration: direction 18.5, update 10.3).
+// The blocks' loop over the listed systems' chunks.  Block j takes chunks [j per, (j + 1) per) of the list; systems
+// that `skip(st)` rejects are jumped over as a whole.  For every visited slice one warp runs `body(s, st, v)`, which
+// returns the lane's contributions; a chunk's sum is its warps' sums in order.  A system that lies in one block is
+// finished there; otherwise the block stores its chunks' sums, and the last block to take the system's ticket adds
+// them.  24 uneven cubes (0.39M rows), ms a solve, mixed / FP64: sums and transition as kernels of their own after
+// every phase, with the check in every iteration, 14.2 / 13.4; a warp's slices of a block added up by the lanes,
+// which made a system's bits depend on the grid and on its companions, 11.0 / 10.5; chunks 9.9 / 9.6.  64 cubes of 8 to
+// 60 hexes a side, mixed: 75.5, 57.4 and 59.4 (a warp sum per slice).  16, 64 and 128 chunks held: within 2%.
 struct Sums {
-    double *part;          // [grid + n_sys][NV]
+    double *part;          // [batch_parts][3]: a system's chunks from its first slice / kChunk + its number on
     unsigned int *ticket;  // per system, zero between uses
     double *relres;        // RED_TRUE only
 };
+inline size_t batch_parts(uint32_t n_slices, uint32_t n_sys) { return size_t(n_slices) / kChunk + n_sys; }
 
 template <int NV, int KIND, class SKIP, class BODY>
 __device__ __forceinline__ void batch_run(const BView &B, const Active L, CgState *S, const Sums &T, SKIP skip, BODY body)
 {
     __shared__ double sh[NV * 32];
+    __shared__ __align__(16) double hold[NV][kHold][kChunk];
     __shared__ CgState s;
     __shared__ int last_sh;
     const uint32_t warp = threadIdx.x >> 5;
-    // the entries that start at or before this block's first slice are the first of the list: count them
+    // the entries that start at or before this block's first chunk are the first of the list: count them
     uint32_t begin = threadIdx.x < B.n_sys ? L.entry[threadIdx.x].y : 0u;
-    const uint32_t total = L.head->n_slices, n_list = L.head->n_sys;
-    const uint32_t per = ((total + gridDim.x - 1) / gridDim.x + kWarpsPerBlock - 1) / kWarpsPerBlock * kWarpsPerBlock;
+    const uint32_t total = L.head->n_chunks, n_list = L.head->n_sys;
+    const uint32_t per = (total + gridDim.x - 1) / gridDim.x;
     uint32_t a = min(uint64_t(total), uint64_t(blockIdx.x) * per);
     const uint32_t a_end = min(total, a + per);
     if (a >= a_end) return;
@@ -238,26 +250,44 @@ __device__ __forceinline__ void batch_run(const BView &B, const Active L, CgStat
     k--;
     for (; a < a_end; k++) {
         const uint4 e = L.entry[k];
-        const uint32_t sys = e.x, k_begin = e.y, k_end = e.z, stop = min(a_end, k_end);
+        const uint32_t sys = e.x & kSysMask, k_begin = e.y, k_end = e.z, stop = min(a_end, k_end);
         CgState *st = &S[sys];
         if (!skip(st)) {
-            const uint32_t base = e.w;
+            const uint32_t chunks = k_end - k_begin;
+            double *part = T.part + (size_t(e.w / kChunk) + sys) * NV;
+            const bool here = chunks <= kHold && a == k_begin && stop == k_end;  // all of it, in one go
             double v[NV];
+            for (; a < stop; a += kHold) {
+                const uint32_t m = min(kHold, stop - a);
+                for (uint32_t j = 0; j < m; j++) {
+                    const uint32_t c = a + j - k_begin;
+                    double t[NV];
 #pragma unroll
-            for (int q = 0; q < NV; q++) v[q] = 0.0;
-            for (uint32_t i = a + warp; i < stop; i += kWarpsPerBlock) {
-                double t[NV];
-                body(base + i, st, t);
+                    for (int q = 0; q < NV; q++) t[q] = 0.0;
+                    if (c + 1 < chunks || warp <= e.x >> 29) body(e.w + c * kChunk + warp, st, t);
 #pragma unroll
-                for (int q = 0; q < NV; q++) v[q] += t[q];
+                    for (int q = 0; q < NV; q++) t[q] = warp_sum(t[q]);
+                    if ((threadIdx.x & 31) == 0)
+#pragma unroll
+                        for (int q = 0; q < NV; q++) hold[q][j][warp] = t[q];
+                }
+                __syncthreads();
+#pragma unroll
+                for (int q = 0; q < NV; q++) {
+                    v[q] = 0.0;
+                    if (threadIdx.x < m) {
+                        const double2 *w = reinterpret_cast<const double2 *>(hold[q][threadIdx.x]);
+                        const double2 w0 = w[0], w2 = w[1], w4 = w[2], w6 = w[3];
+                        v[q] = ((w0.x + w0.y) + (w2.x + w2.y)) + ((w4.x + w4.y) + (w6.x + w6.y));
+                        if (!here) part[size_t(a + threadIdx.x - k_begin) * NV + q] = v[q];
+                    }
+                }
+                __syncthreads();
             }
-            block_sum<NV>(v, sh);
-            const uint32_t first = k_begin / per, n_blocks = (k_end - 1) / per - first + 1;
+            const uint32_t n_blocks = (k_end - 1) / per - k_begin / per + 1;
             if (threadIdx.x == 0) {
                 last_sh = 1;
                 if (n_blocks > 1) {
-#pragma unroll
-                    for (int q = 0; q < NV; q++) T.part[size_t(blockIdx.x + k) * NV + q] = v[q];
                     unsigned int t;
                     asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(t) : "l"(T.ticket + sys) : "memory");
                     last_sh = t == n_blocks - 1;
@@ -267,18 +297,16 @@ __device__ __forceinline__ void batch_run(const BView &B, const Active L, CgStat
             if (last_sh) {
                 for (uint32_t w = threadIdx.x; w < kStateWords; w += blockDim.x)
                     reinterpret_cast<uint32_t *>(&s)[w] = __ldcg(reinterpret_cast<const uint32_t *>(st) + w);
-                if (n_blocks > 1) {
+                if (!here) {
 #pragma unroll
                     for (int q = 0; q < NV; q++) v[q] = 0.0;
 #pragma unroll 4
-                    for (uint32_t i = threadIdx.x; i < n_blocks; i += blockDim.x)
+                    for (uint32_t i = threadIdx.x; i < chunks; i += blockDim.x)
 #pragma unroll
-                        for (int q = 0; q < NV; q++) v[q] += __ldcg(&T.part[size_t(first + k + i) * NV + q]);
-                    block_sum<NV>(v, sh);
+                        for (int q = 0; q < NV; q++) v[q] += __ldcg(&part[size_t(i) * NV + q]);
                     if (threadIdx.x == 0) T.ticket[sys] = 0u;
-                } else {
-                    __syncthreads();
                 }
+                block_sum<NV>(v, sh);
                 if (threadIdx.x == 0) finalize<NV, KIND>(&s, v, T.relres, sys);
                 __syncthreads();
                 if (KIND != RED_TRUE)
@@ -345,7 +373,9 @@ __global__ void __launch_bounds__(kBlock) bk_init_z(BView B, const Active L, uin
         });
 }
 
-// Six blocks an SM (40 registers): 0.39M rows mixed 11.0 ms a solve; seven or eight 11.8, FP64 10.5 against 13.3.
+// Six blocks an SM: 40 registers and 84 to 88 bytes spilled, all the same the fastest but for single sizes; ms a solve
+// with six, five and four, 24 cubes mixed 9.9, 9.9, 10.0, FP64 9.6, 10.0, 9.3; 64 cubes mixed 59.4, 58.8, 64.6, FP64 74.9,
+// 77.4, 75.8.
 template <typename V, bool MIXED>
 __global__ void __launch_bounds__(kBlock, 6) bk_dir(Sell<V> M, BView B, const Active L, const V *__restrict__ z, V *p0,
                                                  V *p1, V *__restrict__ q, double *__restrict__ x,
@@ -659,7 +689,7 @@ rsg_status rsg_batch_solve(rsg_context *ctx, rsg_batch *B, const rsg_solver_conf
     const uint32_t n = B->pad_rows, ns = B->n_sys, nsl = n / 32;
     const uint32_t max_it = std::max<uint32_t>(conf->n_outer, 1);
     const size_t vn = arena_bytes(n, sizeof(double)), vf = arena_bytes(n, sizeof(float));
-    size_t bytes = 8 * vn + arena_bytes((size_t(kMaxGrid) + ns) * 3, sizeof(double)) + arena_bytes(ns, sizeof(CgState)) +
+    size_t bytes = 8 * vn + arena_bytes(batch_parts(nsl, ns) * 3, sizeof(double)) + arena_bytes(ns, sizeof(CgState)) +
                    arena_bytes(ns, sizeof(unsigned int)) +
                    3 * arena_bytes(1, sizeof(ListHead)) + 3 * arena_bytes(ns, sizeof(uint4)) +
                    arena_bytes(ns, sizeof(double)) + arena_bytes(1, sizeof(BatchCtl)) + 2 * arena_bytes(B->user_rows, 8);
@@ -669,7 +699,7 @@ rsg_status rsg_batch_solve(rsg_context *ctx, rsg_batch *B, const rsg_solver_conf
            *z = arena_take<double>(ctx, n), *p0 = arena_take<double>(ctx, n), *p1 = arena_take<double>(ctx, n),
            *q = arena_take<double>(ctx, n), *d = arena_take<double>(ctx, n);
     Sums T = {};
-    T.part = arena_take<double>(ctx, (size_t(kMaxGrid) + ns) * 3);
+    T.part = arena_take<double>(ctx, batch_parts(nsl, ns) * 3);
     T.ticket = arena_take<unsigned int>(ctx, ns);
     CgState *S = arena_take<CgState>(ctx, ns);
     double *relres = T.relres = arena_take<double>(ctx, ns);
@@ -737,9 +767,13 @@ rsg_status rsg_batch_solve(rsg_context *ctx, rsg_batch *B, const rsg_solver_conf
         RSG_CHECK_CUDA(ctx, cudaMemcpyAsync(ctl, &c, sizeof(c), cudaMemcpyHostToDevice, sm));
         // the lists start with every system
         std::vector<uint4> entry(ns);
-        for (uint32_t i = 0; i < ns; i++)
-            entry[i] = make_uint4(i, B->pad_begin[i] / 32, B->pad_begin[i + 1] / 32, 0u);
-        const ListHead head = {ns, nsl};
+        uint32_t chunks = 0;
+        for (uint32_t i = 0; i < ns; i++) {
+            const uint32_t first = B->pad_begin[i] / 32;
+            entry[i] = list_entry(i, chunks, first, B->pad_begin[i + 1] / 32 - first);
+            chunks = entry[i].z;
+        }
+        const ListHead head = {ns, chunks};
         for (const Active *l : {&L_all, &L_act, &L_chk}) {
             RSG_CHECK_CUDA(ctx, cudaMemcpyAsync(l->head, &head, sizeof(head), cudaMemcpyHostToDevice, sm));
             RSG_CHECK_CUDA(ctx, cudaMemcpyAsync(l->entry, entry.data(), ns * sizeof(uint4), cudaMemcpyHostToDevice, sm));
