@@ -231,7 +231,8 @@ __global__ void __launch_bounds__(kBlock) k_asm_heat(uint32_t n_free, const uint
 // coordinates (24 pairs a row; L1 at 63% and FP64 at 21% of peak in the wide form).  Whole numeric assembly
 // of 100^3 hexes (6M tets, 1M rows): 945 us with separate index, offset and node arrays, nine divisions a
 // pair, one thread's scattered stores and three refresh passes (703 + 94 + 136 us); 500 us with the wide
-// form, 464 us with the near form.  Three blocks an SM (80 registers): two 524, four (64, spills) 521 us.
+// form, 464 us with the near form.  Three blocks an SM (80 registers and 20 to 28 bytes spilled): two 524, four (64
+// registers, more spills) 521 us.
 // Loading the next pairs' conductivities a step ahead was slower (503-564 us), as was keeping the row's
 // own node out of the loads.
 constexpr uint32_t kLocalRowMax = 32;

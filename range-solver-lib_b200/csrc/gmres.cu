@@ -170,8 +170,8 @@ __global__ void __launch_bounds__(kBlock) k_gm_vz(uint32_t n, size_t ld, uint32_
 
 // w = A z_k, for matrices without the SELL-32 copy (k_gm_step then starts from the stored w).
 template <int RPW, typename T>
-__global__ void __launch_bounds__(kBlock) k_gm_spmv(Csr<T> M, Sell<T> S, int use_sell, const T *__restrict__ z,
-                                                    T *__restrict__ wv, const double *inv, GmresState *st, uint32_t k)
+__global__ void __launch_bounds__(kBlock) k_gm_spmv(Csr<T> M, const T *__restrict__ z, T *__restrict__ wv,
+                                                    const double *inv, GmresState *st, uint32_t k)
 {
     pdl_wait();
     pdl_release();
@@ -180,7 +180,7 @@ __global__ void __launch_bounds__(kBlock) k_gm_spmv(Csr<T> M, Sell<T> S, int use
     const double s = inv[k];
     auto gx = [&](uint32_t c) { return z[c]; };
     auto epi = [&](uint32_t row, T v) { wv[row] = T(double(v) * s); };
-    for_rows_any<T, RPW>(M, S, use_sell != 0, gx, epi, smem_raw, &st->ticket[7], true);
+    for_rows_tma<T, RPW>(M, gx, epi, smem_raw, &st->ticket[7], true);
 }
 
 // One Arnoldi product: w = A z_k (FUSE; otherwise w is read) and h_i = v_i^T w for i <= k.
@@ -651,8 +651,8 @@ rsg_status run_typed(rsg_context *ctx, const GmresArgs &a, double *seconds)
                 if (us) {
                     launch_step<float, true>(st, pdl, g_dot, a, S32, n, ld, a.V32, z, w, k);
                 } else {
-                    launch_k(st, pdl, k_gm_spmv<RPW, float>, g_sp32, kBlock, s32, M32, S32, us, z, w,
-                             (const double *)a.inv, a.st, k);
+                    launch_k(st, pdl, k_gm_spmv<RPW, float>, g_sp32, kBlock, s32, M32, z, w, (const double *)a.inv,
+                             a.st, k);
                     launch_step<float, false>(st, pdl, g_dot, a, S32, n, ld, a.V32, z, w, k);
                 }
                 launch_k(st, pdl, k_gm_correct<PK, float, float>, g_cor, kBlock, 0, n, ld, a.P.w, a.P.d32, a.V32, w,
@@ -675,8 +675,7 @@ rsg_status run_typed(rsg_context *ctx, const GmresArgs &a, double *seconds)
             if (us) {
                 launch_step<double, true>(st, pdl, g_dot, a, S, n, ld, a.V, z, w, k);
             } else {
-                launch_k(st, pdl, k_gm_spmv<RPW, double>, g_sp, kBlock, s64, M, S, us, z, w, (const double *)a.inv,
-                         a.st, k);
+                launch_k(st, pdl, k_gm_spmv<RPW, double>, g_sp, kBlock, s64, M, z, w, (const double *)a.inv, a.st, k);
                 launch_step<double, false>(st, pdl, g_dot, a, S, n, ld, a.V, z, w, k);
             }
             launch_k(st, pdl, k_gm_correct<PK, double, double>, g_cor, kBlock, 0, n, ld, a.P.w, a.P.d, a.V, w,

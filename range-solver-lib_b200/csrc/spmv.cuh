@@ -421,6 +421,7 @@ __device__ __forceinline__ void ld4(const double *p, double (&v)[4])
 template <int CACHE = kSellStream>
 __device__ __forceinline__ void ld4(const float *p, float (&v)[4])
 {
+    static_assert(CACHE == kSellStream, "FP32 values are only streamed");
     const float4 a = __ldcs(reinterpret_cast<const float4 *>(p));
     v[0] = a.x;
     v[1] = a.y;
