@@ -49,7 +49,8 @@ struct BatchCtl {
     uint32_t body_count;
     uint32_t body_limit;
     int32_t timeout;
-    int32_t pad;
+    int32_t keep;
+    uint32_t cut;  // bodies in a row in which no system made more than one iteration
 };
 
 constexpr int kBatchIterations = 4;
@@ -519,12 +520,19 @@ __global__ void __launch_bounds__(kBlock) bk_list(const CgState *S, const uint32
 
 // Loop control: rebuilds the list of active systems, keeps the graph's while node
 // running while any system is active, enforces the hard limit.
-__global__ void __launch_bounds__(kBlock) bk_tail(const CgState *S, const uint32_t *sys_slice, uint32_t n_sys,
+__global__ void __launch_bounds__(kBlock) bk_tail(CgState *S, const uint32_t *sys_slice, uint32_t n_sys,
                                                   const Active L, BatchCtl *ctl, cudaGraphConditionalHandle h,
-                                                  int use_cond)
+                                                  int use_cond, int iterations)
 {
     pdl_wait();
     pdl_release();
+    bool far = iterations < 4;  // some system made more than one iteration (kCutBodies)
+    for (uint32_t i = threadIdx.x; i < n_sys; i += blockDim.x) {
+        const uint32_t it = S[i].it;
+        far = far || it - S[i].last_it > 1;
+        S[i].last_it = it;
+    }
+    const int any_far = __syncthreads_or(far);
     build_list(n_sys, nullptr, sys_slice, L, [&](uint32_t i) { return S[i].done == 0; });
     if (threadIdx.x == 0) {
         const uint32_t bc = ++ctl->body_count;
@@ -533,8 +541,10 @@ __global__ void __launch_bounds__(kBlock) bk_tail(const CgState *S, const uint32
             ctl->timeout = 1;
             keep = 0;
         }
-        if (use_cond) cudaGraphSetConditional(h, keep ? 1u : 0u);
-        ctl->pad = keep;
+        const uint32_t cut = any_far ? 0u : ctl->cut + 1;
+        ctl->cut = cut;
+        if (use_cond) cudaGraphSetConditional(h, keep && cut < kCutBodies ? 1u : 0u);
+        ctl->keep = keep;
     }
 }
 
@@ -762,7 +772,7 @@ rsg_status rsg_batch_solve(rsg_context *ctx, rsg_batch *B, const rsg_solver_conf
         h.stop_rule = RSG_STOP_TRUE_RELRES;
         std::vector<CgState> hs(ns, h);
         RSG_CHECK_CUDA(ctx, cudaMemcpyAsync(S, hs.data(), ns * sizeof(CgState), cudaMemcpyHostToDevice, sm));
-        BatchCtl c = {0, body_limit_for(max_it), 0, 1};
+        BatchCtl c = {0, body_limit_for(max_it), 0, 1, 0};
         RSG_CHECK_CUDA(ctx, cudaMemsetAsync(T.ticket, 0, ns * sizeof(unsigned int), sm));
         RSG_CHECK_CUDA(ctx, cudaMemcpyAsync(ctl, &c, sizeof(c), cudaMemcpyHostToDevice, sm));
         // the lists start with every system
@@ -798,8 +808,8 @@ rsg_status rsg_batch_solve(rsg_context *ctx, rsg_batch *B, const rsg_solver_conf
         bk_init_z<false><<<g, kBlock, 0, sm>>>(V, L_all, n, jac ? d : nullptr, nullptr, r, z, r32, z32, T, S);
     RSG_CHECK_CUDA(ctx, cudaGetLastError());
 
-    auto body = [&](cudaGraphConditionalHandle h, int use_cond, bool pdl) {
-        for (int it = 0; it < kBatchIterations; it++) {
+    auto body = [&](cudaGraphConditionalHandle h, int use_cond, bool pdl, int iterations) {
+        for (int it = 0; it < iterations; it++) {
             if (!mixed) {
                 launch_k(sm, pdl, bk_dir<double, false>, g, kBlock, 0, M64, V, L_act, z, p0, p1, q, xp,
                          (float *)nullptr, T, S);
@@ -818,27 +828,35 @@ rsg_status rsg_batch_solve(rsg_context *ctx, rsg_batch *B, const rsg_solver_conf
         else
             launch_k(sm, pdl, bk_check<true>, g, kBlock, 0, M64, V, L_chk, (double *)nullptr, jac ? d32 : (float *)nullptr,
                      bp, xp, y32, r, z, r32, z32, T, S);
-        launch_k(sm, pdl, bk_tail, 1, kBlock, 0, S, B->d_sys_slice, ns, L_act, ctl, h, use_cond);
+        launch_k(sm, pdl, bk_tail, 1, kBlock, 0, S, B->d_sys_slice, ns, L_act, ctl, h, use_cond, iterations);
     };
     const bool pdl = pdl_for(B->A, mixed);
 
     if (conf->use_graph) {
-        cudaGraph_t graph = nullptr;
-        cudaGraphExec_t exec = nullptr;
-        RSG_TRY(while_graph(ctx, pdl, [&](cudaGraphConditionalHandle h, bool with_pdl) { body(h, 1, with_pdl); }, &graph,
-                            &exec));
-        cudaError_t e = cudaGraphLaunch(exec, sm);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(sm);
-        cudaGraphExecDestroy(exec);
-        cudaGraphDestroy(graph);
-        if (e != cudaSuccess) return set_error(ctx, RSG_ERR_CUDA, "batch solve: %s", cudaGetErrorString(e));
+        int iterations = kBatchIterations;  // of a body, or one (kCutBodies)
+        int32_t *keep = reinterpret_cast<int32_t *>(ctx->pinned);
+        do {
+            cudaGraph_t graph = nullptr;
+            cudaGraphExec_t exec = nullptr;
+            RSG_TRY(while_graph(ctx, pdl, [&](cudaGraphConditionalHandle h, bool with_pdl) {
+                body(h, 1, with_pdl, iterations);
+            }, &graph, &exec));
+            cudaError_t e = cudaGraphLaunch(exec, sm);
+            if (e == cudaSuccess) e = cudaMemcpyAsync(keep, &ctl->keep, sizeof(int32_t), cudaMemcpyDeviceToHost, sm);
+            const cudaError_t sync = cudaStreamSynchronize(sm);
+            cudaGraphExecDestroy(exec);
+            cudaGraphDestroy(graph);
+            if (e == cudaSuccess) e = sync;
+            if (e != cudaSuccess) return set_error(ctx, RSG_ERR_CUDA, "batch solve: %s", cudaGetErrorString(e));
+            iterations = 1;
+        } while (*keep);
     } else {
         const uint32_t polls = std::max<uint32_t>(1, conf->check_interval / kBatchIterations);
         int32_t *keep = reinterpret_cast<int32_t *>(ctx->pinned);
         for (;;) {
-            for (uint32_t k = 0; k < polls; k++) body(0, 0, pdl);
+            for (uint32_t k = 0; k < polls; k++) body(0, 0, pdl, kBatchIterations);
             RSG_CHECK_CUDA(ctx, cudaGetLastError());
-            RSG_CHECK_CUDA(ctx, cudaMemcpyAsync(keep, &ctl->pad, sizeof(int32_t), cudaMemcpyDeviceToHost, sm));
+            RSG_CHECK_CUDA(ctx, cudaMemcpyAsync(keep, &ctl->keep, sizeof(int32_t), cudaMemcpyDeviceToHost, sm));
             RSG_CHECK_CUDA(ctx, cudaStreamSynchronize(sm));
             if (!*keep) break;
         }

@@ -236,8 +236,8 @@ DirSell pick_blocks(rsg_context *ctx, const rsg_csr *A, int *grid)
 }
 DirSell pick_dir_sell(rsg_context *ctx, const rsg_csr *A, int *grid)
 {
-    const size_t vec = size_t(6) * A->n * sizeof(double), off = A->sell_len * (A->soff ? 2 : 4);
-    if (vec + off + A->sell_len * sizeof(double) <= kL2Keep) return pick_blocks<kSellKeep>(ctx, A, grid);
+    const size_t vec = size_t(6) * A->n * sizeof(double), off = A->sell_elems * (A->soff ? 2 : 4);
+    if (vec + off + A->sell_elems * sizeof(double) <= kL2Keep) return pick_blocks<kSellKeep>(ctx, A, grid);
     if (vec + off <= kL2Keep) return pick_blocks<kSellKeepOffsets>(ctx, A, grid);
     return pick_blocks<kSellOut>(ctx, A, grid);
 }
@@ -578,6 +578,7 @@ __global__ void __launch_bounds__(kBlock) k_mx_check(Csr<double> M, Sell<double>
 
 __global__ void k_mx_fold(uint32_t n, double *__restrict__ x, float *__restrict__ y, const CgState *st)
 {
+    if (!st->done) return;  // a graph that ended for short bodies
     const double inv_sigma = 1.0 / st->sigma;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         x[i] = fma(double(y[i]), inv_sigma, x[i]);
@@ -585,8 +586,8 @@ __global__ void k_mx_fold(uint32_t n, double *__restrict__ x, float *__restrict_
     }
 }
 
-// Loop control: counts bodies, enforces the hard limit, drives the graph's while node.
-__global__ void k_tail(CgState *st, cudaGraphConditionalHandle h, int use_cond)
+// Loop control: counts bodies (of so many iterations), enforces the hard limit, drives the graph's while node.
+__global__ void k_tail(CgState *st, cudaGraphConditionalHandle h, int use_cond, uint32_t iterations)
 {
     pdl_wait();
     pdl_release();
@@ -596,7 +597,11 @@ __global__ void k_tail(CgState *st, cudaGraphConditionalHandle h, int use_cond)
         st->done = 1;
         st->status = RSG_ERR_TIMEOUT;
     }
-    if (use_cond) cudaGraphSetConditional(h, st->done ? 0u : 1u);
+    if (!use_cond) return;
+    const uint32_t it = st->it, cut = iterations >= 4 && 4 * (it - st->last_it) <= iterations ? st->cut + 1 : 0;
+    st->last_it = it;
+    st->cut = cut;
+    cudaGraphSetConditional(h, st->done || cut >= kCutBodies ? 0u : 1u);
 }
 
 // ---------------- host driver ----------------
@@ -713,7 +718,7 @@ void launch_body(rsg_context *ctx, const CgArgs &a, const Launch &L, cudaGraphCo
         }
     }
     if (PK != 3) check();
-    launch_k(st, pdl, k_tail, 1, 32, 0, a.st, h, use_cond);
+    launch_k(st, pdl, k_tail, 1, 32, 0, a.st, h, use_cond, uint32_t(iterations));
 }
 
 template <int RPW, int PK>
@@ -764,26 +769,28 @@ rsg_status run_typed(rsg_context *ctx, const CgArgs &a)
         if (a.mixed) k_mx_fold<<<L.g_vec, kBlock, 0, ctx->stream>>>(a.A->n, a.x, a.y32, a.st);
         RSG_CHECK_CUDA(ctx, cudaEventRecord(ctx->ev[1], ctx->stream));
     } else if (a.use_graph) {
-        cudaGraph_t graph = nullptr;
-        cudaGraphExec_t exec = nullptr;
-        // the solve loop: one while node whose body is kBodyIterations CG iterations
-        rsg_status s = while_graph(ctx, pdl_for(a.A, a.mixed), [&](cudaGraphConditionalHandle h, bool pdl) {
-            launch_body<RPW, PK>(ctx, a, L, h, 1, pdl, PK == 3 ? 2 : kBodyIterations);
-        }, &graph, &exec);
-        if (s == RSG_OK) {
+        // the solve loop: one while node whose body is kBodyIterations CG iterations, or one (kCutBodies)
+        int32_t *done_h = reinterpret_cast<int32_t *>(ctx->pinned);
+        int iterations = PK == 3 ? 2 : kBodyIterations;
+        do {
+            cudaGraph_t graph = nullptr;
+            cudaGraphExec_t exec = nullptr;
+            RSG_TRY(while_graph(ctx, pdl_for(a.A, a.mixed), [&](cudaGraphConditionalHandle h, bool pdl) {
+                launch_body<RPW, PK>(ctx, a, L, h, 1, pdl, iterations);
+            }, &graph, &exec));
             cudaError_t e = cudaGraphLaunch(exec, ctx->stream);
-            if (e != cudaSuccess) s = set_error(ctx, RSG_ERR_CUDA, "graph launch: %s", cudaGetErrorString(e));
-        }
-        if (s == RSG_OK && a.mixed)
-            k_mx_fold<<<L.g_vec, kBlock, 0, ctx->stream>>>(a.A->n, a.x, a.y32, a.st);
-        if (s == RSG_OK) {
-            cudaEventRecord(ctx->ev[1], ctx->stream);
-            cudaError_t e = cudaStreamSynchronize(ctx->stream);
-            if (e != cudaSuccess) s = set_error(ctx, RSG_ERR_CUDA, "solve: %s", cudaGetErrorString(e));
-        }
-        if (exec) cudaGraphExecDestroy(exec);
-        if (graph) cudaGraphDestroy(graph);
-        if (s != RSG_OK) return s;
+            if (e == cudaSuccess && a.mixed)
+                k_mx_fold<<<L.g_vec, kBlock, 0, ctx->stream>>>(a.A->n, a.x, a.y32, a.st);
+            if (e == cudaSuccess) e = cudaEventRecord(ctx->ev[1], ctx->stream);
+            if (e == cudaSuccess)
+                e = cudaMemcpyAsync(done_h, &a.st->done, sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream);
+            const cudaError_t sync = cudaStreamSynchronize(ctx->stream);
+            cudaGraphExecDestroy(exec);
+            cudaGraphDestroy(graph);
+            if (e == cudaSuccess) e = sync;
+            if (e != cudaSuccess) return set_error(ctx, RSG_ERR_CUDA, "solve: %s", cudaGetErrorString(e));
+            iterations = 1;
+        } while (!*done_h);
     } else {
         const uint32_t bodies_per_poll = std::max<uint32_t>(1, a.check_interval / 2);
         int32_t *done_h = reinterpret_cast<int32_t *>(ctx->pinned);

@@ -68,8 +68,7 @@ struct rsg_csr {
     // slice_ptr[s] + (k/4)*128 + 4l + k%4, rows padded to a multiple of 4)
     bool use_sell = false;
     uint32_t n_slices = 0;
-    uint64_t sell_len = 0;            // elements of the padded copy
-    uint64_t sell_elems = 0;
+    uint64_t sell_elems = 0;          // elements of the padded copy
     uint32_t *slice_ptr = nullptr;    // n_slices + 1
     uint32_t *slice_len4 = nullptr;   // padded row length / 4 per slice
     double *sval = nullptr;

@@ -272,7 +272,6 @@ static rsg_status build_sell(rsg_context *ctx, rsg_csr *A, bool force)
     }
     A->sell_elems = total;
     const size_t t = std::max<uint64_t>(total, 1);
-    A->sell_len = t;
     if (cudaMalloc(&A->slice_ptr, ptr.size() * sizeof(uint32_t)) != cudaSuccess ||
         cudaMalloc(&A->sval, t * sizeof(double)) != cudaSuccess ||
         cudaMalloc(&A->sval32, t * sizeof(float)) != cudaSuccess ||
