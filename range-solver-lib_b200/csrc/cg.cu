@@ -592,16 +592,19 @@ __global__ void k_tail(CgState *st, cudaGraphConditionalHandle h, int use_cond, 
     pdl_wait();
     pdl_release();
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    const uint32_t bc = ++st->body_count;
-    if (!st->done && bc >= st->body_limit) {
+    // all loads before the first store: one round trip to L2 instead of one each
+    const uint32_t bc = st->body_count + 1, limit = st->body_limit, it = st->it, last_it = st->last_it, was_cut = st->cut;
+    const int32_t done = st->done;
+    const bool timeout = !done && bc >= limit;
+    const uint32_t cut = iterations >= 4 && 4 * (it - last_it) <= iterations ? was_cut + 1 : 0;
+    if (use_cond) cudaGraphSetConditional(h, done || timeout || cut >= kCutBodies ? 0u : 1u);
+    st->body_count = bc;
+    st->last_it = it;
+    st->cut = cut;
+    if (timeout) {
         st->done = 1;
         st->status = RSG_ERR_TIMEOUT;
     }
-    if (!use_cond) return;
-    const uint32_t it = st->it, cut = iterations >= 4 && 4 * (it - st->last_it) <= iterations ? st->cut + 1 : 0;
-    st->last_it = it;
-    st->cut = cut;
-    cudaGraphSetConditional(h, st->done || cut >= kCutBodies ? 0u : 1u);
 }
 
 // ---------------- host driver ----------------

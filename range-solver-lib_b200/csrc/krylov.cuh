@@ -34,14 +34,15 @@ struct CgState {
     uint32_t pcur;          // which direction buffer holds the latest p (graph and host loops)
     uint32_t body_count;
     uint32_t body_limit;
-    uint32_t last_it;       // it at the end of the graph's last body, and how many bodies in a row were cut short
-    uint32_t cut;
     int32_t evict_first32;  // L2 policy of the FP32 matrix stream (1 evict_first, 0 evict_last)
     int32_t auto_switch;    // RSG_PRECISION_AUTO: a drifted refresh ends the mixed loop (switched = 1)
     int32_t switched;
     double *history;   // error per iteration (may be null)
     double *trend_hist;
     unsigned int ticket[8];  // [7] = bounded-wait error word; not part of a copied state (kStateWords)
+    // the tail's alone, so behind the copied words:
+    uint32_t last_it;        // it at the end of the graph's last body
+    uint32_t cut;            // bodies in a row that were cut short (kCutBodies)
 };
 constexpr uint32_t kStateWords = uint32_t(offsetof(CgState, ticket) / sizeof(uint32_t));
 
