@@ -31,7 +31,7 @@ constexpr int K2 = 2 * H;       // 128
 constexpr int kTileRows = 128;
 constexpr int kThreads = 256;
 constexpr uint32_t kTmemCols = 64;
-// CTAs of the layer kernel per SM.  Three leave 84 registers a thread (four: 64 and spills) and L1 for the gathers,
+// CTAs of the layer kernel per SM.  Three leave a thread the 80 registers that it uses (four: 64 and spills) and L1 for the gathers,
 // two too few loads in flight; six layers of 219k rows and their input: 365, 320 and 381 us with 4, 3 and 2.
 constexpr int kCtasPerSm = 3;
 constexpr int kCarveout = 71;  // percent: their 162 KB; the rest caches gathered rows (100: 323 us instead of 315)
