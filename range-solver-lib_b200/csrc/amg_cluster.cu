@@ -543,9 +543,11 @@ rsg_status amg_cluster_extents(rsg_context *ctx, AmgHierarchy *H)
         }
     }
     s.inv = H->coarse_inv.p;
-    if (!K.ext.ensure(size_t(kAmgMaxLevels) * C * 4)) return set_error(ctx, RSG_ERR_OUT_OF_MEMORY, "amg: cluster extents");
-    if (!K.ext_h && cudaMallocHost(&K.ext_h, size_t(kAmgMaxLevels) * C * 4 * sizeof(uint32_t)) != cudaSuccess)
-        return set_error(ctx, RSG_ERR_OUT_OF_MEMORY, "amg: cluster extents");
+    if (!K.ext.ensure(size_t(kAmgMaxLevels) * C * 4) ||
+        (!K.ext_h && cudaMallocHost(&K.ext_h, size_t(kAmgMaxLevels) * C * 4 * sizeof(uint32_t)) != cudaSuccess)) {
+        (void)cudaGetLastError();  // no memory for it: the launched kernels
+        return RSG_OK;
+    }
     k_cl_extent<<<dim3(C, m.nl), 256, 0, ctx->stream>>>(s, K.ext.p);
     RSG_CHECK_CUDA(ctx, cudaGetLastError());
     RSG_CHECK_CUDA(ctx, cudaMemcpyAsync(K.ext_h, K.ext.p, size_t(m.nl) * C * 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost,
@@ -621,8 +623,10 @@ rsg_status amg_cluster_pack(rsg_context *ctx, AmgHierarchy *H)
         (void)cudaGetLastError();
     }
     if (!K.supported) return RSG_OK;
-    if (!K.blob.ensure(size_t(m.stride) * C) || !K.place.ensure(size_t(C) * m.nl * window))
-        return set_error(ctx, RSG_ERR_OUT_OF_MEMORY, "amg: packed coarse levels");
+    if (!K.blob.ensure(size_t(m.stride) * C) || !K.place.ensure(size_t(C) * m.nl * window)) {
+        (void)cudaGetLastError();
+        return RSG_OK;
+    }
     ClSrcs s = {};
     for (uint32_t j = 0; j < m.nl; j++) {
         const AmgLevel &F = H->L[l0 + int(j)], &N = H->L[l0 + int(j) + 1];
