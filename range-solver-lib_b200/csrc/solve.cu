@@ -138,7 +138,7 @@ extern "C" rsg_status rsg_solve(rsg_context *ctx, rsg_csr *A, const rsg_solver_c
     const uint32_t max_it = std::max<uint32_t>(c.n_outer, 1);
     const uint32_t m = std::max<uint32_t>(c.n_inner, 1);
     const bool want_hist = c.output_frequency > 0 || (c.output_file && c.output_file[0]);
-    const uint32_t hist_len = gmres ? max_it + 1 : max_it;
+    const size_t hist_len = size_t(max_it) + 1;  // GMRES logs its start too, AUTO one iteration after a switch at the cap
 
     // ---- workspace ----
     const size_t vn = arena_bytes(n, sizeof(double)), vf = arena_bytes(n, sizeof(float));
